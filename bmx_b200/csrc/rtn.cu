@@ -13,9 +13,8 @@
 //             rtn_token   -> page x 4 fp16, [row][channel group] (unused groups zero)
 //   V scales: page x 4 fp16, [row][channel group]
 //
-// The decode kernel needs no shared-memory staging: every lane's operands are contiguous 16-byte
-// pieces of the page block, so a warp's global loads are fully coalesced and land directly in the
-// mma fragment registers; the next tile is prefetched into registers while the current one is used.
+// The decode kernel's page blocks arrive by bulk copies in a shared-memory ring; every lane's operands are
+// contiguous 16-byte pieces of the block, adjacent between lanes, in mma fragment order.
 #include "decode_common.cuh"
 
 namespace bmxk {
@@ -188,29 +187,55 @@ struct RtnDecodeParams {
   int batch;
   float scale_log2;
   float* part;
+  int32_t* status;
+  int n_stages;
 };
 
-struct RtnFrag {   // one warp's operands of one tile, as loaded
-  uint4 k0, k1, v, ks[4];
-  uint2 vs0, vs1;
-  bool valid;
-};
+constexpr int RTN_CTAS_PER_SM = 2;   // resident decode CTAs
+constexpr int RTN_THREADS = 288;     // eight computing warps and one that issues the copies
+constexpr int RTN_MAX_STAGES = 6;
+constexpr int RTN_Q_STRIDE = 20;     // words of a lane's query fragments in shared memory (16, padded: 128-bit reads free of conflicts)
+constexpr int RTN_FIXED_SMEM = (8 * 8 * HEAD_DIM + 128 + 32 * RTN_Q_STRIDE) * 4 + 2 * RTN_MAX_STAGES * 8;  // range reduction, queries, barriers
 
-template <int PAGE>
-__global__ void __launch_bounds__(256, 1) rtn_decode_kernel(const RtnDecodeParams p) {
+__device__ __forceinline__ void rtn_consumers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+// What bounds it: instruction issue and latency, not bytes (112 per token and head with groups of 32).  One warp issues the copies of
+// whole page blocks, up to n_stages tiles ahead (a register prefetch of one tile left the page-table lookup and the DRAM latency on the
+// path of every tile); eight warps own 16 token rows each.  The arm and the groups are template parameters, so that every operand index
+// is a constant, and two CTAs share an SM.  Integer operands stay integers until the product:
+//   keys    a nibble becomes the fp16 SUBNORMAL (code + 8) * 2^-24 (low nibbles) or * 2^-20 (high nibbles) with one LOP3; low and
+//           high nibbles go to separate products, whose accumulators differ by an exact factor 16; the offset 8 is taken out by a
+//           second product with constant rows (tensor pipe, idle otherwise) and the same queries, so it cancels exactly up to the
+//           fp32 accumulation.  rtn_channel: the scales of the warp's token group multiply the queries (16 products instead of
+//           32).  The queries are scaled by a power of two so that max |q| < 1: the product with any fp16 scale stays finite.
+//           rtn_token: one accumulator pair per channel group, scaled in float32.
+//   values  codes 0, 1, -2, -1 as fp16 have zero low bytes: one byte-permute lookup yields the high bytes of four codes.
+// The weights' running maximum moves only when a score passes it by more than 8 (log2): that test needs no cross-lane reduction.
+// Measured, 16 sequences x 8192 tokens x 8 heads, 4-bit keys, groups of 32: step (with merge) 123 -> 59 us, kernel 115 -> 50 us = 2.4 TB/s;
+// 43 -> 26 million warp instructions, 650 -> 400 per 16 token rows; the byte permutes and LOP3s (half-rate pipe, 49 % busy) lead.
+template <int PAGE, int ARM, int KG, int VG>
+__global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kernel(const RtnDecodeParams p) {
   constexpr int PAGES_PER_TILE = TILE_TOKENS / PAGE, WR_PER_PAGE = PAGE / 16;
   extern __shared__ __align__(16) uint8_t smem[];
-  float* red = reinterpret_cast<float*>(smem);       // [8 warps][8 q][128]
-  float* red_m = red + 8 * 8 * HEAD_DIM;              // [8][8]
-  float* red_l = red_m + 64;
-  int* cum = reinterpret_cast<int*>(red_l + 64);      // [batch + 1]
-  int* npg_sm = cum + p.batch + 1;
   const RtnGeom g = p.g;
-  const int G = g.n_q_groups, PB = rtn_block_bytes(g);
+  const int G = g.n_q_groups, PB = rtn_block_bytes(g), stage_bytes = PB * PAGES_PER_TILE;
+  uint8_t* ring = smem;
+  float* red = reinterpret_cast<float*>(smem + p.n_stages * stage_bytes);  // [8 warps][8 q][128]
+  float* red_m = red + 8 * 8 * HEAD_DIM;                                    // [8][8]
+  float* red_l = red_m + 64;
+  uint32_t* q_sm = reinterpret_cast<uint32_t*>(red_l + 64);                 // [32 lanes][RTN_Q_STRIDE] query fragments, the same for all warps
+  uint64_t* full = reinterpret_cast<uint64_t*>(q_sm + 32 * RTN_Q_STRIDE);   // [RTN_MAX_STAGES] a tile's blocks have landed
+  uint64_t* empty = full + RTN_MAX_STAGES;                                  // [RTN_MAX_STAGES] all eight warps are done with it
+  int* cum = reinterpret_cast<int*>(empty + RTN_MAX_STAGES);                // [batch + 1]
+  int* npg_sm = cum + p.batch + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t4 = lane & 3;
   asm volatile("griddepcontrol.launch_dependents;");  // the merge kernel is this kernel's programmatic dependent (see launch_merge)
   if (warp == 0) fill_cum(cum, p.n_pages, p.batch, g.h_kv, PAGE, lane);
-  for (int i = tid; i < p.batch; i += 256) npg_sm[i] = p.n_pages[i];
+  if (tid == 32) {
+    for (int i = 0; i < p.n_stages; ++i) mbar_init(full + i, 1), mbar_init(empty + i, 8);
+    fence_barrier_init();
+  }
+  for (int i = tid; i < p.batch; i += RTN_THREADS) npg_sm[i] = p.n_pages[i];
   __syncthreads();
   const int total = cum[p.batch];
   const int per_cta = (total + gridDim.x - 1) / gridDim.x;
@@ -218,43 +243,40 @@ __global__ void __launch_bounds__(256, 1) rtn_decode_kernel(const RtnDecodeParam
   if (f_begin >= f_end) return;
   TileCursor cur;
   cur.init(cum, npg_sm, f_begin, PAGE);
-  const int sub_page = warp / WR_PER_PAGE, wr = warp % WR_PER_PAGE;
-  const int kgrp = (16 * wr) / g.k_group;  // token group of this warp's rows (channel-grouped keys)
 
-  auto load = [&](const TileCursor& c) {
-    RtnFrag f;
-    const int valid_pages = min(PAGES_PER_TILE, npg_sm[c.b] - c.j * PAGES_PER_TILE);
-    f.valid = sub_page < valid_pages;
-    if (f.valid) {
-      const int slot = p.page_table[(int64_t)c.b * p.table_stride + c.j * PAGES_PER_TILE + sub_page];
-      const uint8_t* blk = p.pages + ((int64_t)slot * g.h_kv + c.h) * PB;
-      f.k0 = *reinterpret_cast<const uint4*>(blk + ((wr * 2 + 0) * 32 + lane) * 16);
-      f.k1 = *reinterpret_cast<const uint4*>(blk + ((wr * 2 + 1) * 32 + lane) * 16);
-      f.v = *reinterpret_cast<const uint4*>(blk + rtn_off_vcode(g) + (wr * 32 + lane) * 16);
-      const uint8_t* ks = blk + rtn_off_kscale(g);
-      if (g.k_arm == RTN_CHANNEL) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) f.ks[k] = *reinterpret_cast<const uint4*>(ks + (kgrp * 128 + k * 32 + t4 * 8) * 2);
-      } else {  // [row][4] halfs for rows g and g+8
-        const uint2 a = *reinterpret_cast<const uint2*>(ks + (16 * wr + gq) * 8);
-        const uint2 b = *reinterpret_cast<const uint2*>(ks + (16 * wr + gq + 8) * 8);
-        f.ks[0] = make_uint4(a.x, a.y, b.x, b.y);
+  if (warp == 8) {  // copies
+    if (lane == 0) {
+      int st = 0, issued = 0;
+      uint32_t ph = 1;  // parity to wait for on `empty`: the first pass over the ring finds every stage free
+      for (int f = f_begin; f < f_end; ++f) {
+        if (!wait_or_flag(empty + st, ph, p.status, 60)) break;
+        const int pages_here = min(PAGES_PER_TILE, npg_sm[cur.b] - cur.j * PAGES_PER_TILE);
+        mbar_arrive_expect_tx(full + st, (uint32_t)(pages_here * PB));
+        for (int i = 0; i < pages_here; ++i) {
+          const int slot = p.page_table[(int64_t)cur.b * p.table_stride + cur.j * PAGES_PER_TILE + i];
+          bulk_g2s(ring + st * stage_bytes + i * PB, p.pages + ((int64_t)slot * g.h_kv + cur.h) * PB, (uint32_t)PB, full + st);
+        }
+        ++issued;
+        cur.next(npg_sm, g.h_kv, PAGE, p.batch);
+        if (++st == p.n_stages) st = 0, ph ^= 1;
       }
-      const uint8_t* vs = blk + rtn_off_vscale(g);
-      f.vs0 = *reinterpret_cast<const uint2*>(vs + (16 * wr + gq) * 8);
-      f.vs1 = *reinterpret_cast<const uint2*>(vs + (16 * wr + gq + 8) * 8);
+      if (issued < f_end - f_begin)  // a wait ran out: no copy may be in flight when this CTA ends
+        for (int i = max(0, issued - p.n_stages); i < issued; ++i) mbar_wait_bounded(full + i % p.n_stages, (i / p.n_stages) & 1);
     }
-    return f;
-  };
+    return;
+  }
 
-  uint32_t qb[8][2];
+  const int sub_page = warp / WR_PER_PAGE, wr = warp % WR_PER_PAGE;
+  // byte offsets of this lane's pieces inside a tile's stage
+  const int off_k = sub_page * PB + (wr * 64 + lane) * 16, off_v = sub_page * PB + rtn_off_vcode(g) + (wr * 32 + lane) * 16;
+  const int off_ks = sub_page * PB + rtn_off_kscale(g) + (ARM == RTN_CHANNEL ? (((16 * wr) / KG) * 128 + t4 * 8) * 2 : (16 * wr + gq) * 8);
+  const int off_vs = sub_page * PB + rtn_off_vscale(g) + (16 * wr + gq) * 8;
+
   float O[8][4];
-  float m0 = 0.f, m1 = 0.f, l0 = 0.f, l1 = 0.f;
+  float m0 = 0.f, m1 = 0.f, l0 = 0.f, l1 = 0.f, s_scale = 0.f;  // s_scale: scores in log2 units per accumulated unit
   int cur_bh = -1, cur_b = 0, cur_h = 0;
-  const __half2 c1032 = __floats2half2_rn(1032.f, 1032.f), c16th = __floats2half2_rn(0.0625f, 0.0625f);
-  const __half2 cm72 = __floats2half2_rn(-72.f, -72.f);
-  // two's-complement 2-bit value codes as fp16: 0, 1, -2, -1  (low bytes / high bytes of the four halfs)
-  const uint32_t lut_lo = 0x00000000u, lut_hi = 0xBCC03C00u;
+  // two's-complement 2-bit value codes as fp16: 0, 1, -2, -1 (high bytes; the low bytes are zero)
+  const uint32_t lut_hi = 0xBCC03C00u;
 
   auto flush = [&](int b_, int h_) {
 #pragma unroll
@@ -271,7 +293,7 @@ __global__ void __launch_bounds__(256, 1) rtn_decode_kernel(const RtnDecodeParam
       o[(2 * t4) * HEAD_DIM + 16 * mt + gq + 8] = O[mt][2];
       o[(2 * t4 + 1) * HEAD_DIM + 16 * mt + gq + 8] = O[mt][3];
     }
-    __syncthreads();
+    rtn_consumers_sync();
     float* dst = p.part + ((int64_t)(blockIdx.x + b_ * g.h_kv + h_) * G) * PART_STRIDE;
     for (int o = tid; o < G * HEAD_DIM; o += 256) {
       const int qi = o / HEAD_DIM, ch = o % HEAD_DIM;
@@ -289,114 +311,174 @@ __global__ void __launch_bounds__(256, 1) rtn_decode_kernel(const RtnDecodeParam
       dst[qi * PART_STRIDE + 2 + ch] = acc;
       if (ch == 0) dst[qi * PART_STRIDE] = M, dst[qi * PART_STRIDE + 1] = l;
     }
-    __syncthreads();
+    rtn_consumers_sync();
   };
 
-  RtnFrag fr = load(cur);
+  int st = 0;
+  uint32_t ph = 0;
+  bool alive = true;  // false once a wait ran out: nothing is computed any more, barriers are still met
   for (int f = f_begin; f < f_end; ++f) {
     const int b = cur.b, h = cur.h, bh = cur.b * g.h_kv + cur.h;
-    TileCursor nxt = cur;
-    nxt.next(npg_sm, g.h_kv, PAGE, p.batch);
-    RtnFrag fn;
-    fn.valid = false;
-    if (f + 1 < f_end) fn = load(nxt);  // in flight while this tile is computed
+    const bool valid = cur.j * PAGES_PER_TILE + sub_page < npg_sm[b];
     if (bh != cur_bh) {
       if (cur_bh >= 0) flush(cur_b, cur_h);
       cur_bh = bh, cur_b = b, cur_h = h;
       m0 = (2 * t4 < G) ? -INFINITY : 0.f, m1 = (2 * t4 + 1 < G) ? -INFINITY : 0.f, l0 = l1 = 0.f;
 #pragma unroll
       for (int mt = 0; mt < 8; ++mt) O[mt][0] = O[mt][1] = O[mt][2] = O[mt][3] = 0.f;
+      // B operands: channel pair (8n + 2t, + 1) of query g, n = 0..15, scaled by 2^-e; every warp computes them, warp 0 stores
+      // them (the barriers of flush() lie between the last use of the previous ones and this store)
       const __half* qp = p.q + ((int64_t)bh * G + gq) * HEAD_DIM + 2 * t4;
+      uint32_t qb[16];
+      float qm = 0.f;
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        qb[ks][0] = (gq < G) ? *reinterpret_cast<const uint32_t*>(qp + 16 * ks) : 0u;
-        qb[ks][1] = (gq < G) ? *reinterpret_cast<const uint32_t*>(qp + 16 * ks + 8) : 0u;
+      for (int n = 0; n < 16; ++n) {
+        qb[n] = (gq < G) ? *reinterpret_cast<const uint32_t*>(qp + 8 * n) : 0u;
+        const float2 x = __half22float2(u32_as_h2(qb[n]));
+        qm = fmaxf(qm, fmaxf(fabsf(x.x), fabsf(x.y)));
       }
+#pragma unroll
+      for (int m = 16; m >= 1; m >>= 1) qm = fmaxf(qm, __shfl_xor_sync(0xffffffffu, qm, m));
+      int e = 0;
+      if (qm > 0.f && qm <= 65504.f) e = max(-13, min(15, ilogbf(qm) + 1));  // |q| < 2^e (<= 2^15 * 2); 2^-e is an fp16 number
+      if (warp == 0) {
+        const __half2 dn = __float2half2_rn(exp2f((float)-e));
+#pragma unroll
+        for (int n = 0; n < 16; ++n) q_sm[lane * RTN_Q_STRIDE + n] = h2_as_u32(__hmul2(u32_as_h2(qb[n]), dn));
+      }
+      rtn_consumers_sync();
+      s_scale = p.scale_log2 * exp2f((float)(e + 24));  // the codes enter as multiples of 2^-24
     }
-    if (fr.valid) {
-      // ---- keys: nibble -> half2 (one LOP3 + one exact fix-up), times the group scale ----
-      uint32_t acc[16][2];
-      const uint32_t ww[2][4] = {{fr.k0.x, fr.k0.y, fr.k0.z, fr.k0.w}, {fr.k1.x, fr.k1.y, fr.k1.z, fr.k1.w}};
-      const uint32_t scw[16] = {fr.ks[0].x, fr.ks[0].y, fr.ks[0].z, fr.ks[0].w, fr.ks[1].x, fr.ks[1].y, fr.ks[1].z, fr.ks[1].w,
-                                fr.ks[2].x, fr.ks[2].y, fr.ks[2].z, fr.ks[2].w, fr.ks[3].x, fr.ks[3].y, fr.ks[3].z, fr.ks[3].w};
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int qd = 0; qd < 4; ++qd) {
-          const uint32_t wlo = ww[c][qd], whi = ww[c][qd] >> 8;
-          const __half2 k0 = __hsub2(u32_as_h2(lop3<0x6A>(wlo, 0x000F000Fu, 0x64086408u)), c1032);
-          const __half2 k1 = __hfma2(u32_as_h2(lop3<0x6A>(wlo, 0x00F000F0u, 0x64806480u)), c16th, cm72);
-          const __half2 k2 = __hsub2(u32_as_h2(lop3<0x6A>(whi, 0x000F000Fu, 0x64086408u)), c1032);
-          const __half2 k3 = __hfma2(u32_as_h2(lop3<0x6A>(whi, 0x00F000F0u, 0x64806480u)), c16th, cm72);
-          __half2 s0, s1, s2, s3;
-          if (g.k_arm == RTN_CHANNEL) {
-            s0 = u32_as_h2(scw[4 * qd]), s1 = u32_as_h2(scw[4 * qd + 1]), s2 = u32_as_h2(scw[4 * qd + 2]), s3 = u32_as_h2(scw[4 * qd + 3]);
-          } else {  // per (row, channel group): words 0,1 hold row g's four scales, words 2,3 row g+8's
-            const int gi = (32 * qd) / g.k_group;
-            const uint32_t wsel = scw[2 * c + (gi >> 1)];
-            const __half sc = __ushort_as_half((unsigned short)((gi & 1) ? (wsel >> 16) : (wsel & 0xFFFFu)));
-            s0 = s1 = s2 = s3 = __half2half2(sc);
-          }
-          acc[4 * qd + 0][c] = h2_as_u32(__hmul2(k0, s0));
-          acc[4 * qd + 1][c] = h2_as_u32(__hmul2(k1, s1));
-          acc[4 * qd + 2][c] = h2_as_u32(__hmul2(k2, s2));
-          acc[4 * qd + 3][c] = h2_as_u32(__hmul2(k3, s3));
-        }
+    if (alive) alive = __all_sync(0xffffffffu, wait_or_flag(full + st, ph, p.status, 61));
+    if (alive && valid) {
+      const uint8_t* tile = ring + st * stage_bytes;
+      // ---- keys ----
+      const uint4 k0 = *reinterpret_cast<const uint4*>(tile + off_k), k1 = *reinterpret_cast<const uint4*>(tile + off_k + 512);
+      const uint32_t ww[2][4] = {{k0.x, k0.y, k0.z, k0.w}, {k1.x, k1.y, k1.z, k1.w}};
+      uint32_t tsc[4];  // rtn_token: the four scales of row g, then those of row g + 8
+      if (ARM == RTN_TOKEN) {
+        const uint2 x = *reinterpret_cast<const uint2*>(tile + off_ks), y = *reinterpret_cast<const uint2*>(tile + off_ks + 64);
+        tsc[0] = x.x, tsc[1] = x.y, tsc[2] = y.x, tsc[3] = y.y;
+      }
+      constexpr uint32_t M8A = 0x80088008u, M8B = 0x80808080u;  // -8 * 2^-24 and -8 * 2^-20, as fp16 pairs
       float S[4] = {0.f, 0.f, 0.f, 0.f};
+      constexpr int NG = ARM == RTN_CHANNEL ? 1 : HEAD_DIM / KG, QD_PER = 4 / NG;  // channel groups with an accumulator of their own
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks)
-        mma_f32acc(S[0], S[1], S[2], S[3], acc[2 * ks][0], acc[2 * ks][1], acc[2 * ks + 1][0], acc[2 * ks + 1][1], qb[ks][0], qb[ks][1]);
+      for (int gi = 0; gi < NG; ++gi) {
+        float Sa[4] = {0.f, 0.f, 0.f, 0.f}, Sb[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) S[i] *= p.scale_log2;
-      // ---- online softmax (base 2, lazy rescale), this lane owns queries 2t and 2t+1 ----
-      {
-        __half2 tm = __floats2half2_rn(fmaxf(S[0], S[2]), fmaxf(S[1], S[3]));
-        tm = __hmax2(tm, u32_as_h2(__shfl_xor_sync(0xffffffffu, h2_as_u32(tm), 4)));
-        tm = __hmax2(tm, u32_as_h2(__shfl_xor_sync(0xffffffffu, h2_as_u32(tm), 8)));
-        tm = __hmax2(tm, u32_as_h2(__shfl_xor_sync(0xffffffffu, h2_as_u32(tm), 16)));
-        const float2 tmf = __half22float2(tm);
-        const bool need0 = (2 * t4 < G) && (tmf.x > m0 + 8.f), need1 = (2 * t4 + 1 < G) && (tmf.y > m1 + 8.f);
-        if (__any_sync(0xffffffffu, need0 || need1)) {
-          const float n0 = need0 ? tmf.x + 0.5f : m0, n1 = need1 ? tmf.y + 0.5f : m1;
-          const float f0 = (m0 == -INFINITY) ? 0.f : ex2_approx(m0 - n0), f1 = (m1 == -INFINITY) ? 0.f : ex2_approx(m1 - n1);
-          l0 *= f0, l1 *= f1, m0 = n0, m1 = n1;
+        for (int qd = gi * QD_PER; qd < (gi + 1) * QD_PER; ++qd) {
+          const uint4 q4 = *reinterpret_cast<const uint4*>(q_sm + lane * RTN_Q_STRIDE + 4 * qd);
+          uint32_t b[4] = {q4.x, q4.y, q4.z, q4.w};  // channel octets 4qd .. 4qd+3
+          if (ARM == RTN_CHANNEL) {
+            const uint4 s4 = *reinterpret_cast<const uint4*>(tile + off_ks + 64 * qd);
+            const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
-          for (int mt = 0; mt < 8; ++mt) O[mt][0] *= f0, O[mt][1] *= f1, O[mt][2] *= f0, O[mt][3] *= f1;
+            for (int i = 0; i < 4; ++i) b[i] = h2_as_u32(__hmul2(u32_as_h2(b[i]), u32_as_h2(sw[i])));
+          }
+          const uint32_t w0 = ww[0][qd], w1 = ww[1][qd], x0 = w0 >> 8, x1 = w1 >> 8;
+          mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], lop3<0x6A>(w0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(w1, 0x000F000Fu, 0x00080008u),
+                     lop3<0x6A>(x0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(x1, 0x000F000Fu, 0x00080008u), b[0], b[2]);
+          mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], lop3<0x6A>(w0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(w1, 0x00F000F0u, 0x00800080u),
+                     lop3<0x6A>(x0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(x1, 0x00F000F0u, 0x00800080u), b[1], b[3]);
+          mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], M8A, M8A, M8A, M8A, b[0], b[2]);
+          mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], M8B, M8B, M8B, M8B, b[1], b[3]);
         }
+        if (ARM == RTN_CHANNEL) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) S[i] = fmaf(Sb[i], 0.0625f, Sa[i]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const uint32_t wsel = tsc[2 * c + (gi >> 1)];
+            const float sc = __half2float(__ushort_as_half((unsigned short)((gi & 1) ? (wsel >> 16) : (wsel & 0xFFFFu))));
+            S[2 * c] = fmaf(fmaf(Sb[2 * c], 0.0625f, Sa[2 * c]), sc, S[2 * c]);
+            S[2 * c + 1] = fmaf(fmaf(Sb[2 * c + 1], 0.0625f, Sa[2 * c + 1]), sc, S[2 * c + 1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[i] *= s_scale;
+      // ---- online softmax (base 2, lazy rescale), this lane owns queries 2t and 2t+1 ----
+      if (__any_sync(0xffffffffu, fmaxf(S[0], S[2]) > m0 + 8.f || fmaxf(S[1], S[3]) > m1 + 8.f)) {
+        float t0 = fmaxf(S[0], S[2]), t1 = fmaxf(S[1], S[3]);
+#pragma unroll
+        for (int m = 4; m <= 16; m <<= 1) t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, m)), t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, m));
+        const float n0 = t0 > m0 + 8.f ? t0 + 0.5f : m0, n1 = t1 > m1 + 8.f ? t1 + 0.5f : m1;
+        const float f0 = (m0 == -INFINITY) ? 0.f : ex2_approx(m0 - n0), f1 = (m1 == -INFINITY) ? 0.f : ex2_approx(m1 - n1);
+        l0 *= f0, l1 *= f1, m0 = n0, m1 = n1;
+#pragma unroll
+        for (int mt = 0; mt < 8; ++mt) O[mt][0] *= f0, O[mt][1] *= f1, O[mt][2] *= f0, O[mt][3] *= f1;
       }
       const float p0 = ex2_approx(S[0] - m0), p1 = ex2_approx(S[1] - m1), p2 = ex2_approx(S[2] - m0), p3 = ex2_approx(S[3] - m1);
       l0 += p0 + p2, l1 += p1 + p3;
       // ---- values: weights times the per-(row, channel group) scale, one B fragment per group ----
-      uint32_t pb[4][2];
-      const uint32_t vsw[4] = {fr.vs0.x, fr.vs0.y, fr.vs1.x, fr.vs1.y};
+      constexpr int NV = HEAD_DIM / VG;
+      uint32_t pb[NV][2];
+      const uint2 vs0 = *reinterpret_cast<const uint2*>(tile + off_vs), vs1 = *reinterpret_cast<const uint2*>(tile + off_vs + 64);
+      const uint32_t vsw[4] = {vs0.x, vs0.y, vs1.x, vs1.y};
 #pragma unroll
-      for (int gi = 0; gi < 4; ++gi)
-        if (gi < HEAD_DIM / g.v_group) {
-          const float sa = __half2float(__ushort_as_half((unsigned short)((gi & 1) ? (vsw[gi >> 1] >> 16) : (vsw[gi >> 1] & 0xFFFFu))));
-          const float sb = __half2float(__ushort_as_half((unsigned short)((gi & 1) ? (vsw[2 + (gi >> 1)] >> 16) : (vsw[2 + (gi >> 1)] & 0xFFFFu))));
-          pb[gi][0] = movmatrix_trans(h2_as_u32(__floats2half2_rn(p0 * sa, p1 * sa)));
-          pb[gi][1] = movmatrix_trans(h2_as_u32(__floats2half2_rn(p2 * sb, p3 * sb)));
-        } else {
-          pb[gi][0] = pb[gi][1] = 0u;
-        }
-      const uint32_t vv[4] = {fr.v.x, fr.v.y, fr.v.z, fr.v.w};
+      for (int gi = 0; gi < NV; ++gi) {
+        const float2 a2 = __half22float2(u32_as_h2(vsw[gi >> 1])), b2 = __half22float2(u32_as_h2(vsw[2 + (gi >> 1)]));
+        const float sa = (gi & 1) ? a2.y : a2.x, sb = (gi & 1) ? b2.y : b2.x;
+        pb[gi][0] = movmatrix_trans(h2_as_u32(__floats2half2_rn(p0 * sa, p1 * sa)));
+        pb[gi][1] = movmatrix_trans(h2_as_u32(__floats2half2_rn(p2 * sb, p3 * sb)));
+      }
+      const uint4 vc = *reinterpret_cast<const uint4*>(tile + off_v);
+      const uint32_t vv[4] = {vc.x, vc.y, vc.z, vc.w};
 #pragma unroll
       for (int jw = 0; jw < 4; ++jw) {
         const uint32_t x0 = vv[jw] & 0x33333333u, x1 = (vv[jw] >> 2) & 0x33333333u;
 #pragma unroll
         for (int hs = 0; hs < 2; ++hs) {
-          const uint32_t s0 = hs ? (x0 >> 16) : x0, s1 = hs ? (x1 >> 16) : x1;
-          const uint32_t lo0 = prmt(lut_lo, 0u, s0), hi0 = prmt(lut_hi, 0u, s0), lo1 = prmt(lut_lo, 0u, s1), hi1 = prmt(lut_hi, 0u, s1);
-          const int mt = 2 * jw + hs, gi = (16 * mt) / g.v_group;
-          mma_f32acc(O[mt][0], O[mt][1], O[mt][2], O[mt][3], prmt(lo0, hi0, 0x5140u), prmt(lo0, hi0, 0x7362u),
-                     prmt(lo1, hi1, 0x5140u), prmt(lo1, hi1, 0x7362u), pb[gi][0], pb[gi][1]);
+          const uint32_t hi0 = prmt(lut_hi, 0u, hs ? (x0 >> 16) : x0), hi1 = prmt(lut_hi, 0u, hs ? (x1 >> 16) : x1);
+          constexpr int MT_PER = VG / 16;
+          const int mt = 2 * jw + hs, gi = mt / MT_PER;
+          mma_f32acc(O[mt][0], O[mt][1], O[mt][2], O[mt][3], prmt(hi0, 0u, 0x1404u), prmt(hi0, 0u, 0x3424u), prmt(hi1, 0u, 0x1404u),
+                     prmt(hi1, 0u, 0x3424u), pb[gi][0], pb[gi][1]);
         }
       }
     }
-    fr = fn;
-    cur = nxt;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty + st);
+    cur.next(npg_sm, g.h_kv, PAGE, p.batch);
+    if (++st == p.n_stages) st = 0, ph ^= 1;
   }
   if (cur_bh >= 0) flush(cur_b, cur_h);
+}
+
+template <int PAGE, int ARM, int KG, int VG>
+static int launch_rtn_decode(const RtnDecodeParams& prm, int grid, size_t smem, cudaStream_t s) {
+  static PerDeviceOnce configured;
+  if (configured.first()) {
+    const cudaError_t e = cudaFuncSetAttribute(rtn_decode_kernel<PAGE, ARM, KG, VG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    if (e != cudaSuccess) {
+      configured.retract();
+      set_error("bmxk_rtn_decode: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      return BMXK_ERR_CUDA;
+    }
+  }
+  rtn_decode_kernel<PAGE, ARM, KG, VG><<<grid, RTN_THREADS, smem, s>>>(prm);
+  return check_launch("bmxk_rtn_decode");
+}
+template <int PAGE, int ARM, int KG>
+static int launch_rtn_decode_v(const RtnDecodeParams& prm, int grid, size_t smem, cudaStream_t s) {
+  if (prm.g.v_group == 32) return launch_rtn_decode<PAGE, ARM, KG, 32>(prm, grid, smem, s);
+  if (prm.g.v_group == 64) return launch_rtn_decode<PAGE, ARM, KG, 64>(prm, grid, smem, s);
+  return launch_rtn_decode<PAGE, ARM, KG, 128>(prm, grid, smem, s);
+}
+template <int PAGE>
+static int launch_rtn_decode_k(const RtnDecodeParams& prm, int grid, size_t smem, cudaStream_t s) {
+  const int kg = prm.g.k_group;
+  if (prm.g.k_arm == RTN_CHANNEL) {
+    if (kg == 32) return launch_rtn_decode_v<PAGE, RTN_CHANNEL, 32>(prm, grid, smem, s);
+    if constexpr (PAGE == 128)  // a token group never spans pages
+      if (kg == 128) return launch_rtn_decode_v<PAGE, RTN_CHANNEL, 128>(prm, grid, smem, s);
+    return launch_rtn_decode_v<PAGE, RTN_CHANNEL, 64>(prm, grid, smem, s);
+  }
+  if (kg == 32) return launch_rtn_decode_v<PAGE, RTN_TOKEN, 32>(prm, grid, smem, s);
+  if (kg == 64) return launch_rtn_decode_v<PAGE, RTN_TOKEN, 64>(prm, grid, smem, s);
+  return launch_rtn_decode_v<PAGE, RTN_TOKEN, 128>(prm, grid, smem, s);
 }
 
 static int check_rtn_geom(const bmxk_rtn_geom* g, const char* who) {
@@ -430,7 +512,7 @@ size_t bmxk_rtn_page_block_bytes(const bmxk_rtn_geom* g) { return g ? (size_t)rt
 size_t bmxk_rtn_decode_workspace_bytes(const bmxk_rtn_geom* g, int batch, int max_pages) {
   if (!g || batch <= 0) return 0;
   (void)max_pages;
-  return 256 + ((size_t)num_sms() + (size_t)batch * g->h_kv) * g->n_q_groups * PART_STRIDE * sizeof(float);
+  return 256 + ((size_t)num_sms() * RTN_CTAS_PER_SM + (size_t)batch * g->h_kv) * g->n_q_groups * PART_STRIDE * sizeof(float);
 }
 
 int bmxk_rtn_append(const bmxk_rtn_geom* g, const void* k, const void* v, int src_dtype, int64_t stride_seq,
@@ -497,22 +579,21 @@ int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, co
   cudaStream_t s = (cudaStream_t)stream;
   float* part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + 256);
   const int64_t max_tiles = (int64_t)batch * g->h_kv * (((int64_t)max_pages * g->page + TILE_TOKENS - 1) / TILE_TOKENS);
-  const int grid = (int)(max_tiles < num_sms() ? (max_tiles < 1 ? 1 : max_tiles) : num_sms());
+  const int most = num_sms() * RTN_CTAS_PER_SM;
+  const int grid = (int)(max_tiles < most ? (max_tiles < 1 ? 1 : max_tiles) : most);
   const float scale_log2 = sm_scale * 1.4426950408889634f;
   if (max_pages > 0) {
     RtnDecodeParams prm;
     prm.g = to_rtn(g), prm.q = (const __half*)q, prm.pages = (const uint8_t*)pages, prm.page_table = page_table;
     prm.table_stride = table_stride, prm.n_pages = n_pages, prm.batch = batch, prm.scale_log2 = scale_log2, prm.part = part;
-    const size_t smem = (size_t)(8 * 8 * HEAD_DIM + 128) * 4 + (size_t)(2 * batch + 1) * 4 + 16;
-    static PerDeviceOnce configured;
-    if (configured.first()) {
-      cudaFuncSetAttribute(rtn_decode_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-      cudaFuncSetAttribute(rtn_decode_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    }
-    BMXK_REQUIRE(smem <= 96 * 1024, "bmxk_rtn_decode: batch too large");
-    if (g->page == 128) rtn_decode_kernel<128><<<grid, 256, smem, s>>>(prm);
-    else rtn_decode_kernel<64><<<grid, 256, smem, s>>>(prm);
-    rc = check_launch("bmxk_rtn_decode");
+    prm.status = reinterpret_cast<int32_t*>(workspace);
+    // the ring takes what two CTAs per SM leave of the 227 KB; batches of thousands of sequences (page counts in shared memory) get a
+    // shorter ring, never fewer than two stages
+    const size_t fixed = RTN_FIXED_SMEM + (size_t)(2 * batch + 1) * 4 + 16, stage = (size_t)rtn_block_bytes(prm.g) * (TILE_TOKENS / g->page);
+    prm.n_stages = 2;
+    while (prm.n_stages < RTN_MAX_STAGES && fixed + (prm.n_stages + 1) * stage <= 112 * 1024) ++prm.n_stages;
+    const size_t smem = fixed + prm.n_stages * stage;
+    rc = g->page == 128 ? launch_rtn_decode_k<128>(prm, grid, smem, s) : launch_rtn_decode_k<64>(prm, grid, smem, s);
     if (rc) return rc;
   }
   K2bMergeParams mp;

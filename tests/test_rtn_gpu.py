@@ -183,3 +183,46 @@ def test_reference_golden_rtn():
                      k_tail.to(dev), v_tail.to(dev), torch.tensor([tl], dtype=torch.int32, device=dev), 1.0 / math.sqrt(D), ws, out=out)
         torch.cuda.synchronize()
         _close(out.cpu().numpy(), c[want][:, 0, :][None])
+
+
+@pytest.mark.parametrize("page", [64, 128])
+@pytest.mark.parametrize("arm,k_group", [("rtn_channel", 32), ("rtn_channel", 64), ("rtn_channel", 128), ("rtn_token", 32), ("rtn_token", 64), ("rtn_token", 128)])
+@pytest.mark.parametrize("v_group", [32, 64, 128])
+def test_decode_every_kernel_variant_over_many_tiles(page, arm, k_group, v_group):
+    """Each instantiation of the decode kernel with more tiles per CTA than its copy ring has stages (ranges that cross heads and
+    sequences, ragged page counts, an empty sequence, a half-filled last tile), against float32 attention over the exported
+    dequantized pages; queries and keys scaled by opposite powers of two must give the same attention.  Bar: 2e-3 of the largest
+    output, the one of the other decode tests (fp16 rounding of scaled queries and of weights, 2^-11 each)."""
+    from bmx_b200 import kernels as K
+
+    if arm == "rtn_channel" and k_group > page:
+        pytest.skip("a token group never spans pages")
+    dev = torch.device("cuda:0")
+    h_kv, G, B, max_pages = 4, 3, 9, 61 if page == 128 else 121
+    g = K.rtn_geom(h_kv, G, page, arm, k_group, v_group, 3, 2)
+    gen = torch.Generator(device=dev).manual_seed(page + k_group + v_group)
+    T = max_pages * page
+    k = torch.randn(B, h_kv, T, 128, generator=gen, device=dev).half()
+    v = torch.randn(B, h_kv, T, 128, generator=gen, device=dev).half()
+    q = torch.randn(B, h_kv * G, 128, generator=gen, device=dev).half()
+    table = torch.randperm(B * max_pages, generator=gen, device=dev).to(torch.int32).view(B, max_pages)
+    n_pages = torch.tensor([max_pages, 1, 0, max_pages - 1, 7, 2, max_pages, 3, max_pages - 4], dtype=torch.int32, device=dev)
+    k_tail, v_tail = k[:, :, :32].contiguous(), v[:, :, :32].contiguous()
+    tail_len = torch.full((B,), 32, dtype=torch.int32, device=dev)
+    for ks in (1.0, 2.0 ** -8, 2.0 ** 8):
+        pool = K.RtnPool(g, B * max_pages, dev)
+        K.rtn_append(pool, k * ks, v, table.reshape(-1).contiguous(), max_pages)
+        ws = K.rtn_workspace(g, B, max_pages, dev)
+        out = K.rtn_decode(pool, (q / ks).half(), table, n_pages, max_pages, (k_tail * ks).half(), v_tail, tail_len, 128 ** -0.5, ws)
+        K.check_status(ws)
+        ex = K.rtn_export(pool, table.reshape(-1).contiguous(), dequant=True)
+        kd = ex["k_deq"].view(B, T, h_kv, 128).permute(0, 2, 1, 3)
+        vd = ex["v_deq"].view(B, T, h_kv, 128).permute(0, 2, 1, 3)
+        for b in range(B):
+            n = int(n_pages[b]) * page
+            kk = torch.cat([kd[b, :, :n], k_tail[b].float() * ks], 1)
+            vv = torch.cat([vd[b, :, :n], v_tail[b].float()], 1)
+            s = torch.einsum("hgd,htd->hgt", q[b].float().view(h_kv, G, 128) / ks, kk) * 128 ** -0.5
+            ref = torch.einsum("hgt,htd->hgd", torch.softmax(s, -1), vv).reshape(h_kv * G, 128)
+            err = float((out[b].float() - ref).abs().max() / ref.abs().max())
+            assert err < 2e-3, f"scale {ks}, sequence {b}: {err:.2e}"
