@@ -5,24 +5,45 @@
 //   (bmx: src/bmx/cache/codecs.py:616-636)
 // Block per (slot, head), 4352 bytes: [ V codes, 4096 B | V norms, 128 fp16 ], both in the "row order" of
 // the k2b page block (layout.cuh, layout 1), so that the tcgen05 decode kernels read either pool alike.
-// Compiled with -fmad=false; the arithmetic is the one of k2b_quant_page_kernel, step for step.
-#include "common.cuh"
+// Compiled with -fmad=false; the codes are those of quant_value_token (value_quant.cuh), step for step.
+#include "value_quant.cuh"
 
 namespace bmxk {
 
 constexpr int VBLOCK_BYTES = 128 * 32 + 128 * 2;
 
+// 16-bit sources.  One block of 256 threads per (item, head); see value_quant.cuh for what bounds it.  Measured, 2048 blocks (four
+// sequences of 8192 tokens x 8 heads, fp16): 85 -> 40 us for the values of a spectral append.
 template <typename T>
-__global__ void __launch_bounds__(128) vblock_quant_kernel(int h_kv, const T* __restrict__ v, int64_t stride_seq, int64_t stride_head,
-                                                           int64_t stride_tok, const float* __restrict__ signs,
-                                                           const float* __restrict__ codebook, const int32_t* __restrict__ slots,
-                                                           int n_pages, uint8_t* __restrict__ vpages) {
+__global__ void __launch_bounds__(VQ_THREADS, 2) vblock_quant_kernel(int h_kv, const T* __restrict__ v, int64_t stride_seq,
+                                                                     int64_t stride_head, int64_t stride_tok,
+                                                                     const float* __restrict__ signs, const float* __restrict__ codebook,
+                                                                     const int32_t* __restrict__ slots, int n_pages,
+                                                                     uint8_t* __restrict__ vpages, int vec16) {
+  __shared__ __align__(16) uint8_t smem[VQ_SMEM_BYTES];
+  uint32_t* words = reinterpret_cast<uint32_t*>(smem + VQ_STAGE_BYTES);
+  float* norms = reinterpret_cast<float*>(smem + VQ_STAGE_BYTES + VQ_WORDS_BYTES);
+  uint32_t* redo = reinterpret_cast<uint32_t*>(norms + 128);
+  const int item = blockIdx.x / h_kv, h = blockIdx.x % h_kv;
+  const int seq = item / n_pages, pg = item % n_pages, tid = threadIdx.x;
+  uint8_t* blk = vpages + ((int64_t)slots[item] * h_kv + h) * VBLOCK_BYTES;
+  vq_stage<T>(v + seq * stride_seq + h * stride_head + (int64_t)pg * 128 * stride_tok, stride_tok, vec16 != 0, smem, tid);
+  vq_quant_page<T>(smem, words, norms, redo, signs, codebook, reinterpret_cast<__half*>(blk + 128 * 32), tid);
+  __syncthreads();
+  for (int w = tid; w < 1024; w += VQ_THREADS) reinterpret_cast<uint32_t*>(blk)[w] = words[w];
+}
+
+// float32 sources: every token by the exact sequence (the products of value_quant.cuh are exact for 16-bit sources only).
+__global__ void __launch_bounds__(128) vblock_quant_f32_kernel(int h_kv, const float* __restrict__ v, int64_t stride_seq, int64_t stride_head,
+                                                               int64_t stride_tok, const float* __restrict__ signs,
+                                                               const float* __restrict__ codebook, const int32_t* __restrict__ slots,
+                                                               int n_pages, uint8_t* __restrict__ vpages) {
   __shared__ __align__(16) uint8_t vcode[128 * HEAD_DIM];  // [token][channel]
   const int item = blockIdx.x / h_kv, h = blockIdx.x % h_kv;
   const int seq = item / n_pages, pg = item % n_pages;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint8_t* blk = vpages + ((int64_t)slots[item] * h_kv + h) * VBLOCK_BYTES;
-  const T* vsrc = v + seq * stride_seq + h * stride_head + (int64_t)pg * 128 * stride_tok;
+  const float* vsrc = v + seq * stride_seq + h * stride_head + (int64_t)pg * 128 * stride_tok;
   const float c0 = codebook[0], c1 = codebook[1], c2 = codebook[2], c3 = codebook[3];
   const float m0 = (c0 + c1) / 2.f, m1 = (c1 + c2) / 2.f, m2 = (c2 + c3) / 2.f;
   float sg[4];
@@ -30,26 +51,10 @@ __global__ void __launch_bounds__(128) vblock_quant_kernel(int h_kv, const T* __
   for (int k = 0; k < 4; ++k) sg[k] = signs[4 * lane + k];
   __half* vnorm = reinterpret_cast<__half*>(blk + 128 * 32);
   for (int r = warp; r < 128; r += 4) {  // warp = token
-    float x[4];
+    float x[4], n;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x[k] = load_as_float<T>(vsrc + r * stride_tok + 4 * lane + k);
-    float ss = 0.f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) ss = fmaf(x[k], x[k], ss);
-#pragma unroll
-    for (int m = 16; m >= 1; m >>= 1) ss = ss + __shfl_xor_sync(0xffffffffu, ss, m);
-    const float n = __half2float(__float2half_rn(fmaxf(sqrtf(ss), 1e-12f)));
-#pragma unroll
-    for (int k = 0; k < 4; ++k) x[k] = (x[k] / n) * sg[k];
-    fwht128_warp(x, lane);
-    const float sqrt_d = 11.313708498984761f;
-    uint32_t packed4 = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float y = x[k] * sqrt_d;
-      packed4 |= (uint32_t)((y > m0) + (y > m1) + (y > m2)) << (8 * k);
-    }
-    *reinterpret_cast<uint32_t*>(vcode + r * HEAD_DIM + 4 * lane) = packed4;
+    for (int k = 0; k < 4; ++k) x[k] = vsrc[r * stride_tok + 4 * lane + k];
+    *reinterpret_cast<uint32_t*>(vcode + r * HEAD_DIM + 4 * lane) = quant_value_token(x, sg, m0, m1, m2, lane, n);
     if (lane == 0) vnorm[r] = __float2half_rn(n);
   }
   __syncthreads();
@@ -105,15 +110,17 @@ int bmxk_vblock_append(int h_kv, const void* v, int src_dtype, int64_t stride_se
   BMXK_REQUIRE((int64_t)n_seq * n_pages * h_kv < (1LL << 31), "bmxk_vblock_append: too many pages in one call");
   const int blocks = n_seq * n_pages * h_kv;
   cudaStream_t s = (cudaStream_t)stream;
+  // sixteen-byte loads need every row start aligned to them (16-bit sources)
+  const int vec16 = (uintptr_t)v % 16 == 0 && (n_seq == 1 || stride_seq % 8 == 0) && (h_kv == 1 || stride_head % 8 == 0) && stride_tok % 8 == 0;
   if (src_dtype == BMXK_DTYPE_F16)
-    vblock_quant_kernel<__half><<<blocks, 128, 0, s>>>(h_kv, (const __half*)v, stride_seq, stride_head, stride_tok, signs, codebook,
-                                                        slots, n_pages, (uint8_t*)vpages);
+    vblock_quant_kernel<__half><<<blocks, VQ_THREADS, 0, s>>>(h_kv, (const __half*)v, stride_seq, stride_head, stride_tok, signs, codebook,
+                                                               slots, n_pages, (uint8_t*)vpages, vec16);
   else if (src_dtype == BMXK_DTYPE_BF16)
-    vblock_quant_kernel<__nv_bfloat16><<<blocks, 128, 0, s>>>(h_kv, (const __nv_bfloat16*)v, stride_seq, stride_head, stride_tok, signs,
-                                                               codebook, slots, n_pages, (uint8_t*)vpages);
+    vblock_quant_kernel<__nv_bfloat16><<<blocks, VQ_THREADS, 0, s>>>(h_kv, (const __nv_bfloat16*)v, stride_seq, stride_head, stride_tok, signs,
+                                                                      codebook, slots, n_pages, (uint8_t*)vpages, vec16);
   else if (src_dtype == BMXK_DTYPE_F32)
-    vblock_quant_kernel<float><<<blocks, 128, 0, s>>>(h_kv, (const float*)v, stride_seq, stride_head, stride_tok, signs, codebook, slots,
-                                                       n_pages, (uint8_t*)vpages);
+    vblock_quant_f32_kernel<<<blocks, 128, 0, s>>>(h_kv, (const float*)v, stride_seq, stride_head, stride_tok, signs, codebook, slots, n_pages,
+                                                   (uint8_t*)vpages);
   else {
     set_error("bmxk_vblock_append: unknown src_dtype %d", src_dtype);
     return BMXK_ERR_INVALID;
