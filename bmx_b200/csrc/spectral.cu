@@ -12,7 +12,7 @@
 // [direction][page / group].  Sums run in ascending index order with one accumulator (fmaf for the two
 // matrix products; separate multiply and add inside the step refinement, as the reference does), which
 // makes the result independent of launch shape.  Compiled with -fmad=false.
-#include "common.cuh"
+#include "value_quant.cuh"
 
 namespace bmxk {
 
@@ -22,64 +22,255 @@ struct SpectralGeom {
 
 __device__ __forceinline__ int container_bits(int b) { return b == 0 ? 0 : (b == 2 ? 2 : (b <= 4 ? 4 : 8)); }
 
-template <typename T>
-__global__ void __launch_bounds__(128) spectral_quant_page_kernel(SpectralGeom g, const T* __restrict__ k,
-                                                                  int64_t stride_seq, int64_t stride_head, int64_t stride_tok,
-                                                                  const float* __restrict__ enc, const int32_t* __restrict__ col_bits,
-                                                                  const int32_t* __restrict__ col_off, const int32_t* __restrict__ slots,
-                                                                  int n_pages, uint8_t* __restrict__ pages) {
+// Round-to-nearest-even of a float of magnitude below 2^22, as the low bits of (x + RINT_MAGIC); minus RINT_MAGIC: rintf(x).
+constexpr float RINT_MAGIC = 12582912.f;
+
+// code = clamp(rint(x / scale)) of two values, by the product with r = 1 / scale.  |x r - x / scale| <= 2^-23 |x r| and the true
+// division rounds by another 2^-24, so both round alike unless x r lies within (qmax + 2) 2^-22 of a half; `far` collects the
+// largest distance from the rounded value, and a caller that finds it above 0.5 - (qmax + 2) 2^-22 divides instead.  (Values
+// clamped to -qmax - 1 or qmax are at distance 0.)
+__device__ __forceinline__ F2 codes_by_product(F2 x, F2 r, float lo, float hi, float& far) {
+  const F2 magic = f2_pack(RINT_MAGIC, RINT_MAGIC), unmagic = f2_pack(-RINT_MAGIC, -RINT_MAGIC), minus1 = f2_pack(-1.f, -1.f);
+  float t0, t1, d0, d1;
+  f2_unpack(f2_mul(x, r), t0, t1);
+  const F2 t = f2_pack(fminf(fmaxf(t0, lo), hi), fminf(fmaxf(t1, lo), hi));
+  const F2 q = f2_add(f2_add(t, magic), unmagic);
+  f2_unpack(f2_fma(q, minus1, t), d0, d1);
+  far = fmaxf(far, fmaxf(fabsf(d0), fabsf(d1)));
+  return q;
+}
+__device__ __forceinline__ float code_by_division(float x, float scale, float lo, float hi) { return fminf(fmaxf(rintf(x / scale), lo), hi); }
+
+// One block of 256 threads per (item, head), two blocks per SM.
+// What bounds it: the fp32 pipe.  Y = M @ enc is 2 million fused multiply-adds per block that have to stay float32 sums in ascending
+// order (the scales are float32 numbers derived from every value), the refinement about seven fp32 operations per value and round.
+//   encode      keys transposed in shared memory, 32 encoder rows at a time beside them (the next 32 travel in registers); a warp
+//               owns 16 of the directions that carry bits (the others are never computed), a thread PAGE / 16 rows x 8 directions.
+//   refinement  thread = (direction, token group), num and den in the reference's order (den is a sum of small integers: exact in any).
+//               A round whose scale comes out as it went in is a fixed point: the remaining rounds would repeat it and are skipped.
+//               Divisions become products with the reciprocal (codes_by_product); rounds with a value near a half divide.
+// Measured, 2048 blocks (four sequences of 8192 tokens x 8 heads, 104 of 128 directions with bits, groups of 64): @@SQ@@
+constexpr int SQ_THREADS = 256, SQ_CHUNK = 32;
+__host__ __device__ constexpr int sq_stride(int page) { return page + 4; }  // floats per channel row: 128-bit reads of consecutive rows hit distinct banks
+__host__ __device__ constexpr int sq_smem(int page) { return (HEAD_DIM * sq_stride(page) + 2 * SQ_CHUNK * HEAD_DIM + HEAD_DIM + 4) * 4; }
+
+template <typename T, int PAGE>
+__global__ void __launch_bounds__(SQ_THREADS, 2) spectral_quant_page_kernel(SpectralGeom g, const T* __restrict__ k, int64_t stride_seq,
+                                                                            int64_t stride_head, int64_t stride_tok,
+                                                                            const float* __restrict__ enc, const int32_t* __restrict__ col_bits,
+                                                                            const int32_t* __restrict__ col_off,
+                                                                            const int32_t* __restrict__ slots, int n_pages,
+                                                                            uint8_t* __restrict__ pages, int vec) {
   extern __shared__ __align__(16) uint8_t smem[];
-  float* Ms = reinterpret_cast<float*>(smem);  // [page][128] keys, then Y in place
+  constexpr int STR = sq_stride(PAGE), RPT = PAGE / 16, RB = PAGE / 32;
+  float* Ms = reinterpret_cast<float*>(smem);         // [128 channels][STR] keys, later [direction in the list][STR] Y
+  float* es = Ms + HEAD_DIM * STR;                     // [2][SQ_CHUNK][128] encoder rows, columns of the list
+  int* cols = reinterpret_cast<int*>(es + 2 * SQ_CHUNK * HEAD_DIM);  // directions with bits, ascending
+  int* n_used_sm = cols + HEAD_DIM;
   const int item = blockIdx.x / g.h_kv, h = blockIdx.x % g.h_kv;
-  const int seq = item / n_pages, pg = item % n_pages, page = g.page, j = threadIdx.x;
-  const T* src = k + seq * stride_seq + h * stride_head + (int64_t)pg * page * stride_tok;
-  for (int o = threadIdx.x; o < page * HEAD_DIM; o += 128) Ms[o] = load_as_float<T>(src + (o / HEAD_DIM) * stride_tok + o % HEAD_DIM);
-  __syncthreads();
-  const float* e = enc + (int64_t)h * HEAD_DIM * HEAD_DIM;
-  // Y[:, j]: thread j walks the rows; every thread reads the same key row (shared-memory broadcast)
-  float y[128];
-#pragma unroll 1
-  for (int r = 0; r < page; ++r) {
-    float acc = 0.f;
-    for (int c = 0; c < HEAD_DIM; ++c) acc = fmaf(Ms[r * HEAD_DIM + c], e[c * HEAD_DIM + j], acc);
-    y[r & 127] = acc;
+  const int seq = item / n_pages, pg = item % n_pages, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+  if (warp == 0) {  // the list of directions
+    int n = 0;
+#pragma unroll
+    for (int j0 = 0; j0 < HEAD_DIM; j0 += 32) {
+      const bool used = col_bits[h * HEAD_DIM + j0 + lane] != 0;
+      const uint32_t mask = __ballot_sync(0xffffffffu, used);
+      if (used) cols[n + __popc(mask & ((1u << lane) - 1u))] = j0 + lane;
+      n += __popc(mask);
+    }
+    if (lane == 0) *n_used_sm = n;
+  }
+  {  // keys: a lane takes 16 * RB channels of one row
+    const int r = 32 * (warp % RB) + lane, c_base = (warp / RB) * 16 * RB;
+    const T* src = k + seq * stride_seq + h * stride_head + ((int64_t)pg * PAGE + r) * stride_tok + c_base;
+#pragma unroll
+    for (int c0 = 0; c0 < 16 * RB; c0 += 32) {
+      float f[32];
+      if (vec) {
+        constexpr int PER = 16 / (int)sizeof(T);
+        uint4 u[32 / PER];
+#pragma unroll
+        for (int i = 0; i < 32 / PER; ++i) u[i] = *reinterpret_cast<const uint4*>(src + c0 + i * PER);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = load_as_float<T>(reinterpret_cast<const T*>(u) + i);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) f[i] = load_as_float<T>(src + c0 + i);
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) Ms[(c_base + c0 + i) * STR + r] = f[i];
+    }
   }
   __syncthreads();
-  for (int r = 0; r < page; ++r) Ms[r * HEAD_DIM + j] = y[r];
+  const int n_used = *n_used_sm;
+  const float* e = enc + (int64_t)h * HEAD_DIM * HEAD_DIM;
+  // ---- Y[:, list] ----
+  {
+    const int jl = tid & 127, cl = tid >> 7, col = jl < n_used ? cols[jl] : -1;
+    float nxt[16];
+    auto fetch = [&](int c0) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) nxt[i] = col >= 0 ? e[(c0 + cl + 2 * i) * HEAD_DIM + col] : 0.f;
+    };
+    auto put = [&](float* dst) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) dst[(cl + 2 * i) * HEAD_DIM + jl] = nxt[i];
+    };
+    const bool works = 16 * warp < n_used;
+    const int rg = lane & 15, j0 = 16 * warp + 8 * (lane >> 4);
+    float acc[RPT][8];
+#pragma unroll
+    for (int a = 0; a < RPT; ++a)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
+    fetch(0);
+    put(es);
+    __syncthreads();
+#pragma unroll 1
+    for (int c0 = 0; c0 < HEAD_DIM; c0 += SQ_CHUNK) {
+      const float* eb = es + ((c0 / SQ_CHUNK) & 1) * SQ_CHUNK * HEAD_DIM;
+      if (c0 + SQ_CHUNK < HEAD_DIM) fetch(c0 + SQ_CHUNK);
+      if (works) {
+#pragma unroll 4
+        for (int c = 0; c < SQ_CHUNK; ++c) {
+          float m[RPT], w[8];
+#pragma unroll
+          for (int a = 0; a < RPT; a += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(Ms + (c0 + c) * STR + RPT * rg + a);
+            m[a] = t.x, m[a + 1] = t.y, m[a + 2] = t.z, m[a + 3] = t.w;
+          }
+#pragma unroll
+          for (int b = 0; b < 8; b += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(eb + c * HEAD_DIM + j0 + b);
+            w[b] = t.x, w[b + 1] = t.y, w[b + 2] = t.z, w[b + 3] = t.w;
+          }
+#pragma unroll
+          for (int a = 0; a < RPT; ++a)
+#pragma unroll
+            for (int b = 0; b < 8; ++b) acc[a][b] = fmaf(m[a], w[b], acc[a][b]);
+        }
+      }
+      if (c0 + SQ_CHUNK < HEAD_DIM) put(es + (((c0 / SQ_CHUNK) + 1) & 1) * SQ_CHUNK * HEAD_DIM);
+      __syncthreads();  // the chunk read here is overwritten two rounds on; after the last one Y may replace the keys
+    }
+    if (works)
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+#pragma unroll
+        for (int a = 0; a < RPT; a += 4)
+          *reinterpret_cast<float4*>(Ms + (j0 + b) * STR + RPT * rg + a) = make_float4(acc[a][b], acc[a + 1][b], acc[a + 2][b], acc[a + 3][b]);
+  }
   __syncthreads();
-  const int b = col_bits[h * HEAD_DIM + j];
-  if (b == 0) return;
+  // ---- scales and codes: thread = (token group, direction) ----
   uint8_t* blk = pages + ((int64_t)slots[item] * g.h_kv + h) * g.block_bytes;
-  uint8_t* row = blk + col_off[h * HEAD_DIM + j];
-  float* scales = reinterpret_cast<float*>(blk + g.scale_off) + j * (page / g.group);
-  const float qmax = (float)((1 << (b - 1)) - 1);
-  const int cb = container_bits(b);
-  for (int grp = 0; grp < page / g.group; ++grp) {
-    const int r0 = grp * g.group;
+  const int n_grp = PAGE / g.group;
+  for (int q = tid; q < n_used * n_grp; q += SQ_THREADS) {
+    const int grp = q / n_used, jl = q - grp * n_used, j = cols[jl], r0 = grp * g.group;
+    const int b = col_bits[h * HEAD_DIM + j], cb = container_bits(b);
+    const float qmax = (float)((1 << (b - 1)) - 1), lo = -qmax - 1.f, hi = qmax, near_half = 0.5f - (qmax + 2.f) * 2.384185791015625e-7f;
+    const float* x = Ms + jl * STR + r0;
     float amax = 0.f;
-    for (int r = r0; r < r0 + g.group; ++r) amax = fmaxf(amax, fabsf(Ms[r * HEAD_DIM + j]));
+    for (int r = 0; r < g.group; r += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(x + r);
+      amax = fmaxf(fmaxf(fmaxf(amax, fabsf(t.x)), fmaxf(fabsf(t.y), fabsf(t.z))), fabsf(t.w));
+    }
     float scale = fmaxf(amax, 1e-12f) / qmax;
     for (int it = 0; it < 10; ++it) {
-      float num = 0.f, den = 0.f;
-      for (int r = r0; r < r0 + g.group; ++r) {
-        const float x = Ms[r * HEAD_DIM + j];
-        const float q = fminf(fmaxf(rintf(x / scale), -qmax - 1.f), qmax);
-        num = num + x * q;
-        den = den + q * q;
+      float num = 0.f, den = 0.f, far = 0.f;
+      const bool recip = scale < 1e30f;  // 1 / scale is a normal number
+      if (recip) {
+        const float inv = 1.f / scale;
+        const F2 r2 = f2_pack(inv, inv);
+        F2 d2 = f2_pack(0.f, 0.f);
+#pragma unroll 2
+        for (int r = 0; r < g.group; r += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(x + r);
+          const F2 xa = f2_pack(t.x, t.y), xb = f2_pack(t.z, t.w);
+          const F2 qa = codes_by_product(xa, r2, lo, hi, far), qb = codes_by_product(xb, r2, lo, hi, far);
+          float p0, p1, p2, p3;
+          f2_unpack(f2_mul(xa, qa), p0, p1), f2_unpack(f2_mul(xb, qb), p2, p3);
+          num = num + p0, num = num + p1, num = num + p2, num = num + p3;
+          d2 = f2_fma(qa, qa, d2), d2 = f2_fma(qb, qb, d2);
+        }
+        float e0, e1;
+        f2_unpack(d2, e0, e1);
+        den = e0 + e1;
       }
+      if (!recip || !(far < near_half)) {
+        num = den = 0.f;
+        for (int r = 0; r < g.group; ++r) {
+          const float c = code_by_division(x[r], scale, lo, hi);
+          num = num + x[r] * c;
+          den = den + c * c;
+        }
+      }
+      const float was = scale;
       scale = fmaxf(num / fmaxf(den, 1e-12f), 1e-12f);
+      if (scale == was) break;
     }
-    scales[grp] = scale;
-    for (int r = r0; r < r0 + g.group; r += 8 / cb) {
-      uint32_t byte = 0;
-      for (int u = 0; u < 8 / cb; ++u) {
-        const int q = (int)fminf(fmaxf(rintf(Ms[(r + u) * HEAD_DIM + j] / scale), -qmax - 1.f), qmax);
-        const uint32_t field = (b == 2 || b == 4) ? (uint32_t)(q + (1 << (b - 1))) : ((uint32_t)q & ((1u << cb) - 1u));
-        byte |= field << (cb * u);
+    reinterpret_cast<float*>(blk + g.scale_off)[j * n_grp + grp] = scale;
+    uint8_t* row = blk + col_off[h * HEAD_DIM + j] + r0 * cb / 8;
+    const float inv = 1.f / scale;
+    const F2 r2 = f2_pack(inv, inv), magic = f2_pack(RINT_MAGIC, RINT_MAGIC);
+    const uint32_t off = (b == 2 || b == 4) ? 1u << (b - 1) : 0u, mask = (1u << cb) - 1u;
+    const bool wide = ((uintptr_t)row & 7) == 0;
+    for (int r = 0; r < g.group; r += 8) {  // eight codes: cb bytes
+      F2 qv[4];
+      float far = 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) qv[u] = codes_by_product(f2_pack(x[r + 2 * u], x[r + 2 * u + 1]), r2, lo, hi, far);
+      if (!(scale < 1e30f) || !(far < near_half))
+#pragma unroll
+        for (int u = 0; u < 4; ++u) qv[u] = f2_pack(code_by_division(x[r + 2 * u], scale, lo, hi), code_by_division(x[r + 2 * u + 1], scale, lo, hi));
+      uint32_t w0 = 0, w1 = 0;  // codes 0..3 and 4..7, cb bits each
+#pragma unroll
+      for (int u = 3; u >= 0; --u) {
+        float a, c;
+        f2_unpack(f2_add(qv[u], magic), a, c);  // the code sits in the low bits
+        const uint32_t f0 = (__float_as_uint(a) + off) & mask, f1 = (__float_as_uint(c) + off) & mask;
+        uint32_t& w = u >= 2 ? w1 : w0;
+        w = (((w << cb) | f1) << cb) | f0;
       }
-      row[r * cb / 8] = (uint8_t)byte;
+      uint8_t* dst = row + r * cb / 8;
+      if (cb == 8) {
+        if (wide) *reinterpret_cast<uint2*>(dst) = make_uint2(w0, w1);
+        else
+          for (int i = 0; i < 8; ++i) dst[i] = (uint8_t)((i < 4 ? w0 : w1) >> (8 * (i & 3)));
+      } else {
+        const uint32_t w = w0 | (w1 << (4 * cb));
+        if (!wide)
+          for (int i = 0; i < cb; ++i) dst[i] = (uint8_t)(w >> (8 * i));
+        else if (cb == 4) *reinterpret_cast<uint32_t*>(dst) = w;
+        else *reinterpret_cast<uint16_t*>(dst) = (uint16_t)w;
+      }
     }
   }
+}
+
+template <typename T, int PAGE>
+static int launch_spectral_quant(const SpectralGeom& g, const T* k, int64_t ss, int64_t sh, int64_t st, const float* enc, const int32_t* col_bits,
+                                 const int32_t* col_off, const int32_t* slots, int blocks, int n_pages, uint8_t* pages, int vec, cudaStream_t s) {
+  static PerDeviceOnce configured;
+  if (configured.first()) {
+    const cudaError_t e = cudaFuncSetAttribute(spectral_quant_page_kernel<T, PAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sq_smem(PAGE));
+    if (e != cudaSuccess) {
+      configured.retract();
+      set_error("bmxk_spectral_append: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      return BMXK_ERR_CUDA;
+    }
+  }
+  spectral_quant_page_kernel<T, PAGE><<<blocks, SQ_THREADS, sq_smem(PAGE), s>>>(g, k, ss, sh, st, enc, col_bits, col_off, slots, n_pages, pages, vec);
+  return check_launch("bmxk_spectral_append");
+}
+template <typename T>
+static int spectral_append_impl(const SpectralGeom& g, const void* k, int64_t ss, int64_t sh, int64_t st, const float* enc, const int32_t* col_bits,
+                                const int32_t* col_off, const int32_t* slots, int n_seq, int n_pages, uint8_t* pages, cudaStream_t s) {
+  constexpr int64_t PER = 16 / sizeof(T);  // sixteen-byte loads need every row start aligned to them
+  const int vec = (uintptr_t)k % 16 == 0 && (n_seq == 1 || ss % PER == 0) && (g.h_kv == 1 || sh % PER == 0) && st % PER == 0;
+  const int blocks = n_seq * n_pages * g.h_kv;
+  if (g.page == 128) return launch_spectral_quant<T, 128>(g, (const T*)k, ss, sh, st, enc, col_bits, col_off, slots, blocks, n_pages, pages, vec, s);
+  return launch_spectral_quant<T, 64>(g, (const T*)k, ss, sh, st, enc, col_bits, col_off, slots, blocks, n_pages, pages, vec, s);
 }
 
 __device__ __forceinline__ int spectral_code(const uint8_t* row, int r, int b) {
@@ -154,30 +345,16 @@ int bmxk_spectral_append(const bmxk_spectral_geom* g, const void* k_pre, int src
   if (n_seq == 0 || n_pages == 0) return BMXK_OK;
   BMXK_REQUIRE(k_pre && enc && col_bits && col_off && slots && pages, "bmxk_spectral_append: null pointer");
   const SpectralGeom gg = to_s(g);
-  const int blocks = n_seq * n_pages * g->h_kv;
-  const size_t smem = (size_t)g->page * HEAD_DIM * 4;
   cudaStream_t s = (cudaStream_t)stream;
-  static PerDeviceOnce configured;
-  if (configured.first()) {
-    cudaFuncSetAttribute(spectral_quant_page_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    cudaFuncSetAttribute(spectral_quant_page_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    cudaFuncSetAttribute(spectral_quant_page_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-  }
+  uint8_t* dst = (uint8_t*)pages;
   if (src_dtype == BMXK_DTYPE_F16)
-    spectral_quant_page_kernel<__half><<<blocks, 128, smem, s>>>(gg, (const __half*)k_pre, stride_seq, stride_head, stride_tok, enc,
-                                                                  col_bits, col_off, slots, n_pages, (uint8_t*)pages);
-  else if (src_dtype == BMXK_DTYPE_BF16)
-    spectral_quant_page_kernel<__nv_bfloat16><<<blocks, 128, smem, s>>>(gg, (const __nv_bfloat16*)k_pre, stride_seq, stride_head,
-                                                                         stride_tok, enc, col_bits, col_off, slots, n_pages,
-                                                                         (uint8_t*)pages);
-  else if (src_dtype == BMXK_DTYPE_F32)
-    spectral_quant_page_kernel<float><<<blocks, 128, smem, s>>>(gg, (const float*)k_pre, stride_seq, stride_head, stride_tok, enc,
-                                                                 col_bits, col_off, slots, n_pages, (uint8_t*)pages);
-  else {
-    set_error("bmxk_spectral_append: unknown src_dtype %d", src_dtype);
-    return BMXK_ERR_INVALID;
-  }
-  return check_launch("bmxk_spectral_append");
+    return spectral_append_impl<__half>(gg, k_pre, stride_seq, stride_head, stride_tok, enc, col_bits, col_off, slots, n_seq, n_pages, dst, s);
+  if (src_dtype == BMXK_DTYPE_BF16)
+    return spectral_append_impl<__nv_bfloat16>(gg, k_pre, stride_seq, stride_head, stride_tok, enc, col_bits, col_off, slots, n_seq, n_pages, dst, s);
+  if (src_dtype == BMXK_DTYPE_F32)
+    return spectral_append_impl<float>(gg, k_pre, stride_seq, stride_head, stride_tok, enc, col_bits, col_off, slots, n_seq, n_pages, dst, s);
+  set_error("bmxk_spectral_append: unknown src_dtype %d", src_dtype);
+  return BMXK_ERR_INVALID;
 }
 
 int bmxk_spectral_dequant_pages(const bmxk_spectral_geom* g, const void* pages, const float* dec, const int32_t* col_bits,
