@@ -46,13 +46,17 @@ __device__ __forceinline__ float code_by_division(float x, float scale, float lo
 // order (the scales are float32 numbers derived from every value), the refinement about seven fp32 operations per value and round.
 //   encode      keys transposed in shared memory, 32 encoder rows at a time beside them (the next 32 travel in registers); a warp
 //               owns 16 of the directions that carry bits (the others are never computed), a thread PAGE / 16 rows x 8 directions.
-//   refinement  thread = (direction, token group), num and den in the reference's order (den is a sum of small integers: exact in any).
-//               A round whose scale comes out as it went in is a fixed point: the remaining rounds would repeat it and are skipped.
+//   refinement  thread = chain (direction, token group), num and den in the reference's order (den is a sum of small integers: exact
+//               in any).  A round whose scale comes out as it went in is a fixed point: the remaining rounds would repeat it and are
+//               skipped.  Chains need 3 to 10 rounds (mean 6), the slowest of 32 nearly always 10: after rounds 4, 6 and 8 the chains
+//               that still move are packed to the front of the block (after every round costs more in barriers than it saves).
 //               Divisions become products with the reciprocal (codes_by_product); rounds with a value near a half divide.
-// Measured, 2048 blocks (four sequences of 8192 tokens x 8 heads, 104 of 128 directions with bits, groups of 64): @@SQ@@
+// Measured, 2048 blocks (four sequences of 8192 tokens x 8 heads, 104 of 128 directions with bits, groups of 64), with the value half
+// (60 us): 968 -> 375 us; of the rest about 150 are the product (104 at the fp32 peak), 90 the refinement, 50 the loads, 20 the codes.
+// Packed fp32 pairs for the product (409 us: operand bandwidth), 64-row blocks at three or four per SM (397, 427 us) are slower.
 constexpr int SQ_THREADS = 256, SQ_CHUNK = 32;
 __host__ __device__ constexpr int sq_stride(int page) { return page + 4; }  // floats per channel row: 128-bit reads of consecutive rows hit distinct banks
-__host__ __device__ constexpr int sq_smem(int page) { return (HEAD_DIM * sq_stride(page) + 2 * SQ_CHUNK * HEAD_DIM + HEAD_DIM + 4) * 4; }
+__host__ __device__ constexpr int sq_smem(int page) { return (HEAD_DIM * sq_stride(page) + 2 * SQ_CHUNK * HEAD_DIM + 2 * HEAD_DIM + 16) * 4; }
 
 template <typename T, int PAGE>
 __global__ void __launch_bounds__(SQ_THREADS, 2) spectral_quant_page_kernel(SpectralGeom g, const T* __restrict__ k, int64_t stride_seq,
@@ -65,60 +69,57 @@ __global__ void __launch_bounds__(SQ_THREADS, 2) spectral_quant_page_kernel(Spec
   constexpr int STR = sq_stride(PAGE), RPT = PAGE / 16, RB = PAGE / 32;
   float* Ms = reinterpret_cast<float*>(smem);         // [128 channels][STR] keys, later [direction in the list][STR] Y
   float* es = Ms + HEAD_DIM * STR;                     // [2][SQ_CHUNK][128] encoder rows, columns of the list
-  int* cols = reinterpret_cast<int*>(es + 2 * SQ_CHUNK * HEAD_DIM);  // directions with bits, ascending
-  int* n_used_sm = cols + HEAD_DIM;
+  float* scale_s = es;                                 // [256] later: scales of the chains at hand,
+  uint8_t* list = reinterpret_cast<uint8_t*>(scale_s + SQ_THREADS);  // [2][256] and the chains that still move
+  int* cols = reinterpret_cast<int*>(es + 2 * SQ_CHUNK * HEAD_DIM);  // list of the directions with bits, ascending: direction | bits << 8
+  int* offs = cols + HEAD_DIM;                         // their code rows' byte offsets
+  int* moved = offs + HEAD_DIM;                        // [8] chains of each warp that still move (first: directions per warp)
   const int item = blockIdx.x / g.h_kv, h = blockIdx.x % g.h_kv;
   const int seq = item / n_pages, pg = item % n_pages, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-  if (warp == 0) {  // the list of directions
-    int n = 0;
-#pragma unroll
-    for (int j0 = 0; j0 < HEAD_DIM; j0 += 32) {
-      const bool used = col_bits[h * HEAD_DIM + j0 + lane] != 0;
-      const uint32_t mask = __ballot_sync(0xffffffffu, used);
-      if (used) cols[n + __popc(mask & ((1u << lane) - 1u))] = j0 + lane;
-      n += __popc(mask);
-    }
-    if (lane == 0) *n_used_sm = n;
-  }
+  // every global read that the rest waits for is issued here together
+  const int my_bits = tid < HEAD_DIM ? col_bits[h * HEAD_DIM + tid] : 0, my_off = tid < HEAD_DIM ? col_off[h * HEAD_DIM + tid] : 0;
+  uint8_t* blk = pages + ((int64_t)slots[item] * g.h_kv + h) * g.block_bytes;
   {  // keys: a lane takes 16 * RB channels of one row
     const int r = 32 * (warp % RB) + lane, c_base = (warp / RB) * 16 * RB;
     const T* src = k + seq * stride_seq + h * stride_head + ((int64_t)pg * PAGE + r) * stride_tok + c_base;
+    if (vec) {
+      constexpr int PER = 16 / (int)sizeof(T);
+      uint4 u[16 * RB / PER];
 #pragma unroll
-    for (int c0 = 0; c0 < 16 * RB; c0 += 32) {
-      float f[32];
-      if (vec) {
-        constexpr int PER = 16 / (int)sizeof(T);
-        uint4 u[32 / PER];
+      for (int i = 0; i < 16 * RB / PER; ++i) u[i] = *reinterpret_cast<const uint4*>(src + i * PER);
 #pragma unroll
-        for (int i = 0; i < 32 / PER; ++i) u[i] = *reinterpret_cast<const uint4*>(src + c0 + i * PER);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) f[i] = load_as_float<T>(reinterpret_cast<const T*>(u) + i);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) f[i] = load_as_float<T>(src + c0 + i);
-      }
-#pragma unroll
-      for (int i = 0; i < 32; ++i) Ms[(c_base + c0 + i) * STR + r] = f[i];
+      for (int i = 0; i < 16 * RB; ++i) Ms[(c_base + i) * STR + r] = load_as_float<T>(reinterpret_cast<const T*>(u) + i);
+    } else {
+#pragma unroll 8
+      for (int i = 0; i < 16 * RB; ++i) Ms[(c_base + i) * STR + r] = load_as_float<T>(src + i);
     }
   }
+  const uint32_t used_mask = __ballot_sync(0xffffffffu, my_bits != 0);
+  if (lane == 0) moved[warp] = __popc(used_mask);
   __syncthreads();
-  const int n_used = *n_used_sm;
+  const int n_used = moved[0] + moved[1] + moved[2] + moved[3];
+  if (my_bits != 0) {
+    int n = __popc(used_mask & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; ++w) n += moved[w];
+    cols[n] = tid | (my_bits << 8), offs[n] = my_off;
+  }
+  __syncthreads();
   const float* e = enc + (int64_t)h * HEAD_DIM * HEAD_DIM;
   // ---- Y[:, list] ----
   {
-    const int jl = tid & 127, cl = tid >> 7, col = jl < n_used ? cols[jl] : -1;
-    float nxt[16];
+    const int jl = tid & 127, cl = tid >> 7, col = jl < n_used ? cols[jl] & 0xFF : -1;
+    float nxt[SQ_CHUNK / 2];
     auto fetch = [&](int c0) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) nxt[i] = col >= 0 ? e[(c0 + cl + 2 * i) * HEAD_DIM + col] : 0.f;
+      for (int i = 0; i < SQ_CHUNK / 2; ++i) nxt[i] = col >= 0 ? e[(c0 + cl + 2 * i) * HEAD_DIM + col] : 0.f;
     };
     auto put = [&](float* dst) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) dst[(cl + 2 * i) * HEAD_DIM + jl] = nxt[i];
+      for (int i = 0; i < SQ_CHUNK / 2; ++i) dst[(cl + 2 * i) * HEAD_DIM + jl] = nxt[i];
     };
     const bool works = 16 * warp < n_used;
-    const int rg = lane & 15, j0 = 16 * warp + 8 * (lane >> 4);
+    const int rg = lane & 15, j0 = 16 * warp + 8 * (lane >> 4);  // rows 4 rg .. + 3 (and 64 + 4 rg ..): a quarter-warp reads 128 bytes on end
     float acc[RPT][8];
 #pragma unroll
     for (int a = 0; a < RPT; ++a)
@@ -132,12 +133,12 @@ __global__ void __launch_bounds__(SQ_THREADS, 2) spectral_quant_page_kernel(Spec
       const float* eb = es + ((c0 / SQ_CHUNK) & 1) * SQ_CHUNK * HEAD_DIM;
       if (c0 + SQ_CHUNK < HEAD_DIM) fetch(c0 + SQ_CHUNK);
       if (works) {
-#pragma unroll 4
+#pragma unroll 2
         for (int c = 0; c < SQ_CHUNK; ++c) {
           float m[RPT], w[8];
 #pragma unroll
           for (int a = 0; a < RPT; a += 4) {
-            const float4 t = *reinterpret_cast<const float4*>(Ms + (c0 + c) * STR + RPT * rg + a);
+            const float4 t = *reinterpret_cast<const float4*>(Ms + (c0 + c) * STR + 4 * rg + 16 * a);
             m[a] = t.x, m[a + 1] = t.y, m[a + 2] = t.z, m[a + 3] = t.w;
           }
 #pragma unroll
@@ -159,92 +160,138 @@ __global__ void __launch_bounds__(SQ_THREADS, 2) spectral_quant_page_kernel(Spec
       for (int b = 0; b < 8; ++b)
 #pragma unroll
         for (int a = 0; a < RPT; a += 4)
-          *reinterpret_cast<float4*>(Ms + (j0 + b) * STR + RPT * rg + a) = make_float4(acc[a][b], acc[a + 1][b], acc[a + 2][b], acc[a + 3][b]);
+          *reinterpret_cast<float4*>(Ms + (j0 + b) * STR + 4 * rg + 16 * a) = make_float4(acc[a][b], acc[a + 1][b], acc[a + 2][b], acc[a + 3][b]);
   }
   __syncthreads();
-  // ---- scales and codes: thread = (token group, direction) ----
-  uint8_t* blk = pages + ((int64_t)slots[item] * g.h_kv + h) * g.block_bytes;
+  // ---- scales and codes: chain = (token group, direction), up to 256 at a time ----
   const int n_grp = PAGE / g.group;
-  for (int q = tid; q < n_used * n_grp; q += SQ_THREADS) {
-    const int grp = q / n_used, jl = q - grp * n_used, j = cols[jl], r0 = grp * g.group;
-    const int b = col_bits[h * HEAD_DIM + j], cb = container_bits(b);
-    const float qmax = (float)((1 << (b - 1)) - 1), lo = -qmax - 1.f, hi = qmax, near_half = 0.5f - (qmax + 2.f) * 2.384185791015625e-7f;
-    const float* x = Ms + jl * STR + r0;
-    float amax = 0.f;
-    for (int r = 0; r < g.group; r += 4) {
-      const float4 t = *reinterpret_cast<const float4*>(x + r);
-      amax = fmaxf(fmaxf(fmaxf(amax, fabsf(t.x)), fmaxf(fabsf(t.y), fabsf(t.z))), fabsf(t.w));
+  for (int q0 = 0; q0 < n_used * n_grp; q0 += SQ_THREADS) {
+    const int n_here = min(SQ_THREADS, n_used * n_grp - q0);
+    if (tid < n_here) {
+      const int q = q0 + tid, grp = q / n_used, jl = q - grp * n_used, b = cols[jl] >> 8;
+      const float* x = Ms + jl * STR + grp * g.group;
+      float amax = 0.f;
+      for (int r = 0; r < g.group; r += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(x + r);
+        amax = fmaxf(fmaxf(fmaxf(amax, fabsf(t.x)), fmaxf(fabsf(t.y), fabsf(t.z))), fabsf(t.w));
+      }
+      scale_s[tid] = fmaxf(amax, 1e-12f) / (float)((1 << (b - 1)) - 1);
+      list[tid] = (uint8_t)tid;
     }
-    float scale = fmaxf(amax, 1e-12f) / qmax;
-    for (int it = 0; it < 10; ++it) {
-      float num = 0.f, den = 0.f, far = 0.f;
-      const bool recip = scale < 1e30f;  // 1 / scale is a normal number
-      if (recip) {
-        const float inv = 1.f / scale;
-        const F2 r2 = f2_pack(inv, inv);
-        F2 d2 = f2_pack(0.f, 0.f);
-#pragma unroll 2
-        for (int r = 0; r < g.group; r += 4) {
-          const float4 t = *reinterpret_cast<const float4*>(x + r);
-          const F2 xa = f2_pack(t.x, t.y), xb = f2_pack(t.z, t.w);
-          const F2 qa = codes_by_product(xa, r2, lo, hi, far), qb = codes_by_product(xb, r2, lo, hi, far);
-          float p0, p1, p2, p3;
-          f2_unpack(f2_mul(xa, qa), p0, p1), f2_unpack(f2_mul(xb, qb), p2, p3);
-          num = num + p0, num = num + p1, num = num + p2, num = num + p3;
-          d2 = f2_fma(qa, qa, d2), d2 = f2_fma(qb, qb, d2);
+    __syncthreads();
+    int n_act = n_here;
+    for (int seg = 0; seg < 4 && n_act > 0; ++seg) {  // rounds 0..3, 4..5, 6..7, 8..9
+      const uint8_t* cur = list + (seg & 1) * SQ_THREADS;
+      uint8_t* nxt = list + ((seg & 1) ^ 1) * SQ_THREADS;
+      bool moves = false;
+      int id = 0;
+      if (tid < n_act) {
+        id = cur[tid];
+        const int q = q0 + id, grp = q / n_used, jl = q - grp * n_used, b = cols[jl] >> 8;
+        const float qmax = (float)((1 << (b - 1)) - 1), lo = -qmax - 1.f, hi = qmax, near_half = 0.5f - (qmax + 2.f) * 2.384185791015625e-7f;
+        const float* x = Ms + jl * STR + grp * g.group;
+        float scale = scale_s[id];
+        moves = true;
+#pragma unroll 1
+        for (int it = seg ? 2 : 4; it > 0 && moves; --it) {
+          float num = 0.f, den = 0.f, far = 0.f;
+          const bool recip = scale < 1e30f;  // 1 / scale is a normal number
+          if (recip) {
+            const float inv = 1.f / scale;
+            const F2 r2 = f2_pack(inv, inv);
+            F2 d2 = f2_pack(0.f, 0.f);
+#pragma unroll 4
+            for (int r = 0; r < g.group; r += 4) {
+              const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(x + r);
+              F2 xa, xb;
+              xa.v = t.x, xb.v = t.y;
+              const F2 qa = codes_by_product(xa, r2, lo, hi, far), qb = codes_by_product(xb, r2, lo, hi, far);
+              float p0, p1, p2, p3;
+              f2_unpack(f2_mul(xa, qa), p0, p1), f2_unpack(f2_mul(xb, qb), p2, p3);
+              num = num + p0, num = num + p1, num = num + p2, num = num + p3;
+              d2 = f2_fma(qa, qa, d2), d2 = f2_fma(qb, qb, d2);
+            }
+            float e0, e1;
+            f2_unpack(d2, e0, e1);
+            den = e0 + e1;
+          }
+          if (!recip || !(far < near_half)) {
+            num = den = 0.f;
+            for (int r = 0; r < g.group; ++r) {
+              const float c = code_by_division(x[r], scale, lo, hi);
+              num = num + x[r] * c;
+              den = den + c * c;
+            }
+          }
+          const float now = fmaxf(num / fmaxf(den, 1e-12f), 1e-12f);
+          moves = now != scale;
+          scale = now;
         }
-        float e0, e1;
-        f2_unpack(d2, e0, e1);
-        den = e0 + e1;
+        scale_s[id] = scale;
       }
-      if (!recip || !(far < near_half)) {
-        num = den = 0.f;
-        for (int r = 0; r < g.group; ++r) {
-          const float c = code_by_division(x[r], scale, lo, hi);
-          num = num + x[r] * c;
-          den = den + c * c;
+      // the chains that moved, packed to the front: whole warps fall idle instead of waiting for their slowest lane
+      const uint32_t mask = __ballot_sync(0xffffffffu, moves);
+      if (lane == 0) moved[warp] = __popc(mask);
+      __syncthreads();
+      int before = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < SQ_THREADS / 32; ++w) {
+        const int m = moved[w];
+        before += w < warp ? m : 0, all += m;
+      }
+      if (moves) nxt[before + __popc(mask & ((1u << lane) - 1u))] = (uint8_t)id;
+      n_act = all;
+      __syncthreads();
+    }
+    if (tid < n_here) {
+      const int q = q0 + tid, grp = q / n_used, jl = q - grp * n_used, j = cols[jl] & 0xFF, r0 = grp * g.group;
+      const int b = cols[jl] >> 8, cb = container_bits(b);
+      const float qmax = (float)((1 << (b - 1)) - 1), lo = -qmax - 1.f, hi = qmax, near_half = 0.5f - (qmax + 2.f) * 2.384185791015625e-7f;
+      const float* x = Ms + jl * STR + r0;
+      const float scale = scale_s[tid];
+      reinterpret_cast<float*>(blk + g.scale_off)[j * n_grp + grp] = scale;
+      uint8_t* row = blk + offs[jl] + r0 * cb / 8;
+      const float inv = 1.f / scale;
+      const F2 r2 = f2_pack(inv, inv), magic = f2_pack(RINT_MAGIC, RINT_MAGIC);
+      const uint32_t off = (b == 2 || b == 4) ? 1u << (b - 1) : 0u, mask = (1u << cb) - 1u;
+      const bool wide = ((uintptr_t)row & 7) == 0;
+      for (int r = 0; r < g.group; r += 8) {  // eight codes: cb bytes
+        F2 qv[4];
+        float far = 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+          const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(x + r + 2 * u);
+          F2 xa, xb;
+          xa.v = t.x, xb.v = t.y;
+          qv[u] = codes_by_product(xa, r2, lo, hi, far), qv[u + 1] = codes_by_product(xb, r2, lo, hi, far);
+        }
+        if (!(scale < 1e30f) || !(far < near_half))
+#pragma unroll
+          for (int u = 0; u < 4; ++u) qv[u] = f2_pack(code_by_division(x[r + 2 * u], scale, lo, hi), code_by_division(x[r + 2 * u + 1], scale, lo, hi));
+        uint32_t w0 = 0, w1 = 0;  // codes 0..3 and 4..7, cb bits each
+#pragma unroll
+        for (int u = 3; u >= 0; --u) {
+          float a, c;
+          f2_unpack(f2_add(qv[u], magic), a, c);  // the code sits in the low bits
+          const uint32_t f0 = (__float_as_uint(a) + off) & mask, f1 = (__float_as_uint(c) + off) & mask;
+          uint32_t& w = u >= 2 ? w1 : w0;
+          w = (((w << cb) | f1) << cb) | f0;
+        }
+        uint8_t* dst = row + r * cb / 8;
+        if (cb == 8) {
+          if (wide) *reinterpret_cast<uint2*>(dst) = make_uint2(w0, w1);
+          else
+            for (int i = 0; i < 8; ++i) dst[i] = (uint8_t)((i < 4 ? w0 : w1) >> (8 * (i & 3)));
+        } else {
+          const uint32_t w = w0 | (w1 << (4 * cb));
+          if (!wide)
+            for (int i = 0; i < cb; ++i) dst[i] = (uint8_t)(w >> (8 * i));
+          else if (cb == 4) *reinterpret_cast<uint32_t*>(dst) = w;
+          else *reinterpret_cast<uint16_t*>(dst) = (uint16_t)w;
         }
       }
-      const float was = scale;
-      scale = fmaxf(num / fmaxf(den, 1e-12f), 1e-12f);
-      if (scale == was) break;
     }
-    reinterpret_cast<float*>(blk + g.scale_off)[j * n_grp + grp] = scale;
-    uint8_t* row = blk + col_off[h * HEAD_DIM + j] + r0 * cb / 8;
-    const float inv = 1.f / scale;
-    const F2 r2 = f2_pack(inv, inv), magic = f2_pack(RINT_MAGIC, RINT_MAGIC);
-    const uint32_t off = (b == 2 || b == 4) ? 1u << (b - 1) : 0u, mask = (1u << cb) - 1u;
-    const bool wide = ((uintptr_t)row & 7) == 0;
-    for (int r = 0; r < g.group; r += 8) {  // eight codes: cb bytes
-      F2 qv[4];
-      float far = 0.f;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) qv[u] = codes_by_product(f2_pack(x[r + 2 * u], x[r + 2 * u + 1]), r2, lo, hi, far);
-      if (!(scale < 1e30f) || !(far < near_half))
-#pragma unroll
-        for (int u = 0; u < 4; ++u) qv[u] = f2_pack(code_by_division(x[r + 2 * u], scale, lo, hi), code_by_division(x[r + 2 * u + 1], scale, lo, hi));
-      uint32_t w0 = 0, w1 = 0;  // codes 0..3 and 4..7, cb bits each
-#pragma unroll
-      for (int u = 3; u >= 0; --u) {
-        float a, c;
-        f2_unpack(f2_add(qv[u], magic), a, c);  // the code sits in the low bits
-        const uint32_t f0 = (__float_as_uint(a) + off) & mask, f1 = (__float_as_uint(c) + off) & mask;
-        uint32_t& w = u >= 2 ? w1 : w0;
-        w = (((w << cb) | f1) << cb) | f0;
-      }
-      uint8_t* dst = row + r * cb / 8;
-      if (cb == 8) {
-        if (wide) *reinterpret_cast<uint2*>(dst) = make_uint2(w0, w1);
-        else
-          for (int i = 0; i < 8; ++i) dst[i] = (uint8_t)((i < 4 ? w0 : w1) >> (8 * (i & 3)));
-      } else {
-        const uint32_t w = w0 | (w1 << (4 * cb));
-        if (!wide)
-          for (int i = 0; i < cb; ++i) dst[i] = (uint8_t)(w >> (8 * i));
-        else if (cb == 4) *reinterpret_cast<uint32_t*>(dst) = w;
-        else *reinterpret_cast<uint16_t*>(dst) = (uint16_t)w;
-      }
-    }
+    __syncthreads();  // the next 256 chains take over the lists
   }
 }
 
