@@ -19,7 +19,7 @@
 // The channel bits are dealt out for 16-byte operand loads: bits 0, 1, 3, 4 are the 16-point part (pair, operand half, lane of
 // the quad), bits 2, 5, 6 the 8-point part.
 #pragma once
-#include "common.cuh"
+#include "f32x2.cuh"
 
 namespace bmxk {
 
@@ -80,32 +80,6 @@ template <>
 struct VqOne<__half> { static constexpr uint32_t bits = 0x3C00u; };
 template <>
 struct VqOne<__nv_bfloat16> { static constexpr uint32_t bits = 0x3F80u; };
-
-// two floats per 64-bit register: one instruction for both (each rounds as the scalar operation does)
-struct F2 {
-  unsigned long long v;
-};
-__device__ __forceinline__ F2 f2_pack(float a, float b) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-  F2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
 
 // Stages the page (128 rows of 128 elements, stride_tok apart).  vec16: rows start on 16-byte boundaries.
 template <typename T>

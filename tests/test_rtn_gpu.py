@@ -226,3 +226,62 @@ def test_decode_every_kernel_variant_over_many_tiles(page, arm, k_group, v_group
             ref = torch.einsum("hgt,htd->hgd", torch.softmax(s, -1), vv).reshape(h_kv * G, 128)
             err = float((out[b].float() - ref).abs().max() / ref.abs().max())
             assert err < 2e-3, f"scale {ks}, sequence {b}: {err:.2e}"
+
+
+def _rtn_codes(x, bits, group, dim):
+    """Codes and float32 scales along `dim` of x (CPU float32): the reference's divisions and roundings."""
+    qmax = 2 ** (bits - 1) - 1
+    x = x.movedim(dim, -1)
+    t = x.reshape(*x.shape[:-1], x.shape[-1] // group, group)
+    am = torch.where(torch.isnan(t), torch.zeros_like(t), t.abs()).amax(-1, keepdim=True)
+    scale = am.clamp_min(1e-12) / qmax
+    q = torch.round(t / scale)
+    q = torch.where(torch.isnan(q), torch.full_like(q, -qmax - 1), q).clamp(-qmax - 1, qmax)
+    return q.reshape(x.shape).movedim(-1, dim).to(torch.int8), scale.squeeze(-1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("page,arm,k_group,v_group,kbits", [
+    (128, "rtn_channel", 64, 64, 2), (128, "rtn_channel", 32, 128, 4), (128, "rtn_channel", 128, 32, 3), (128, "rtn_token", 32, 64, 4),
+    (128, "rtn_token", 128, 128, 2), (64, "rtn_channel", 32, 32, 3), (64, "rtn_channel", 64, 64, 4), (64, "rtn_token", 64, 32, 2)])
+@pytest.mark.parametrize("kind", ["normal", "ties", "extremes"])
+def test_append_codes_equal_the_divided_ones(dtype, page, arm, k_group, v_group, kbits, kind):
+    """Every code and scale of the page quantizer, whose divisions are products with the inverse scale, equals the divided one, ties,
+    zeros, infinities and NaN included; also from rows that start off the sixteen-byte boundaries."""
+    from bmx_b200 import kernels as K
+
+    dev = torch.device("cuda:0")
+    n, h, pages = 2, 3, 3
+    T = pages * page
+    gen = torch.Generator().manual_seed(page + k_group + kbits)
+    k, v = torch.randn(n, h, T, 128, generator=gen), torch.randn(n, h, T, 128, generator=gen)
+    if kind == "ties":  # a coarse grid: quotients fall on halves
+        k, v = torch.randint(-7, 8, k.shape, generator=gen) * 0.5, torch.randint(-3, 4, v.shape, generator=gen) * 0.25
+    elif kind == "extremes":
+        for x in (k, v):
+            x[:, :, 3::17] = 0
+            x[:, :, 5::19] *= 1e-7
+            x[:, :, 7::23] *= 3e4 if dtype == torch.float16 else 1e35
+            x[0, 0, 11, 5], x[0, 1, 40, 77], x[1, 2, 70, 127] = float("inf"), float("nan"), float("-inf")
+    k, v = k.to(dtype), v.to(dtype)
+    g = K.rtn_geom(h, 4, page, arm, k_group, v_group, kbits, 2)
+    slots = torch.arange(n * pages, dtype=torch.int32, device=dev)
+    pools = [K.RtnPool(g, n * pages, dev) for _ in range(2)]
+    K.rtn_append(pools[0], k.to(dev), v.to(dev), slots, pages)
+    wide = torch.zeros(2, n, h, T, 128 + 3, dtype=dtype)
+    wide[0, ..., 1:129], wide[1, ..., 1:129] = k, v
+    wide = wide.to(dev)
+    K.rtn_append(pools[1], wide[0, ..., 1:129], wide[1, ..., 1:129], slots, pages)
+    assert torch.equal(pools[0].pages, pools[1].pages)
+    ex = {name: t.cpu() for name, t in K.rtn_export(pools[0], slots).items()}
+    kk = k.float().view(n, h, pages, page, 128).permute(0, 2, 1, 3, 4).reshape(n * pages, h, page, 128)
+    vv = v.float().view(n, h, pages, page, 128).permute(0, 2, 1, 3, 4).reshape(n * pages, h, page, 128)
+    vc, vs = _rtn_codes(vv, 2, v_group, 3)
+    assert torch.equal(ex["v_codes"], vc) and torch.equal(ex["v_scales"].view(torch.int16), vs.half().view(torch.int16))
+    if arm == "rtn_token":
+        kc, ks = _rtn_codes(kk, kbits, k_group, 3)
+        assert torch.equal(ex["k_codes"], kc) and torch.equal(ex["k_scales"].view(torch.int16), ks.half().view(torch.int16))
+    else:
+        kc, ks = _rtn_codes(kk, kbits, k_group, 2)  # codes (items, h, page, 128), scales (items, h, 128, groups)
+        assert torch.equal(ex["k_codes"], kc.transpose(2, 3).reshape(n * pages, h * 128, page))
+        assert torch.equal(ex["k_scales"].view(torch.int16), ks.half().reshape(n * pages, h * 128, -1).view(torch.int16))
