@@ -39,8 +39,10 @@ BMXK_HD int rtn_block_bytes(const RtnGeom& g) { return rtn_off_vscale(g) + g.pag
 // channel pairs of the word, codes are summed up at their bit position in float32 (offset binary, at most 16 bits: exact) and a final
 // XOR makes them two's complement: no byte codes, no second pass.
 // Divisions become products with 1 / scale: t = x (1 / scale) + offset differs from the true quotient, rounded, by at most
-// 4.2e-7 + 4.8e-7 + 4.2e-7, so both round alike unless t lies within RTN_NEAR of a half; a thread that sees such a value (or a
-// NaN) divides all of its values.  |x| <= absmax keeps the codes inside the clamp.
+// 4.2e-7 + 4.8e-7 + 4.2e-7, so both round alike unless t lies within RTN_NEAR of a half; the eight or sixteen values of a (half)
+// word that holds such a value (or a NaN) are divided.  With 16-bit sources exact halves are common (a value that is half of the
+// group's maximum: 4e-4 of the values of 2-bit codes), so it matters that no more than a word is done again.  |x| <= absmax keeps
+// the codes inside the clamp.
 // Measured, 4096 blocks (four sequences of 16384 tokens x 8 heads, 2-bit keys per channel, groups of 64, fp16): 417 -> 176 us.
 // ---------------------------------------------------------------------------------------------
 constexpr int RTNQ_THREADS = 256;
@@ -83,21 +85,23 @@ __device__ __forceinline__ F2 rtn_add_codes(F2 acc, float2 x, F2 inv, float offs
   far = max_nan(far, max_nan(fabsf(d0), fabsf(d1)));
   return f2_fma(q, f2_pack(weight, weight), acc);
 }
-__device__ __forceinline__ F2 rtn_add_codes_divided(F2 acc, float2 x, float2 scale, float qmax, float offset, float weight) {
-  const float a = fminf(fmaxf(rintf(x.x / scale.x), -qmax - 1.f), qmax) + offset, b = fminf(fmaxf(rintf(x.y / scale.y), -qmax - 1.f), qmax) + offset;
-  return f2_fma(f2_pack(a, b), f2_pack(weight, weight), acc);
-}
+// Out of line: it runs for about 1 % of the words.
+__device__ __noinline__ float rtn_code_divided(float x, float scale, float qmax) { return fminf(fmaxf(rintf(x / scale), -qmax - 1.f), qmax); }
 
 template <typename T, int PAGE>
 struct RtnQuantSmem {
-  static constexpr int ROW = HEAD_DIM * (int)sizeof(T) + 16;  // bytes per staged row: consecutive rows start four banks apart
+  static constexpr int ROW = HEAD_DIM * (int)sizeof(T);  // bytes per staged row; its 16-byte chunks are XORed with the row's low bits (rtn_at)
   static constexpr int SC = (PAGE / 32) * HEAD_DIM;            // scales: [token group][channel] or [row][4 channel groups], whichever is used
   static constexpr int SC_WORDS = SC > PAGE * 4 ? SC : PAGE * 4;
   static constexpr int BYTES = 2 * PAGE * ROW + 4 * SC_WORDS * 4;  // both pages, both scales and their inverses
 };
 
+// Byte `b` of staged row `r`: consecutive rows' equal chunks lie in different banks, and three blocks of 16-bit pages share an SM.
+template <int ROW>
+__device__ __forceinline__ int rtn_at(int r, int b) { return r * ROW + (b ^ ((r & 7) << 4)); }
+
 template <typename T, int PAGE>
-__global__ void __launch_bounds__(RTNQ_THREADS) rtn_quant_page_kernel(RtnGeom g, const T* __restrict__ k, const T* __restrict__ v,
+__global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quant_page_kernel(RtnGeom g, const T* __restrict__ k, const T* __restrict__ v,
                                                                       int64_t stride_seq, int64_t stride_head, int64_t stride_tok,
                                                                       const int32_t* __restrict__ slots, int n_pages,
                                                                       uint8_t* __restrict__ pages, int vec) {
@@ -133,15 +137,16 @@ __global__ void __launch_bounds__(RTNQ_THREADS) rtn_quant_page_kernel(RtnGeom g,
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const int o = i * RTNQ_THREADS + tid, r = o / PER_ROW, c = o % PER_ROW;
-      *reinterpret_cast<uint4*>(kst + r * ROW + c * 16) = a[i];
-      *reinterpret_cast<uint4*>(vst + r * ROW + c * 16) = b[i];
+      *reinterpret_cast<uint4*>(kst + rtn_at<ROW>(r, c * 16)) = a[i];
+      *reinterpret_cast<uint4*>(vst + rtn_at<ROW>(r, c * 16)) = b[i];
     }
   } else {
 #pragma unroll 8
     for (int o = tid; o < PAGE * HEAD_DIM; o += RTNQ_THREADS) {
       const int r = o >> 7, c = o & 127;
-      reinterpret_cast<T*>(kst + r * ROW)[c] = ksrc[r * stride_tok + c];
-      reinterpret_cast<T*>(vst + r * ROW)[c] = vsrc[r * stride_tok + c];
+      const int at = rtn_at<ROW>(r, c * (int)sizeof(T));
+      *reinterpret_cast<T*>(kst + at) = ksrc[r * stride_tok + c];
+      *reinterpret_cast<T*>(vst + at) = vsrc[r * stride_tok + c];
     }
   }
   __syncthreads();
@@ -151,11 +156,10 @@ __global__ void __launch_bounds__(RTNQ_THREADS) rtn_quant_page_kernel(RtnGeom g,
     constexpr int CH = 2 * (int)sizeof(T);  // sixteen-byte chunks of 32 channels
     for (int u = tid; u < PAGE * 4; u += RTNQ_THREADS) {
       const int r = u >> 2, qt = u & 3;
-      const uint4* p = reinterpret_cast<const uint4*>(st + r * ROW) + CH * qt;
       Pair m = Pair{};
 #pragma unroll
       for (int i = 0; i < CH; ++i) {
-        const uint4 w = p[(i + qt * (CH / 4)) & (CH - 1)];  // the four lanes of a row start in different banks
+        const uint4 w = *reinterpret_cast<const uint4*>(st + rtn_at<ROW>(r, 16 * (CH * qt + ((i + qt * (CH / 4)) & (CH - 1)))));  // the lanes of a row start in different banks
 #pragma unroll
         for (int e = 0; e < 16 / (int)sizeof(Pair); ++e) m = S::absmax(m, reinterpret_cast<const Pair*>(&w)[e]);
       }
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(RTNQ_THREADS) rtn_quant_page_kernel(RtnGeom g,
       const int c2 = u & 63, rb = u >> 6;
       Pair m = Pair{};
 #pragma unroll 16
-      for (int r = 0; r < 32; ++r) m = S::absmax(m, reinterpret_cast<const Pair*>(kst + (32 * rb + r) * ROW)[c2]);
+      for (int r = 0; r < 32; ++r) m = S::absmax(m, *reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(32 * rb + r, c2 * (int)sizeof(Pair))));
       const float2 mf = S::f(m);
       *reinterpret_cast<float2*>(ksc + rb * HEAD_DIM + 2 * c2) = mf;
     }
@@ -209,43 +213,33 @@ __global__ void __launch_bounds__(RTNQ_THREADS) rtn_quant_page_kernel(RtnGeom g,
 #pragma unroll
     for (int th = 0; th < 2; ++th) {
       const int r = 16 * wr + 8 * th + gg;
-      const Pair* p = reinterpret_cast<const Pair*>(kst + r * ROW) + t;
       const int chan = (r >> 5) * HEAD_DIM + 2 * t;
-      float far = 0.f;
+      auto pair = [&](int n) { return S::f(*reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(r, (4 * n + t) * (int)sizeof(Pair)))); };
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         F2 acc = f2_pack(8388608.f, 8388608.f);  // 2^23: the sum sits in the low bits
+        float far = 0.f;
         const float rs = g.k_arm == RTN_CHANNEL ? 0.f : kinv[4 * r + q];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           F2 inv;
-          if (g.k_arm == RTN_CHANNEL) {
-            inv.v = *reinterpret_cast<const unsigned long long*>(kinv + chan + 8 * (4 * q + i));
-          } else {
-            inv = f2_pack(rs, rs);
+          if (g.k_arm == RTN_CHANNEL) inv.v = *reinterpret_cast<const unsigned long long*>(kinv + chan + 8 * (4 * q + i));
+          else inv = f2_pack(rs, rs);
+          acc = rtn_add_codes(acc, pair(4 * q + i), inv, 8.f, (float)(1 << (4 * i)), far);
+        }
+        if (!(far < 0.5f - RTN_NEAR)) {
+          acc = f2_pack(8388608.f, 8388608.f);
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            const float2 x = pair(4 * q + i);
+            const float* sc = g.k_arm == RTN_CHANNEL ? ksc + chan + 8 * (4 * q + i) : ksc + 4 * r + q;
+            const float w = (float)(1 << (4 * i));
+            acc = f2_fma(f2_pack(rtn_code_divided(x.x, sc[0], kq) + 8.f, rtn_code_divided(x.y, sc[g.k_arm == RTN_CHANNEL], kq) + 8.f), f2_pack(w, w), acc);
           }
-          acc = rtn_add_codes(acc, S::f(p[4 * (4 * q + i)]), inv, 8.f, (float)(1 << (4 * i)), far);
         }
         float lo, hi;
         f2_unpack(acc, lo, hi);
         out[th][q] = prmt(__float_as_uint(lo), __float_as_uint(hi), 0x5410u) ^ 0x88888888u;
-      }
-      if (!(far < 0.5f - RTN_NEAR)) {
-#pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          F2 acc = f2_pack(8388608.f, 8388608.f);
-          for (int i = 0; i < 4; ++i) {
-            const float2 s = g.k_arm == RTN_CHANNEL ? *reinterpret_cast<const float2*>(ksc + chan + 8 * (4 * q + i)) : make_float2(ksc[4 * r + q], ksc[4 * r + q]);
-            acc = rtn_add_codes_divided(acc, S::f(p[4 * (4 * q + i)]), s, kq, 8.f, (float)(1 << (4 * i)));
-          }
-          float lo, hi;
-          f2_unpack(acc, lo, hi);
-          const uint32_t w = prmt(__float_as_uint(lo), __float_as_uint(hi), 0x5410u) ^ 0x88888888u;
-          if (q == 0) out[th][0] = w;
-          if (q == 1) out[th][1] = w;
-          if (q == 2) out[th][2] = w;
-          if (q == 3) out[th][3] = w;
-        }
       }
       uint32_t* dst = reinterpret_cast<uint32_t*>(blk) + ((wr * 2 + th) * 32 + 4 * gg + t) * 4;
       if (vec & 2) *reinterpret_cast<uint4*>(dst) = make_uint4(out[th][0], out[th][1], out[th][2], out[th][3]);
@@ -258,42 +252,39 @@ __global__ void __launch_bounds__(RTNQ_THREADS) rtn_quant_page_kernel(RtnGeom g,
   uint32_t* vout = reinterpret_cast<uint32_t*>(blk + rtn_off_vcode(g));
   for (int u = tid; u < PAGE * 2; u += RTNQ_THREADS) {
     const int wr = u >> 5, g2 = (u >> 3) & 3, t = (u >> 1) & 3, jh = u & 1;
-    const uint8_t* rows = vst + (16 * wr + 2 * t) * ROW;
-    const int srow = 4 * (16 * wr + 2 * t);
+    const int r0 = 16 * wr + 2 * t;
     uint32_t words[2][2];  // [channel of the pair][word of the half]
-    auto make = [&](bool divide, float& far) {
 #pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int j = 2 * jh + jj;
-        float half_lo[2], half_hi[2];
+    for (int jj = 0; jj < 2; ++jj) {
+      const int j = 2 * jh + jj;
+      float half_lo[2], half_hi[2];
 #pragma unroll
-        for (int hs = 0; hs < 2; ++hs) {
-          F2 acc = f2_pack(8388608.f, 8388608.f);
+      for (int hs = 0; hs < 2; ++hs) {
+        // value k = (thi, chi, e): row r0 + 8 thi + e, channels 32 j + 16 hs + 8 chi + 2 g2, + 1
+        auto pair = [&](int chi, int row) { return S::f(*reinterpret_cast<const Pair*>(vst + rtn_at<ROW>(r0 + row, (16 * j + 8 * hs + 4 * chi + g2) * (int)sizeof(Pair)))); };
+        F2 acc = f2_pack(8388608.f, 8388608.f);
+        float far = 0.f;
 #pragma unroll
-          for (int a = 0; a < 4; ++a) {
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int chi = a & 1, thi = a >> 1, row = 8 * thi + e;  // channels 32 j + 16 hs + 8 chi + 2 g2, + 1
-              const float2 x = S::f(reinterpret_cast<const Pair*>(rows + row * ROW)[16 * j + 8 * hs + 4 * chi + g2]);
-              const float weight = (float)(1 << (4 * (2 * chi + e) + 2 * thi));
-              if (divide) {
-                const float sc = vsc[srow + 4 * row + j];
-                acc = rtn_add_codes_divided(acc, x, make_float2(sc, sc), vq, 2.f, weight);
-              } else {
-                const float inv = vinv[srow + 4 * row + j];
-                acc = rtn_add_codes(acc, x, f2_pack(inv, inv), 2.f, weight, far);
-              }
-            }
-          }
-          f2_unpack(acc, half_lo[hs], half_hi[hs]);
+        for (int k = 0; k < 8; ++k) {
+          const int e = k & 1, chi = (k >> 1) & 1, thi = k >> 2, row = 8 * thi + e;
+          const float inv = vinv[4 * (r0 + row) + j];
+          acc = rtn_add_codes(acc, pair(chi, row), f2_pack(inv, inv), 2.f, (float)(1 << (4 * (2 * chi + e) + 2 * thi)), far);
         }
-        words[0][jj] = prmt(__float_as_uint(half_lo[0]), __float_as_uint(half_lo[1]), 0x5410u) ^ 0xAAAAAAAAu;
-        words[1][jj] = prmt(__float_as_uint(half_hi[0]), __float_as_uint(half_hi[1]), 0x5410u) ^ 0xAAAAAAAAu;
+        if (!(far < 0.5f - RTN_NEAR)) {
+          acc = f2_pack(8388608.f, 8388608.f);
+#pragma unroll 1
+          for (int k = 0; k < 8; ++k) {
+            const int e = k & 1, chi = (k >> 1) & 1, thi = k >> 2, row = 8 * thi + e;
+            const float2 x = pair(chi, row);
+            const float sc = vsc[4 * (r0 + row) + j], w = (float)(1 << (4 * (2 * chi + e) + 2 * thi));
+            acc = f2_fma(f2_pack(rtn_code_divided(x.x, sc, vq) + 2.f, rtn_code_divided(x.y, sc, vq) + 2.f), f2_pack(w, w), acc);
+          }
+        }
+        f2_unpack(acc, half_lo[hs], half_hi[hs]);
       }
-    };
-    float far = 0.f;
-    make(false, far);
-    if (!(far < 0.5f - RTN_NEAR)) make(true, far);
+      words[0][jj] = prmt(__float_as_uint(half_lo[0]), __float_as_uint(half_lo[1]), 0x5410u) ^ 0xAAAAAAAAu;
+      words[1][jj] = prmt(__float_as_uint(half_hi[0]), __float_as_uint(half_hi[1]), 0x5410u) ^ 0xAAAAAAAAu;
+    }
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       uint32_t* dst = vout + (wr * 32 + 4 * (2 * g2 + c) + t) * 4 + 2 * jh;
