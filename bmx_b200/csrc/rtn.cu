@@ -43,7 +43,12 @@ BMXK_HD int rtn_block_bytes(const RtnGeom& g) { return rtn_off_vscale(g) + g.pag
 // word that holds such a value (or a NaN) are divided.  With 16-bit sources exact halves are common (a value that is half of the
 // group's maximum: 4e-4 of the values of 2-bit codes), so it matters that no more than a word is done again.  |x| <= absmax keeps
 // the codes inside the clamp.
-// Measured, 4096 blocks (four sequences of 16384 tokens x 8 heads, 2-bit keys per channel, groups of 64, fp16): 417 -> 176 us.
+// Two-bit codes of 16-bit sources (all values; keys of the kivi recipe) need no quotient: qmax is 1, the scale is the group's
+// maximum s itself, and x / s > 1/2 exactly when x > s / 2 (two 11-bit numbers whose quotient is not 1/2 are 2^-12 away from it, so
+// the division's rounding cannot reach it; a tie is code 0 either way): two packed compares per pair.  A page with a NaN, an
+// infinite, zero or subnormal maximum takes the general way.
+// Measured, 4096 blocks (four sequences of 16384 tokens x 8 heads, 2-bit keys per channel, groups of 64, fp16): 417 -> 109 us = 3.0 TB/s;
+// 4-bit keys in groups of 32, half as many blocks: 243 -> 82 us (float32 sources 253 -> 121 us).
 // ---------------------------------------------------------------------------------------------
 constexpr int RTNQ_THREADS = 256;
 constexpr float RTN_NEAR = 4e-6f, RTN_MAGIC = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer, ties to even
@@ -55,21 +60,43 @@ struct RtnSrc<__half> {
   typedef uint32_t Pair;
   static __device__ __forceinline__ float2 f(Pair p) { return __half22float2(u32_as_h2(p)); }
   static __device__ __forceinline__ Pair absmax(Pair a, Pair b) { return h2_as_u32(__hmax2(u32_as_h2(a), __habs2(u32_as_h2(b)))); }
+  static __device__ __forceinline__ Pair absmax_nan(Pair a, Pair b) { return h2_as_u32(__hmax2_nan(u32_as_h2(a), __habs2(u32_as_h2(b)))); }
+  static __device__ __forceinline__ uint32_t above(Pair x, uint32_t t) { return __hgt2_mask(u32_as_h2(x), u32_as_h2(t)); }  // 0xFFFF per half
+  static __device__ __forceinline__ uint32_t below(Pair x, uint32_t t) { return __hlt2_mask(u32_as_h2(x), __hneg2(u32_as_h2(t))); }
+  static __device__ __forceinline__ uint32_t halves(float a, float b) { return h2_as_u32(__floats2half2_rn(0.5f * a, 0.5f * b)); }
+  static __device__ __forceinline__ bool plain(float m) { return m >= 2.5e-4f && m <= 65504.f; }  // m / 2 is a normal number of the type
 };
 template <>
 struct RtnSrc<__nv_bfloat16> {
   typedef uint32_t Pair;
   static __device__ __forceinline__ float2 f(Pair p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xFFFF0000u)); }
   static __device__ __forceinline__ Pair absmax(Pair a, Pair b) {
-    const __nv_bfloat162 r = __hmax2(*reinterpret_cast<__nv_bfloat162*>(&a), __habs2(*reinterpret_cast<__nv_bfloat162*>(&b)));
+    const __nv_bfloat162 r = __hmax2(bf2(a), __habs2(bf2(b)));
     return *reinterpret_cast<const uint32_t*>(&r);
   }
+  static __device__ __forceinline__ Pair absmax_nan(Pair a, Pair b) {
+    const __nv_bfloat162 r = __hmax2_nan(bf2(a), __habs2(bf2(b)));
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  static __device__ __forceinline__ __nv_bfloat162 bf2(uint32_t a) { return *reinterpret_cast<__nv_bfloat162*>(&a); }
+  static __device__ __forceinline__ uint32_t above(Pair x, uint32_t t) { return __hgt2_mask(bf2(x), bf2(t)); }
+  static __device__ __forceinline__ uint32_t below(Pair x, uint32_t t) { return __hlt2_mask(bf2(x), __hneg2(bf2(t))); }
+  static __device__ __forceinline__ uint32_t halves(float a, float b) {
+    const __nv_bfloat162 r = __floats2bfloat162_rn(0.5f * a, 0.5f * b);
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  static __device__ __forceinline__ bool plain(float m) { return m >= 1e-30f && m <= 3.3e38f; }
 };
 template <>
 struct RtnSrc<float> {
   typedef float2 Pair;
   static __device__ __forceinline__ float2 f(Pair p) { return p; }
   static __device__ __forceinline__ Pair absmax(Pair a, Pair b) { return make_float2(fmaxf(a.x, fabsf(b.x)), fmaxf(a.y, fabsf(b.y))); }
+  static __device__ __forceinline__ Pair absmax_nan(Pair a, Pair b) { return absmax(a, b); }
+  static __device__ __forceinline__ uint32_t above(Pair, uint32_t) { return 0u; }  // not used: float sources take the general way
+  static __device__ __forceinline__ uint32_t below(Pair, uint32_t) { return 0u; }
+  static __device__ __forceinline__ uint32_t halves(float, float) { return 0u; }
+  static __device__ __forceinline__ bool plain(float) { return true; }
 };
 __device__ __forceinline__ float max_nan(float a, float b) {
   float r;
@@ -151,8 +178,11 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
   }
   __syncthreads();
 
-  // ---- scales ----
-  auto token_scales = [&](const uint8_t* st, int grp, float qmax, float* sc, float* inv, __half* out) {  // four lanes per row, 32 channels each
+  // ---- scales; beside them 1 / scale, or (two-bit codes of 16-bit sources) half the scale as a pair of the source's type ----
+  constexpr bool V2 = sizeof(T) == 2;
+  const bool k2 = sizeof(T) == 2 && g.kbits == 2;
+  bool odd = false;  // a group that the packed compares do not cover
+  auto token_scales = [&](const uint8_t* st, int grp, float qmax, bool two, float* sc, float* inv, __half* out) {  // four lanes per row, 32 channels each
     constexpr int CH = 2 * (int)sizeof(T);  // sixteen-byte chunks of 32 channels
     for (int u = tid; u < PAGE * 4; u += RTNQ_THREADS) {
       const int r = u >> 2, qt = u & 3;
@@ -161,14 +191,23 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       for (int i = 0; i < CH; ++i) {
         const uint4 w = *reinterpret_cast<const uint4*>(st + rtn_at<ROW>(r, 16 * (CH * qt + ((i + qt * (CH / 4)) & (CH - 1)))));  // the lanes of a row start in different banks
 #pragma unroll
-        for (int e = 0; e < 16 / (int)sizeof(Pair); ++e) m = S::absmax(m, reinterpret_cast<const Pair*>(&w)[e]);
+        for (int e = 0; e < 16 / (int)sizeof(Pair); ++e) m = S::absmax_nan(m, reinterpret_cast<const Pair*>(&w)[e]);
       }
-      const float2 mf = S::f(m);
+      float2 mf = S::f(m);
+      if (mf.x != mf.x || mf.y != mf.y) {  // the reference's maximum passes over NaN
+        m = Pair{};
+        odd = true;
+        for (int i = 0; i < 16; ++i) m = S::absmax(m, *reinterpret_cast<const Pair*>(st + rtn_at<ROW>(r, (16 * qt + i) * (int)sizeof(Pair))));
+        mf = S::f(m);
+      }
       float am = fmaxf(mf.x, mf.y);
       if (grp >= 64) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
       if (grp == 128) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
       const float s = fmaxf(am, 1e-12f) / qmax;
-      sc[u] = s, inv[u] = 1.f / s;  // [row][32-channel quarter]
+      sc[u] = s;  // [row][32-channel quarter]
+      odd |= !S::plain(am);
+      if (two) reinterpret_cast<uint32_t*>(inv)[u] = S::halves(s, s);
+      else inv[u] = 1.f / s;
       const int per = grp / 32;
       if (qt % per == 0) out[r * 4 + qt / per] = __float2half_rn(s);
       if (qt >= HEAD_DIM / grp) out[r * 4 + qt] = __float2half_rn(0.f);
@@ -179,8 +218,14 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       const int c2 = u & 63, rb = u >> 6;
       Pair m = Pair{};
 #pragma unroll 16
-      for (int r = 0; r < 32; ++r) m = S::absmax(m, *reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(32 * rb + r, c2 * (int)sizeof(Pair))));
-      const float2 mf = S::f(m);
+      for (int r = 0; r < 32; ++r) m = S::absmax_nan(m, *reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(32 * rb + r, c2 * (int)sizeof(Pair))));
+      float2 mf = S::f(m);
+      if (mf.x != mf.x || mf.y != mf.y) {
+        m = Pair{};
+        odd = true;
+        for (int r = 0; r < 32; ++r) m = S::absmax(m, *reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(32 * rb + r, c2 * (int)sizeof(Pair))));
+        mf = S::f(m);
+      }
       *reinterpret_cast<float2*>(ksc + rb * HEAD_DIM + 2 * c2) = mf;
     }
     __syncthreads();
@@ -192,19 +237,26 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       float am = 0.f;
       for (int i = 0; i < per; ++i) am = fmaxf(am, ksc[(g0 + i) * HEAD_DIM + c]);
       sc[n] = fmaxf(am, 1e-12f) / kq;
+      odd |= !S::plain(am);
       if (rb == g0) kscale[k2b_kscale_idx(rb / per, c)] = __float2half_rn(sc[n]);
     }
     __syncthreads();
 #pragma unroll
     for (int n = 0; n < PAGE / 64; ++n) {
       const int o = ((tid >> 7) + 2 * n) * HEAD_DIM + c;
-      ksc[o] = sc[n], kinv[o] = 1.f / sc[n];
+      ksc[o] = sc[n];
+      if (k2) {  // channel pairs: [32-token block][64]
+        const float other = __shfl_xor_sync(0xffffffffu, sc[n], 1);
+        if (!(c & 1)) reinterpret_cast<uint32_t*>(kinv)[o >> 1] = S::halves(sc[n], other);
+      } else {
+        kinv[o] = 1.f / sc[n];
+      }
     }
   } else {
-    token_scales(kst, g.k_group, kq, ksc, kinv, kscale);
+    token_scales(kst, g.k_group, kq, k2, ksc, kinv, kscale);
   }
-  token_scales(vst, g.v_group, vq, vsc, vinv, vscale);
-  __syncthreads();
+  token_scales(vst, g.v_group, vq, V2, vsc, vinv, vscale);
+  const bool packed = !__syncthreads_or(odd);
 
   // ---- keys: thread = (16-row block, row g and g + 8, lane t of the quad): channels 8n + 2t, + 1 of two rows, 16 bytes each ----
   for (int u = tid; u < PAGE * 2; u += RTNQ_THREADS) {
@@ -215,15 +267,30 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       const int r = 16 * wr + 8 * th + gg;
       const int chan = (r >> 5) * HEAD_DIM + 2 * t;
       auto pair = [&](int n) { return S::f(*reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(r, (4 * n + t) * (int)sizeof(Pair)))); };
+      if (k2 && packed) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t w = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const Pair x = *reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(r, (4 * (4 * q + i) + t) * (int)sizeof(Pair)));
+            const uint32_t thr = reinterpret_cast<const uint32_t*>(kinv)[g.k_arm == RTN_CHANNEL ? (chan >> 1) + 4 * (4 * q + i) : 4 * r + q];
+            const uint32_t up = S::above(x, thr), dn = S::below(x, thr);
+            w |= ((up | dn) & (0x00010001u << (4 * i))) | (dn & (0x000E000Eu << (4 * i)));  // 0001 or 1111
+          }
+          out[th][q] = w;
+        }
+      } else
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         F2 acc = f2_pack(8388608.f, 8388608.f);  // 2^23: the sum sits in the low bits
         float far = 0.f;
-        const float rs = g.k_arm == RTN_CHANNEL ? 0.f : kinv[4 * r + q];
+        const float rs = g.k_arm == RTN_CHANNEL ? 0.f : k2 ? 1.f / ksc[4 * r + q] : kinv[4 * r + q];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           F2 inv;
-          if (g.k_arm == RTN_CHANNEL) inv.v = *reinterpret_cast<const unsigned long long*>(kinv + chan + 8 * (4 * q + i));
+          if (g.k_arm == RTN_CHANNEL && k2) inv = f2_pack(1.f / ksc[chan + 8 * (4 * q + i)], 1.f / ksc[chan + 8 * (4 * q + i) + 1]);
+          else if (g.k_arm == RTN_CHANNEL) inv.v = *reinterpret_cast<const unsigned long long*>(kinv + chan + 8 * (4 * q + i));
           else inv = f2_pack(rs, rs);
           acc = rtn_add_codes(acc, pair(4 * q + i), inv, 8.f, (float)(1 << (4 * i)), far);
         }
@@ -257,6 +324,23 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
 #pragma unroll
     for (int jj = 0; jj < 2; ++jj) {
       const int j = 2 * jh + jj;
+      if (V2 && packed) {
+        uint32_t w[2];  // 16 bits of each of the two channels' words
+#pragma unroll
+        for (int hs = 0; hs < 2; ++hs) {
+          w[hs] = 0;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int e = k & 1, chi = (k >> 1) & 1, thi = k >> 2, row = r0 + 8 * thi + e, bit = 4 * (2 * chi + e) + 2 * thi;
+            const Pair x = *reinterpret_cast<const Pair*>(vst + rtn_at<ROW>(row, (16 * j + 8 * hs + 4 * chi + g2) * (int)sizeof(Pair)));
+            const uint32_t thr = reinterpret_cast<const uint32_t*>(vinv)[4 * row + j];
+            const uint32_t up = S::above(x, thr), dn = S::below(x, thr);
+            w[hs] |= ((up | dn) & (0x00010001u << bit)) | (dn & (0x00020002u << bit));  // 01 or 11
+          }
+        }
+        words[0][jj] = prmt(w[0], w[1], 0x5410u), words[1][jj] = prmt(w[0], w[1], 0x7632u);
+        continue;
+      }
       float half_lo[2], half_hi[2];
 #pragma unroll
       for (int hs = 0; hs < 2; ++hs) {
@@ -267,7 +351,7 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const int e = k & 1, chi = (k >> 1) & 1, thi = k >> 2, row = 8 * thi + e;
-          const float inv = vinv[4 * (r0 + row) + j];
+          const float inv = V2 ? 1.f / vsc[4 * (r0 + row) + j] : vinv[4 * (r0 + row) + j];
           acc = rtn_add_codes(acc, pair(chi, row), f2_pack(inv, inv), 2.f, (float)(1 << (4 * (2 * chi + e) + 2 * thi)), far);
         }
         if (!(far < 0.5f - RTN_NEAR)) {
