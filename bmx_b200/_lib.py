@@ -89,6 +89,8 @@ _SIGNATURES = {
                                  c_int, c_void_p, c_void_p]),
     "bmxk_rtn_export": (c_int, [POINTER(RtnGeom), c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_void_p, c_void_p]),
+    "bmxk_rtn_dequant_dense": (c_int, [POINTER(RtnGeom), c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
+                                       c_void_p, c_void_p, c_int64, c_int, c_void_p]),
     "bmxk_rtn_decode": (c_int, [POINTER(RtnGeom), c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                                  c_void_p, c_void_p, c_int, c_float, c_void_p, c_size_t, c_void_p, c_int, c_void_p,
                                  c_void_p]),

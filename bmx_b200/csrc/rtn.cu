@@ -431,6 +431,124 @@ __global__ void rtn_export_kernel(RtnGeom g, const uint8_t* __restrict__ pages, 
 }
 
 // ---------------------------------------------------------------------------------------------
+// Page dequantizer of the dense prompt route: code * fp16 scale rounded once to the model's 16-bit type, written straight into
+// (batch, h_kv, row_stride, 128) tensors with the fp16 window behind the pages.  One block per (sequence, page, head); the last
+// blocks of a sequence copy 128 window rows each.  What bounds it: the writes (512 bytes per token and head, 112 read).  A thread
+// decodes the words of the layout and drops channel pairs into swizzled rows in shared memory, which leave as sixteen-byte stores.
+// Measured, 8192 tokens x 8 heads: @@RD@@
+// ---------------------------------------------------------------------------------------------
+constexpr int RTND_THREADS = 256;
+template <typename OutT>
+struct RtnOut;
+template <>
+struct RtnOut<__half> {
+  static __device__ __forceinline__ uint32_t scaled(__half2 code, __half2 sc) { return h2_as_u32(__hmul2(code, sc)); }  // one rounding
+  static __device__ __forceinline__ uint4 copied(uint4 w) { return w; }
+};
+template <>
+struct RtnOut<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t two(float2 x) {
+    const __nv_bfloat162 r = __floats2bfloat162_rn(x.x, x.y);
+    return *reinterpret_cast<const uint32_t*>(&r);
+  }
+  static __device__ __forceinline__ uint32_t scaled(__half2 code, __half2 sc) {  // the product of a code and an fp16 scale is exact in float32
+    const float2 a = __half22float2(code), b = __half22float2(sc);
+    return two(make_float2(a.x * b.x, a.y * b.y));
+  }
+  static __device__ __forceinline__ uint4 copied(uint4 w) {
+    return make_uint4(two(__half22float2(u32_as_h2(w.x))), two(__half22float2(u32_as_h2(w.y))), two(__half22float2(u32_as_h2(w.z))),
+                      two(__half22float2(u32_as_h2(w.w))));
+  }
+};
+
+template <typename OutT, int PAGE>
+__global__ void __launch_bounds__(RTND_THREADS) rtn_dequant_dense_kernel(RtnGeom g, const uint8_t* __restrict__ pages,
+                                                                         const int32_t* __restrict__ page_table, int table_stride, int n_pg,
+                                                                         const __half* __restrict__ k_tail, const __half* __restrict__ v_tail,
+                                                                         int tail_len, int tail_cap, OutT* __restrict__ k_out,
+                                                                         OutT* __restrict__ v_out, int64_t row_stride) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint8_t *kst = smem, *vst = smem + PAGE * 256;
+  const int per_seq = n_pg + (tail_len + 127) / 128, b = blockIdx.x / per_seq, j = blockIdx.x % per_seq, h = blockIdx.y, tid = threadIdx.x;
+  const int64_t bh = (int64_t)b * g.h_kv + h;
+  if (j >= n_pg) {  // window rows
+    const int t0 = (j - n_pg) * 128, n = min(128, tail_len - t0);
+    const uint4* ks = reinterpret_cast<const uint4*>(k_tail + (bh * tail_cap + t0) * HEAD_DIM);
+    const uint4* vs = reinterpret_cast<const uint4*>(v_tail + (bh * tail_cap + t0) * HEAD_DIM);
+    uint4* kd = reinterpret_cast<uint4*>(k_out + (bh * row_stride + (int64_t)n_pg * PAGE + t0) * HEAD_DIM);
+    uint4* vd = reinterpret_cast<uint4*>(v_out + (bh * row_stride + (int64_t)n_pg * PAGE + t0) * HEAD_DIM);
+    for (int o = tid; o < n * 16; o += RTND_THREADS) kd[o] = RtnOut<OutT>::copied(ks[o]), vd[o] = RtnOut<OutT>::copied(vs[o]);
+    return;
+  }
+  const uint8_t* blk = pages + ((int64_t)page_table[(int64_t)b * table_stride + j] * g.h_kv + h) * rtn_block_bytes(g);
+  const __half* ks = reinterpret_cast<const __half*>(blk + rtn_off_kscale(g));
+  const __half* vs = reinterpret_cast<const __half*>(blk + rtn_off_vscale(g));
+  const __half2 c1032 = __floats2half2_rn(1032.f, 1032.f), c16th = __floats2half2_rn(0.0625f, 0.0625f), cm72 = __floats2half2_rn(-72.f, -72.f);
+  // keys: thread = (16-row block, row g and g + 8, lane t): channels 8n + 2t, + 1
+  for (int u = tid; u < PAGE * 2; u += RTND_THREADS) {
+    const int wr = u >> 5, gg = (u >> 2) & 7, t = u & 3;
+    uint4 sc4[4];  // rtn_channel: the scales of the token group, both rows
+    if (g.k_arm == RTN_CHANNEL) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) sc4[q] = *reinterpret_cast<const uint4*>(ks + ((16 * wr) / g.k_group) * 128 + q * 32 + t * 8);
+    }
+#pragma unroll
+    for (int th = 0; th < 2; ++th) {
+      const int r = 16 * wr + 8 * th + gg;
+      const uint4 w4 = *reinterpret_cast<const uint4*>(blk + ((wr * 2 + th) * 32 + 4 * gg + t) * 16);
+      const uint32_t ww[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t lo = ww[q], hi = ww[q] >> 8;
+        __half2 c[4] = {__hsub2(u32_as_h2(lop3<0x6A>(lo, 0x000F000Fu, 0x64086408u)), c1032),
+                        __hfma2(u32_as_h2(lop3<0x6A>(lo, 0x00F000F0u, 0x64806480u)), c16th, cm72),
+                        __hsub2(u32_as_h2(lop3<0x6A>(hi, 0x000F000Fu, 0x64086408u)), c1032),
+                        __hfma2(u32_as_h2(lop3<0x6A>(hi, 0x00F000F0u, 0x64806480u)), c16th, cm72)};
+        const uint32_t chan[4] = {sc4[q].x, sc4[q].y, sc4[q].z, sc4[q].w};
+        const __half2 tok = g.k_arm == RTN_CHANNEL ? __half2half2(__ushort_as_half(0)) : __half2half2(ks[r * 4 + (32 * q) / g.k_group]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint32_t*>(kst + rtn_at<256>(r, (4 * (4 * q + i) + t) * 4)) =
+              RtnOut<OutT>::scaled(c[i], g.k_arm == RTN_CHANNEL ? u32_as_h2(chan[i]) : tok);
+      }
+    }
+  }
+  // values: thread = (16-row block, channels 8m + 2g2, + 1, lane t, half of the words)
+  for (int u = tid; u < PAGE * 2; u += RTND_THREADS) {
+    const int wr = u >> 5, g2 = (u >> 3) & 3, t = (u >> 1) & 3, jh = u & 1, r0 = 16 * wr + 2 * t;
+    const uint2 wa = *reinterpret_cast<const uint2*>(blk + rtn_off_vcode(g) + (wr * 32 + 8 * g2 + t) * 16 + 8 * jh);
+    const uint2 wb = *reinterpret_cast<const uint2*>(blk + rtn_off_vcode(g) + (wr * 32 + 8 * g2 + 4 + t) * 16 + 8 * jh);
+    const uint32_t lut = 0xBCC03C00u;  // high bytes of 0, 1, -2, -1 as fp16
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+      for (int hs = 0; hs < 2; ++hs)
+#pragma unroll
+        for (int thi = 0; thi < 2; ++thi) {
+          const uint32_t sa = ((jj ? wa.y : wa.x) >> (16 * hs + 2 * thi)) & 0x3333u, sb = ((jj ? wb.y : wb.x) >> (16 * hs + 2 * thi)) & 0x3333u;
+          const uint32_t ha = prmt(lut, 0u, sa), hb = prmt(lut, 0u, sb);  // bytes: (chi 0, e 0), (0, 1), (1, 0), (1, 1)
+          const uint32_t c0 = prmt(ha, hb, 0x5140u), c1 = prmt(ha, hb, 0x7362u);
+#pragma unroll
+          for (int chi = 0; chi < 2; ++chi)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int r = r0 + 8 * thi + e, c = 32 * (2 * jh + jj) + 16 * hs + 8 * chi + 2 * g2;
+              const __half2 code = u32_as_h2(prmt(chi ? c1 : c0, 0u, e ? 0x3424u : 0x1404u));
+              *reinterpret_cast<uint32_t*>(vst + rtn_at<256>(r, 2 * c)) =
+                  RtnOut<OutT>::scaled(code, __half2half2(vs[r * 4 + (32 * (2 * jh + jj)) / g.v_group]));
+            }
+        }
+  }
+  __syncthreads();
+  uint4* kd = reinterpret_cast<uint4*>(k_out + (bh * row_stride + (int64_t)j * PAGE) * HEAD_DIM);
+  uint4* vd = reinterpret_cast<uint4*>(v_out + (bh * row_stride + (int64_t)j * PAGE) * HEAD_DIM);
+  for (int o = tid; o < PAGE * 16; o += RTND_THREADS) {
+    const int at = rtn_at<256>(o >> 4, (o & 15) * 16);
+    kd[o] = *reinterpret_cast<const uint4*>(kst + at), vd[o] = *reinterpret_cast<const uint4*>(vst + at);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Split-KV decode.  Persistent grid, 8 warps per CTA, warp w owns token rows 16w..16w+15 of every
 // 128-token tile of its CTA's range; same flat decomposition, partial record and merge kernel as k2b.
 // ---------------------------------------------------------------------------------------------
@@ -834,6 +952,44 @@ int bmxk_rtn_export(const bmxk_rtn_geom* g, const void* pages, const int32_t* sl
   rtn_export_kernel<<<n * g->h_kv, 256, 0, (cudaStream_t)stream>>>(to_rtn(g), (const uint8_t*)pages, slots, k_codes,
                                                                   (__half*)k_scales, v_codes, (__half*)v_scales, k_deq, v_deq);
   return check_launch("bmxk_rtn_export");
+}
+
+int bmxk_rtn_dequant_dense(const bmxk_rtn_geom* g, const void* pages, const int32_t* page_table, int table_stride, int n_pages, int batch,
+                           const void* k_tail, const void* v_tail, int tail_len, int tail_cap, void* k_out, void* v_out,
+                           int64_t row_stride, int out_dtype, void* stream) {
+  int rc = check_rtn_geom(g, "bmxk_rtn_dequant_dense");
+  if (rc) return rc;
+  BMXK_REQUIRE(n_pages >= 0 && batch >= 1 && tail_len >= 0 && tail_len <= tail_cap, "bmxk_rtn_dequant_dense: n_pages=%d batch=%d tail_len=%d of %d",
+               n_pages, batch, tail_len, tail_cap);
+  const int64_t blocks = ((int64_t)n_pages + (tail_len + 127) / 128) * batch;
+  if (blocks == 0) return BMXK_OK;
+  BMXK_REQUIRE(blocks <= 0x7fffffff, "bmxk_rtn_dequant_dense: too many pages in one call");
+  BMXK_REQUIRE(k_out && v_out && (n_pages == 0 || (pages && page_table && table_stride >= n_pages)) && (tail_len == 0 || (k_tail && v_tail)),
+               "bmxk_rtn_dequant_dense: null pointer or table_stride=%d < n_pages", table_stride);
+  BMXK_REQUIRE(row_stride >= (int64_t)n_pages * g->page + tail_len, "bmxk_rtn_dequant_dense: row_stride=%lld below the rows written",
+               (long long)row_stride);
+  BMXK_REQUIRE(out_dtype == BMXK_DTYPE_F16 || out_dtype == BMXK_DTYPE_BF16, "bmxk_rtn_dequant_dense: out_dtype=%d (fp16 or bf16)", out_dtype);
+  BMXK_REQUIRE((((uintptr_t)pages | (uintptr_t)k_out | (uintptr_t)v_out | (uintptr_t)k_tail | (uintptr_t)v_tail) & 15) == 0,
+               "bmxk_rtn_dequant_dense: misaligned buffer");
+  const dim3 grid((unsigned)blocks, (unsigned)g->h_kv);
+  cudaStream_t s = (cudaStream_t)stream;
+#define BMXK_RTN_DENSE(OutT, PAGE)                                                                                                          \
+  {                                                                                                                                          \
+    static PerDeviceOnce configured;                                                                                                         \
+    if (configured.first()) cudaFuncSetAttribute(rtn_dequant_dense_kernel<OutT, PAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * PAGE * 256); \
+    rtn_dequant_dense_kernel<OutT, PAGE><<<grid, RTND_THREADS, 2 * PAGE * 256, s>>>(to_rtn(g), (const uint8_t*)pages, page_table, table_stride, n_pages,   \
+                                                                     (const __half*)k_tail, (const __half*)v_tail, tail_len, tail_cap,      \
+                                                                     (OutT*)k_out, (OutT*)v_out, row_stride);     \
+  }
+  if (out_dtype == BMXK_DTYPE_F16) {
+    if (g->page == 128) BMXK_RTN_DENSE(__half, 128)
+    else BMXK_RTN_DENSE(__half, 64)
+  } else {
+    if (g->page == 128) BMXK_RTN_DENSE(__nv_bfloat16, 128)
+    else BMXK_RTN_DENSE(__nv_bfloat16, 64)
+  }
+#undef BMXK_RTN_DENSE
+  return check_launch("bmxk_rtn_dequant_dense");
 }
 
 int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,

@@ -570,6 +570,14 @@ class RtnLayerState(K2bLayerState):
         shp = (self.batch, n_pg * self.page, h_kv, HEAD_DIM)
         return ex["k_deq"].view(*shp).permute(0, 2, 1, 3), ex["v_deq"].view(*shp).permute(0, 2, 1, 3)
 
+    def dense_kv(self, dtype: torch.dtype) -> tuple[torch.Tensor, torch.Tensor]:
+        """Everything held as dense tensors (batch, h_kv, committed + window, 128) of the model's 16-bit type, by one kernel."""
+        assert dtype in (torch.float16, torch.bfloat16), dtype
+        kd = torch.empty(self.batch, self.geom.h_kv, self.seq_len(), HEAD_DIM, dtype=dtype, device=self.device)
+        vd = torch.empty_like(kd)
+        K.rtn_dequant_dense(self.pool, self.page_table, self.committed // self.page, self.k_win, self.v_win, self.tail_len, kd, vd)
+        return kd, vd
+
     def packed_bytes(self) -> int:
         return int(self.batch * self.geom.h_kv * (self.committed // self.page) * self.pool.pages.shape[2])
 

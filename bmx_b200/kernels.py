@@ -499,6 +499,24 @@ def rtn_export(pool: RtnPool, slots: torch.Tensor, dequant: bool = False) -> dic
     return out
 
 
+def rtn_dequant_dense(pool: RtnPool, page_table: torch.Tensor, n_pages: int, k_tail: torch.Tensor, v_tail: torch.Tensor, tail_len: int,
+                      k_out: torch.Tensor, v_out: torch.Tensor) -> None:
+    """The first n_pages pages of every sequence and tail_len rows of the fp16 windows behind them, dequantized into k_out / v_out
+    (batch, h_kv, rows, 128), fp16 or bf16."""
+    g = pool.geom
+    _require_cuda(page_table, k_tail, v_tail, k_out, v_out)
+    batch = page_table.shape[0]
+    assert page_table.dtype == torch.int32 and page_table.dim() == 2 and page_table.stride(1) == 1
+    assert k_out.shape == v_out.shape and k_out.shape[:2] == (batch, g.h_kv) and k_out.shape[3] == HEAD_DIM
+    assert k_out.is_contiguous() and v_out.is_contiguous() and k_out.dtype == v_out.dtype
+    assert k_out.dtype in (torch.float16, torch.bfloat16), k_out.dtype
+    assert k_tail.dtype == v_tail.dtype == torch.float16 and k_tail.is_contiguous() and v_tail.is_contiguous()
+    assert k_tail.shape == v_tail.shape and k_tail.shape[:2] == (batch, g.h_kv) and k_tail.shape[3] == HEAD_DIM
+    call("bmxk_rtn_dequant_dense", ctypes.byref(g), _ptr(pool.pages), _ptr(page_table), page_table.stride(0), int(n_pages), batch, _ptr(k_tail),
+         _ptr(v_tail), int(tail_len), k_tail.shape[2], _ptr(k_out), _ptr(v_out), k_out.shape[2],
+         DTYPE_BF16 if k_out.dtype == torch.bfloat16 else DTYPE_F16, _stream())
+
+
 def rtn_workspace(g: RtnGeom, batch: int, max_pages: int, device) -> torch.Tensor:
     n = int(_lib.lib().bmxk_rtn_decode_workspace_bytes(ctypes.byref(g), batch, max_pages))
     return torch.zeros(n, dtype=torch.uint8, device=device)

@@ -368,7 +368,7 @@ class PackedStreamingLayer(DynamicLayer):
         """All committed pages dequantized (keys rotated at their positions) + the window: (b, h_kv, S, d)."""
         st = self._state
         n_pg = st.committed // self._page
-        if self._kind == "k2b" and dtype in (torch.float16, torch.bfloat16):
+        if self._kind in ("k2b", "rtn") and dtype in (torch.float16, torch.bfloat16):
             return st.dense_kv(dtype)
         parts_k, parts_v = [], []
         if n_pg:

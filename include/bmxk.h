@@ -259,6 +259,13 @@ int bmxk_rtn_append(const bmxk_rtn_geom* g, const void* k, const void* v, int sr
 int bmxk_rtn_export(const bmxk_rtn_geom* g, const void* pages, const int32_t* slots, int n, int8_t* k_codes,
                     void* k_scales, int8_t* v_codes, void* v_scales, float* k_deq, float* v_deq, void* stream);
 
+/* Everything a sequence holds as dense 16-bit K and V (batch, h_kv, row_stride, 128): n_pages committed pages per sequence
+ * (code * scale rounded once; keys are stored rotated) and tail_len rows of the fp16 window (batch, h_kv, tail_cap, 128)
+ * behind them.  bmx: src/bmx/cache/chunked_attention.py:320-395, which dequantizes to float32 and casts.
+ * out_dtype: F16 or BF16; buffers 16-byte aligned. */
+int bmxk_rtn_dequant_dense(const bmxk_rtn_geom* g, const void* pages, const int32_t* page_table, int table_stride, int n_pages, int batch,
+                           const void* k_tail, const void* v_tail, int tail_len, int tail_cap, void* k_out, void* v_out,
+                           int64_t row_stride, int out_dtype, void* stream);
 /* One decode step over RTN pages + the fp16 window; arguments as in bmxk_k2b_decode.
  * bmx: src/bmx/cache/triton_dequant_attention.py:580-832 fused_decode_attention_packed (+ tail, merge). */
 int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table,

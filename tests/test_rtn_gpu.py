@@ -285,3 +285,27 @@ def test_append_codes_equal_the_divided_ones(dtype, page, arm, k_group, v_group,
         kc, ks = _rtn_codes(kk, kbits, k_group, 2)  # codes (items, h, page, 128), scales (items, h, 128, groups)
         assert torch.equal(ex["k_codes"], kc.transpose(2, 3).reshape(n * pages, h * 128, page))
         assert torch.equal(ex["k_scales"].view(torch.int16), ks.half().reshape(n * pages, h * 128, -1).view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("page,arm,k_group,v_group,kbits", [(128, "rtn_channel", 64, 64, 2), (128, "rtn_channel", 32, 128, 4),
+                                                            (128, "rtn_token", 32, 32, 3), (64, "rtn_channel", 64, 32, 4), (64, "rtn_token", 128, 64, 2)])
+@pytest.mark.parametrize("tokens", [5, 700, 1290])
+def test_dense_kv_equals_dequantize_and_cast(dtype, page, arm, k_group, v_group, kbits, tokens):
+    """One kernel writes pages and window in the model's type: equal to dequantizing in float32, casting and concatenating."""
+    from bmx_b200 import kernels as K
+    from bmx_b200.engine import RtnLayerState
+
+    dev = torch.device("cuda:0")
+    B, h = 2, 3
+    st = RtnLayerState(K.rtn_geom(h, 4, page, arm, k_group, v_group, kbits, 2), B, 2048, 200, dev)
+    st.page_table.copy_(torch.randperm(st.page_table.numel(), device=dev).view_as(st.page_table).to(torch.int32))
+    gen = torch.Generator(device=dev).manual_seed(tokens + page)
+    k, v = (torch.randn(B, h, tokens, 128, generator=gen, device=dev).half() for _ in range(2))
+    st.append(None, k, v)
+    kd, vd = st.dense_kv(dtype)
+    wk, wv = [st.k_win[:, :, : st.tail_len].to(dtype)], [st.v_win[:, :, : st.tail_len].to(dtype)]
+    if st.committed:
+        pk, pv = st.dense_pages()
+        wk, wv = [pk.to(dtype)] + wk, [pv.to(dtype)] + wv
+    assert torch.equal(kd, torch.cat(wk, 2)) and torch.equal(vd, torch.cat(wv, 2))
