@@ -394,6 +394,16 @@ def gather_next_slots(page_table: torch.Tensor, n_pages: torch.Tensor, n: int, o
     return out
 
 
+def mask_is_causal(mask: torch.Tensor, n_q: int, S: int) -> bool:
+    """True when the boolean mask (batch, 1, n_q, S) hides exactly the keys at positions after each query row.  Waits for the answer."""
+    _require_cuda(mask)
+    assert mask.dtype == torch.bool and mask.shape[1:] == (1, n_q, S) and mask.stride(3) == 1
+    differs = torch.zeros(1, dtype=torch.int32, device=mask.device)
+    call("bmxk_mask_is_causal", _ptr(mask), mask.stride(0) if mask.shape[0] > 1 else 0, mask.stride(2), mask.shape[0], int(n_q), int(S),
+         _ptr(differs), _stream())
+    return int(differs) == 0
+
+
 def window_shift(k_win: torch.Tensor, v_win: torch.Tensor, k_src_win: torch.Tensor, off: int, rest: int, tail_len: torch.Tensor,
                  n_pages: torch.Tensor | None = None, pages_added: int = 0) -> None:
     """Moves tokens [off, off + rest) of every (sequence, head) window to the front (one launch for the three windows),

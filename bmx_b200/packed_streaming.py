@@ -397,6 +397,8 @@ class PackedStreamingLayer(DynamicLayer):
         m = attention_mask
         if m.dim() != 4 or m.shape[-2] != n_q or m.shape[-1] != S or m.shape[1] != 1:
             return False
+        if m.dtype == torch.bool and m.is_cuda and m.stride(3) == 1 and 1 <= n_q <= S and m.shape[0] >= 1:
+            return K.mask_is_causal(m, n_q, S)
         vis = m if m.dtype == torch.bool else (m > -1.0)
         want = torch.ones(n_q, S, dtype=torch.bool, device=m.device).tril(S - n_q)
         return bool((vis == want).all())
@@ -433,7 +435,10 @@ class PackedStreamingLayer(DynamicLayer):
         if self._mask_is_causal(attention_mask, n_q, S):  # the model's plain causal mask: no per-sequence mask, no copies of K / V
             if n_q == S:
                 return F.scaled_dot_product_attention(q, Kd, Vd, is_causal=n_q > 1, scale=scaling, enable_gqa=gqa)
-            mask = torch.ones(n_q, S, dtype=torch.bool, device=q.device).tril(S - n_q)
+            if attention_mask.dtype == torch.bool:  # it is that mask: one row block for all sequences
+                mask = attention_mask[:1]
+            else:
+                mask = torch.ones(n_q, S, dtype=torch.bool, device=q.device).tril(S - n_q)
             return F.scaled_dot_product_attention(q, Kd, Vd, attn_mask=mask, scale=scaling, enable_gqa=gqa)
         Kx = Kd.repeat_interleave(self._n_q_groups, dim=1)
         Vx = Vd.repeat_interleave(self._n_q_groups, dim=1)

@@ -387,6 +387,10 @@ int bmxk_window_append_devpos(const void* k_post, const void* v, const void* k_s
                               int64_t stride_head, void* k_win, void* v_win, void* k_src_win, int32_t* tail_len,
                               int32_t* counters, int32_t* status, int batch, int h_kv, int tail_cap, void* stream);
 
+/* Sets *differs to 1 if the boolean mask (batch, n_q rows of S bytes, strides in bytes) is not the causal one of the last n_q
+ * positions of S; *differs is left alone otherwise (device memory, zeroed by the caller). */
+int bmxk_mask_is_causal(const void* mask, int64_t stride_b, int64_t stride_q, int batch, int n_q, int S, int32_t* differs, void* stream);
+
 /* After pages were committed out of the windows: the remaining tokens [off, off + rest) of every (sequence, head) move to
  * the front of the three windows in one launch, tail_len[s] becomes rest and, when n_pages is not NULL, n_pages[s] grows by
  * pages_added.  bmx slices its tail tensors instead (src/bmx/cache/packed_streaming.py:700-730).  k_src_win may be k_win. */
