@@ -30,4 +30,11 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
   return r;
 }
 
+// Maximum that hands NaN on (fmaxf drops it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 }  // namespace bmxk

@@ -5,7 +5,7 @@
 // float32 operations stays two operations here; the sums that ARE fused use fmaf explicitly
 // and run in a fixed order (ascending index, one accumulator), which `oracle/cpu_ref.c`
 // repeats step for step.
-#include "common.cuh"
+#include "value_quant.cuh"
 
 namespace bmxk {
 
@@ -117,7 +117,7 @@ __global__ void k2b_store_coefs_kernel(K2bGeom g, const float* __restrict__ us, 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Page quantizer.  One block of 256 threads per (item, kv head); two blocks share an SM.
+// Page quantizer for layout 0 (64-token pages, or 128 on request).  One block of 256 threads per (item, kv head); two blocks share an SM.
 //   staging: the head's key page (float32, KF_STRIDE per row) and its basis slice go to shared memory.
 //   coefficients (FUSED: one basis per head): thread = (row slot, four i), ROWS rows each;
 //           Us[r,i] = fmaf chain over c ascending, rounded to fp16, written to the coefficient block.
@@ -331,29 +331,6 @@ __global__ void __launch_bounds__(QP_THREADS, 2) k2b_quant_page_kernel(K2bGeom g
   __syncthreads();
   // ---- assemble native words ----
   uint32_t* kres = reinterpret_cast<uint32_t*>(blk);
-  if (g.layout == 1) {
-    // row order: word w of the K residual = (chunk k, token r, word j); of the V codes = (chunk cc, channel c, word j)
-    for (int w = tid; w < page * 16; w += blockDim.x) {
-      const int j = w & 3, r = (w >> 2) & 127, k = w >> 9;
-      const int base = (j < 2) ? 16 * k + 8 * j : 64 + 16 * k + 8 * (j - 2);
-      uint32_t word = 0;
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) word |= ((uint32_t)kcode[r * HEAD_DIM + base + 2 * i + e] & 0xFu) << (16 * e + 4 * i);
-      kres[w] = word;
-    }
-    uint32_t* vw1 = reinterpret_cast<uint32_t*>(blk + k2b_off_vcode(page, group));
-    for (int w = tid; w < page * 8; w += blockDim.x) {
-      const int j = w & 3, c = (w >> 2) & 127, cc = w >> 9;
-      uint32_t word = 0;
-#pragma unroll
-      for (int tau = 0; tau < 16; ++tau)
-        word |= (uint32_t)vcode[(64 * cc + 16 * j + tau) * HEAD_DIM + c] << (tau < 8 ? 4 * tau : 4 * (tau - 8) + 2);
-      vw1[w] = word;
-    }
-    return;
-  }
   for (int w = tid; w < page * 16; w += blockDim.x) {
     const int q = w & 3, ln = (w >> 2) & 31, th = (w >> 7) & 1, wr = w >> 8;
     const int gg = ln >> 2, t = ln & 3;
@@ -384,6 +361,295 @@ __global__ void __launch_bounds__(QP_THREADS, 2) k2b_quant_page_kernel(K2bGeom g
           word |= (uint32_t)vcode[r * HEAD_DIM + c] << (16 * hs + 4 * (2 * (a & 1) + e) + 2 * (a >> 1));
         }
     vw[w] = word;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Page quantizer for layout 1 (128-token pages): the same bytes as k2b_quant_page_kernel, which serves layout 0.  One block of 256
+// threads per (item, kv head), two blocks per SM.
+// What bounds it: warp instructions.  The two products (128 x 128 x rank each) have to stay float32 sums in ascending order, so they
+// run as register tiles on operands stored so that a thread reads four of a kind with one 128-bit load (keys and coefficients
+// token-minor); the value codes come from value_quant.cuh.
+//   coefficients (FUSED: one basis per head): thread = 4 rows x RANK / 8 of the basis vectors.
+//   keys    thread = 8 channels x 8 rows (4 rg .. + 3 and 64 + 4 rg ..): residuals stay in registers, absmax by shuffles over the 16
+//           lanes that share the channels, one lane per (channel, half) divides and hands scale and inverse back through shared memory;
+//           codes are products with the inverse scale (a thread that sees one within K2BQ_NEAR of a half, or a NaN, divides all of
+//           its 64: 3 * 2^-24 * 7.5 = 1.3e-6 is the largest difference to the rounded quotient), and eight channels of a row are one
+//           word of the layout: codes are summed at their bit position in float32 (offset binary, 16 bits: exact).
+// Measured, 4096 blocks (four sequences of 16384 tokens x 8 heads, rank 32 per head, bf16): 656 -> 402 us.
+// ---------------------------------------------------------------------------------------------
+constexpr float K2BQ_NEAR = 2e-6f, K2BQ_MAGIC = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer, ties to even
+constexpr int K2BQ_STR = 132;                                // floats per channel row (tokens) and per basis-vector row
+template <int RANK>
+struct K2bQuantSmem {
+  static constexpr int OPERAND = (RANK * K2BQ_STR > HEAD_DIM * RANK ? RANK * K2BQ_STR : HEAD_DIM * RANK) * 4;  // basis rows, later coefficients
+  static constexpr int MS = HEAD_DIM * K2BQ_STR * 4;          // keys; later the staged value page, its words, norms
+  static constexpr int V16 = RANK * K2BQ_STR * 4;             // fp16-rounded basis, one row per vector
+  static constexpr int WORDS = HEAD_DIM * 64;                 // key words, over the operands once they are dead
+  static constexpr int SCALES = 2 * 4 * HEAD_DIM * 4;         // scale and inverse by (32-token block, channel)
+  static constexpr int BYTES = MS + (OPERAND + V16 > WORDS ? OPERAND + V16 : WORDS) + SCALES;
+  static_assert(VQ_SMEM_BYTES <= MS && 128 * HEAD_DIM <= MS, "the value page is staged over the keys");
+};
+
+__device__ __noinline__ float k2b_code_divided(float x, float scale, float qmax) { return fminf(fmaxf(rintf(x / scale), -qmax - 1.f), qmax); }
+
+template <typename T, int RANK, bool FUSED>
+__global__ void __launch_bounds__(QP_THREADS, 2) k2b_quant_rows_kernel(K2bGeom g, const T* __restrict__ k_pre, const T* __restrict__ v,
+                                                                       int64_t stride_seq, int64_t stride_head, int64_t stride_tok,
+                                                                       const float* __restrict__ basis, const float* __restrict__ signs,
+                                                                       const float* __restrict__ codebook, const int32_t* __restrict__ slots,
+                                                                       int n_pages, uint8_t* __restrict__ pages, __half* __restrict__ coefs,
+                                                                       int vec) {
+  typedef K2bQuantSmem<RANK> L;
+  extern __shared__ __align__(16) uint8_t smem[];
+  float* Ms = reinterpret_cast<float*>(smem);                       // [128 channels][K2BQ_STR]
+  float* op = reinterpret_cast<float*>(smem + L::MS);               // basis [128][RANK], later coefficients [RANK][K2BQ_STR]
+  float* v16 = reinterpret_cast<float*>(smem + L::MS + L::OPERAND); // [RANK][K2BQ_STR]
+  float* ksc = reinterpret_cast<float*>(smem + L::BYTES - L::SCALES);  // [4][128] scales by 32-token block
+  float* kinv = ksc + 4 * HEAD_DIM;
+  const int item = blockIdx.x / g.h_kv, h = blockIdx.x % g.h_kv;
+  const int seq = item / n_pages, pg = item % n_pages, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slot = slots[item], ch = (g.n_coef_heads == 1) ? 0 : h;
+  __half* cblk = coefs + ((int64_t)slot * g.n_coef_heads + ch) * (128 * RANK);
+  uint8_t* blk = pages + ((int64_t)slot * g.h_kv + h) * k2b_page_block_bytes(128, g.group);
+  const T* ksrc = k_pre + seq * stride_seq + h * stride_head + (int64_t)pg * 128 * stride_tok;
+  const T* vsrc = v + seq * stride_seq + h * stride_head + (int64_t)pg * 128 * stride_tok;
+
+  // ---- staging: a lane takes 64 channels of one row; the values are fetched into L2 meanwhile ----
+  {
+    const int r = 32 * (warp & 3) + lane, c_base = 64 * (warp >> 2);
+    const T* src = ksrc + r * stride_tok + c_base;
+    constexpr int PER = 16 / (int)sizeof(T), CHUNK = 32;
+    if (tid < 128) {
+      const char* row = reinterpret_cast<const char*>(vsrc + tid * stride_tok);
+#pragma unroll
+      for (int o = 0; o < HEAD_DIM * (int)sizeof(T); o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + o));
+    }
+    if (vec & 1) {
+      uint4 u[64 / PER];
+#pragma unroll
+      for (int i = 0; i < 64 / PER; ++i) u[i] = *reinterpret_cast<const uint4*>(src + i * PER);
+#pragma unroll
+      for (int i = 0; i < 64; ++i) Ms[(c_base + i) * K2BQ_STR + r] = load_as_float<T>(reinterpret_cast<const T*>(u) + i);
+    } else {
+      for (int c0 = 0; c0 < 64; c0 += CHUNK) {
+#pragma unroll 8
+        for (int i = 0; i < CHUNK; ++i) Ms[(c_base + c0 + i) * K2BQ_STR + r] = load_as_float<T>(src + c0 + i);
+      }
+    }
+    const float4* bsrc = reinterpret_cast<const float4*>(basis + (int64_t)h * HEAD_DIM * RANK);
+    for (int o = tid; o < HEAD_DIM * RANK / 4; o += QP_THREADS) {
+      const float4 b = bsrc[o];
+      const int c = o / (RANK / 4), i4 = 4 * (o % (RANK / 4));
+      if (FUSED) *reinterpret_cast<float4*>(op + 4 * o) = b;
+      v16[i4 * K2BQ_STR + c] = half_round(b.x), v16[(i4 + 1) * K2BQ_STR + c] = half_round(b.y);
+      v16[(i4 + 2) * K2BQ_STR + c] = half_round(b.z), v16[(i4 + 3) * K2BQ_STR + c] = half_round(b.w);
+    }
+    if (!FUSED)
+      for (int o = tid; o < 128 * RANK; o += QP_THREADS) op[(o % RANK) * K2BQ_STR + o / RANK] = __half2float(cblk[k2b_coef_idx(1, o / RANK, o % RANK, RANK)]);
+  }
+  __syncthreads();
+
+  // ---- coefficients ----
+  if (FUSED) {
+    constexpr int NI = RANK / 8;  // basis vectors per thread
+    const int rg = tid >> 3, iq = tid & 7;
+    float acc[4][NI];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < NI; ++b) acc[a][b] = 0.f;
+#pragma unroll 8
+    for (int c = 0; c < HEAD_DIM; ++c) {
+      const float4 m4 = *reinterpret_cast<const float4*>(Ms + c * K2BQ_STR + 4 * rg);
+      const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+      float w[NI];
+      if constexpr (NI == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(op + c * RANK + 4 * iq);
+        w[0] = t.x, w[1] = t.y, w[2] = t.z, w[3] = t.w;
+      } else {
+        const float2 t = *reinterpret_cast<const float2*>(op + c * RANK + 2 * iq);
+        w[0] = t.x, w[1] = t.y;
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < NI; ++b) acc[a][b] = fmaf(m[a], w[b], acc[a][b]);
+    }
+    __syncthreads();  // the basis rows are dead: the coefficients take their place
+    __half hv[4][NI];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < NI; ++b) hv[a][b] = __float2half_rn(acc[a][b]);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {  // the thread's vectors of a row are adjacent in the operand order
+      __half* dst = cblk + k2b_coef_idx(1, 4 * rg + a, NI * iq, RANK);
+      if (vec & 2) {
+        if constexpr (NI == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(h2_as_u32(__halves2half2(hv[a][0], hv[a][1])), h2_as_u32(__halves2half2(hv[a][2], hv[a][3])));
+        else *reinterpret_cast<uint32_t*>(dst) = h2_as_u32(__halves2half2(hv[a][0], hv[a][1]));
+      } else {
+#pragma unroll
+        for (int b = 0; b < NI; ++b) dst[b] = hv[a][b];
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NI; ++b)
+      *reinterpret_cast<float4*>(op + (NI * iq + b) * K2BQ_STR + 4 * rg) =
+          make_float4(__half2float(hv[0][b]), __half2float(hv[1][b]), __half2float(hv[2][b]), __half2float(hv[3][b]));
+    __syncthreads();
+  }
+
+  // ---- keys ----
+  const float qmax = (float)((1 << (g.kbits - 1)) - 1);
+  {
+    const int rg = lane & 15, j0 = 16 * warp + 8 * (lane >> 4);
+    float res[8][8];  // [row][channel]: L, then M - L
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) res[a][b] = 0.f;
+#pragma unroll 4
+    for (int i = 0; i < RANK; ++i) {
+      const float4 ua = *reinterpret_cast<const float4*>(op + i * K2BQ_STR + 4 * rg), ub = *reinterpret_cast<const float4*>(op + i * K2BQ_STR + 64 + 4 * rg);
+      const float4 va = *reinterpret_cast<const float4*>(v16 + i * K2BQ_STR + j0), vb = *reinterpret_cast<const float4*>(v16 + i * K2BQ_STR + j0 + 4);
+      const float u[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w}, w[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int b = 0; b < 8; ++b) res[a][b] = fmaf(u[a], w[b], res[a][b]);
+    }
+    float am[2][8];  // absmax by half of the page
+#pragma unroll
+    for (int b = 0; b < 8; ++b)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const float4 m4 = *reinterpret_cast<const float4*>(Ms + (j0 + b) * K2BQ_STR + 64 * hf + 4 * rg);
+        res[4 * hf][b] = m4.x - res[4 * hf][b], res[4 * hf + 1][b] = m4.y - res[4 * hf + 1][b];
+        res[4 * hf + 2][b] = m4.z - res[4 * hf + 2][b], res[4 * hf + 3][b] = m4.w - res[4 * hf + 3][b];
+        float x = fmaxf(fmaxf(fabsf(res[4 * hf][b]), fabsf(res[4 * hf + 1][b])), fmaxf(fabsf(res[4 * hf + 2][b]), fabsf(res[4 * hf + 3][b])));
+#pragma unroll
+        for (int m = 1; m <= 4; m <<= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, m));
+        am[hf][b] = x;  // of 32 tokens
+      }
+    if (g.group >= 64)
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        am[0][b] = fmaxf(am[0][b], __shfl_xor_sync(0xffffffffu, am[0][b], 8));
+        am[1][b] = fmaxf(am[1][b], __shfl_xor_sync(0xffffffffu, am[1][b], 8));
+        if (g.group == 128) am[0][b] = am[1][b] = fmaxf(am[0][b], am[1][b]);
+      }
+    {  // lane rg: channel j0 + (rg & 7); a block of 32 tokens is (half, rg >> 3), lane rg and rg ^ 8 hold its two blocks of each half
+      float a0 = am[0][0], a1 = am[1][0];
+#pragma unroll
+      for (int b = 1; b < 8; ++b)
+        if ((rg & 7) == b) a0 = am[0][b], a1 = am[1][b];
+      __half* kscale = reinterpret_cast<__half*>(blk + k2b_off_kscale(128));
+      const int c = j0 + (rg & 7), per = g.group >> 5;
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int tb = 2 * hf + (rg >> 3);  // 32-token block
+        const float s = fmaxf(hf ? a1 : a0, 1e-12f) / qmax;
+        ksc[tb * HEAD_DIM + c] = s, kinv[tb * HEAD_DIM + c] = s < 8e37f ? 1.f / s : __int_as_float(0x7fffffff);  // NaN where 1 / s is subnormal: divided
+        if (tb % per == 0) kscale[k2b_kscale_idx(1, tb / per, c)] = __float2half_rn(s);
+      }
+    }
+    __syncthreads();  // scales visible; operands dead: the words take their place
+    float far = 0.f;
+    uint32_t word[8];
+    const F2 magic = f2_pack(K2BQ_MAGIC, K2BQ_MAGIC), unmagic = f2_pack(8.f - K2BQ_MAGIC, 8.f - K2BQ_MAGIC), minus1 = f2_pack(-1.f, -1.f), eight = f2_pack(8.f, 8.f);
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int o = (2 * hf + (rg >> 3)) * HEAD_DIM + j0;
+      const ulonglong2 ia = *reinterpret_cast<const ulonglong2*>(kinv + o), ib = *reinterpret_cast<const ulonglong2*>(kinv + o + 4);
+      F2 inv[4];
+      inv[0].v = ia.x, inv[1].v = ia.y, inv[2].v = ib.x, inv[3].v = ib.y;
+#pragma unroll
+      for (int a = 4 * hf; a < 4 * hf + 4; ++a) {
+        F2 acc = f2_pack(8388608.f, 8388608.f);  // 2^23: the sum sits in the low bits
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const F2 t = f2_mul(f2_pack(res[a][2 * i], res[a][2 * i + 1]), inv[i]);
+          const F2 q8 = f2_add(f2_add(t, magic), unmagic);  // code + 8
+          float d0, d1;
+          f2_unpack(f2_fma(q8, minus1, f2_add(t, eight)), d0, d1);
+          far = max_nan(far, max_nan(fabsf(d0), fabsf(d1)));
+          acc = i == 0 ? f2_add(acc, q8) : f2_fma(q8, f2_pack((float)(1 << (4 * i)), (float)(1 << (4 * i))), acc);
+        }
+        float lo, hi;
+        f2_unpack(acc, lo, hi);
+        word[a] = prmt(__float_as_uint(lo), __float_as_uint(hi), 0x5410u) ^ 0x88888888u;
+      }
+    }
+    uint32_t* kw = reinterpret_cast<uint32_t*>(op);
+    const int cc = j0 & 63, unit0 = (cc >> 4) * 128, j = 2 * (j0 >> 6) + ((cc & 15) >> 3);
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int u = unit0 + 64 * (a >> 2) + 4 * rg + (a & 3);
+      kw[(u ^ ((u >> 2) & 7)) * 4 + j] = word[a];  // 16-byte units swizzled: the lanes' rows lie in different banks
+    }
+    if (!(far < 0.5f - K2BQ_NEAR)) {  // rare; the residuals go through this thread's own cells of the key page
+#pragma unroll
+      for (int b = 0; b < 8; ++b)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+          *reinterpret_cast<float4*>(Ms + (j0 + b) * K2BQ_STR + 64 * hf + 4 * rg) = make_float4(res[4 * hf][b], res[4 * hf + 1][b], res[4 * hf + 2][b], res[4 * hf + 3][b]);
+#pragma unroll 1
+      for (int a = 0; a < 8; ++a) {
+        const int r = 64 * (a >> 2) + 4 * rg + (a & 3), u = unit0 + r;
+        uint32_t w = 0;
+#pragma unroll 1
+        for (int b = 0; b < 8; ++b) {
+          const int code = (int)k2b_code_divided(Ms[(j0 + b) * K2BQ_STR + r], ksc[(r >> 5) * HEAD_DIM + j0 + b], qmax);
+          w |= ((uint32_t)code & 0xFu) << (16 * (b & 1) + 4 * (b >> 1));
+        }
+        kw[(u ^ ((u >> 2) & 7)) * 4 + j] = w;
+      }
+    }
+  }
+  __syncthreads();
+  {
+    uint32_t* kres = reinterpret_cast<uint32_t*>(blk);
+    const uint4* kw = reinterpret_cast<const uint4*>(op);
+    for (int u = tid; u < 512; u += QP_THREADS) {
+      const uint4 w = kw[u ^ ((u >> 2) & 7)];
+      if (vec & 2) reinterpret_cast<uint4*>(kres)[u] = w;
+      else kres[4 * u] = w.x, kres[4 * u + 1] = w.y, kres[4 * u + 2] = w.z, kres[4 * u + 3] = w.w;
+    }
+  }
+  // ---- values, over the keys ----
+  uint32_t* vw = reinterpret_cast<uint32_t*>(blk + k2b_off_vcode(128, g.group));
+  __half* vnorm = reinterpret_cast<__half*>(blk + k2b_off_vnorm(128, g.group));
+  if constexpr (sizeof(T) == 2) {
+    uint32_t* words = reinterpret_cast<uint32_t*>(smem + VQ_STAGE_BYTES);
+    float* norms = reinterpret_cast<float*>(smem + VQ_STAGE_BYTES + VQ_WORDS_BYTES);
+    vq_stage<T>(vsrc, stride_tok, vec & 1, smem, tid);
+    vq_quant_page<T>(smem, words, norms, reinterpret_cast<uint32_t*>(norms + 128), signs, codebook, vnorm, tid);
+    __syncthreads();
+    for (int w = tid; w < 1024; w += QP_THREADS) vw[w] = words[w];
+  } else {  // float32 sources: every token by the exact sequence
+    uint8_t* vcode = smem;  // [128 tokens][128]
+    const float c0 = codebook[0], c1 = codebook[1], c2 = codebook[2], c3 = codebook[3];
+    const float m0 = (c0 + c1) / 2.f, m1 = (c1 + c2) / 2.f, m2 = (c2 + c3) / 2.f;
+    float sg[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sg[i] = signs[4 * lane + i];
+#pragma unroll 2
+    for (int r = warp; r < 128; r += QP_THREADS / 32) {
+      float x[4], n;
+      load4_as_float<T>(vsrc + r * stride_tok + 4 * lane, (vec & 1) != 0, x);
+      *reinterpret_cast<uint32_t*>(vcode + r * HEAD_DIM + 4 * lane) = quant_value_token(x, sg, m0, m1, m2, lane, n);
+      if (lane == 0) vnorm[r] = __float2half_rn(n);
+    }
+    __syncthreads();
+    for (int w = tid; w < 1024; w += QP_THREADS) {
+      const int j = w & 3, c = (w >> 2) & 127, cc = w >> 9;
+      uint32_t word = 0;
+#pragma unroll
+      for (int tau = 0; tau < 16; ++tau)
+        word |= (uint32_t)vcode[(64 * cc + 16 * j + tau) * HEAD_DIM + c] << (tau < 8 ? 4 * tau : 4 * (tau - 8) + 2);
+      vw[w] = word;
+    }
   }
 }
 
@@ -680,6 +946,28 @@ static int launch_quant(const K2bGeom& gg, const T* k_pre, const T* v, int64_t s
   return check_launch("bmxk_k2b_append(quantize)");
 }
 
+template <typename T, int RANK, bool FUSED>
+static int launch_quant_rows(const K2bGeom& gg, const T* k_pre, const T* v, int64_t ss, int64_t sh, int64_t st, const float* basis,
+                             const float* signs, const float* codebook, const int32_t* slots, int n_seq, int n_pages, uint8_t* pages,
+                             __half* coefs, cudaStream_t s) {
+  constexpr int smem = K2bQuantSmem<RANK>::BYTES;
+  static PerDeviceOnce configured;
+  if (configured.first()) {
+    const cudaError_t e = cudaFuncSetAttribute(k2b_quant_rows_kernel<T, RANK, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+      configured.retract();
+      set_error("bmxk_k2b_append: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      return BMXK_ERR_CUDA;
+    }
+  }
+  constexpr int64_t PER = 16 / sizeof(T);  // bit 0: sixteen-byte loads of every row; bit 1: wide stores
+  const int loads = ((uintptr_t)k_pre | (uintptr_t)v) % 16 == 0 && (n_seq == 1 || ss % PER == 0) && (gg.h_kv == 1 || sh % PER == 0) && st % PER == 0;
+  const int vec = loads | (((uintptr_t)pages | (uintptr_t)coefs) % 16 == 0 ? 2 : 0);
+  k2b_quant_rows_kernel<T, RANK, FUSED><<<n_seq * n_pages * gg.h_kv, QP_THREADS, smem, s>>>(gg, k_pre, v, ss, sh, st, basis, signs, codebook, slots,
+                                                                                           n_pages, pages, coefs, vec);
+  return check_launch("bmxk_k2b_append(quantize)");
+}
+
 template <typename T>
 static int append_impl(const bmxk_k2b_geom* g, const void* k_pre, const void* v, int64_t ss, int64_t sh, int64_t st,
                        const float* basis, const float* signs, const float* codebook, const int32_t* slots, int n_seq,
@@ -707,6 +995,14 @@ static int append_impl(const bmxk_k2b_geom* g, const void* k_pre, const void* v,
 #define BMXK_LAUNCH_QUANT(PAGE, FUSED)                                                                                              \
   launch_quant<T, PAGE, FUSED>(gg, (const T*)k_pre, (const T*)v, ss, sh, st, basis, signs, codebook, slots, items, n_pages, \
                                (uint8_t*)pages, (__half*)coefs, vec ? 1 : 0, s)
+  if (g->layout == 1) {
+#define BMXK_LAUNCH_ROWS(RANK, FUSED)                                                                                                    \
+  launch_quant_rows<T, RANK, FUSED>(gg, (const T*)k_pre, (const T*)v, ss, sh, st, basis, signs, codebook, slots, n_seq, n_pages,          \
+                                    (uint8_t*)pages, (__half*)coefs, s)
+    if (g->rank == 32) return fused ? BMXK_LAUNCH_ROWS(32, true) : BMXK_LAUNCH_ROWS(32, false);
+    return fused ? BMXK_LAUNCH_ROWS(16, true) : BMXK_LAUNCH_ROWS(16, false);
+#undef BMXK_LAUNCH_ROWS
+  }
   if (g->page == 128) return fused ? BMXK_LAUNCH_QUANT(128, true) : BMXK_LAUNCH_QUANT(128, false);
   return fused ? BMXK_LAUNCH_QUANT(64, true) : BMXK_LAUNCH_QUANT(64, false);
 #undef BMXK_LAUNCH_QUANT

@@ -98,11 +98,6 @@ struct RtnSrc<float> {
   static __device__ __forceinline__ uint32_t halves(float, float) { return 0u; }
   static __device__ __forceinline__ bool plain(float) { return true; }
 };
-__device__ __forceinline__ float max_nan(float a, float b) {
-  float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
 // Two codes plus `offset` (8 or 2), times weight, added to acc; `far`: the largest distance from a rounded value so far.
 __device__ __forceinline__ F2 rtn_add_codes(F2 acc, float2 x, F2 inv, float offset, float weight, float& far) {
   const F2 t = f2_fma(f2_pack(x.x, x.y), inv, f2_pack(offset, offset));
