@@ -414,7 +414,7 @@ static int prefill_impl(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t 
                         const void* basis_f16, const int32_t* page_table, int table_stride, const int32_t* n_pages, int batch,
                         const void* rope_cos, const void* rope_sin, int64_t pos_offset, const void* k_tail, const void* v_tail,
                         const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
-                        int32_t* status, void* out, int n_split, void* workspace, size_t workspace_bytes, void* stream);
+                        int32_t* status, void* out, int n_split, int rope_pages, void* workspace, size_t workspace_bytes, void* stream);
 
 int bmxk_k2b_prefill(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t q_pos0, const void* pages, const void* coefs,
                      const void* basis_f16, const int32_t* page_table, int table_stride, const int32_t* n_pages, int batch,
@@ -422,7 +422,7 @@ int bmxk_k2b_prefill(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t q_p
                      const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
                      int32_t* status, void* out, void* stream) {
   return prefill_impl(g, q, n_q, q_pos0, pages, coefs, basis_f16, page_table, table_stride, n_pages, batch, rope_cos, rope_sin, pos_offset,
-                      k_tail, v_tail, tail_len, tail_cap, v_lut, signs, sm_scale, status, out, 1, nullptr, 0, stream);
+                      k_tail, v_tail, tail_len, tail_cap, v_lut, signs, sm_scale, status, out, 1, 0, nullptr, 0, stream);
 }
 
 int bmxk_k2b_prefill_split(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t q_pos0, const void* pages, const void* coefs,
@@ -431,7 +431,20 @@ int bmxk_k2b_prefill_split(const bmxk_k2b_geom* g, const void* q, int n_q, int64
                            const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
                            int32_t* status, void* out, int n_split, void* workspace, size_t workspace_bytes, void* stream) {
   return prefill_impl(g, q, n_q, q_pos0, pages, coefs, basis_f16, page_table, table_stride, n_pages, batch, rope_cos, rope_sin, pos_offset,
-                      k_tail, v_tail, tail_len, tail_cap, v_lut, signs, sm_scale, status, out, n_split, workspace, workspace_bytes, stream);
+                      k_tail, v_tail, tail_len, tail_cap, v_lut, signs, sm_scale, status, out, n_split, 0, workspace, workspace_bytes, stream);
+}
+
+size_t bmxk_k2b_prefill_rope_bytes(int rope_pages) { return rope_pages > 0 ? (size_t)rope_pages * ROPE_FRAG_UINT4 * 16 : 0; }
+
+int bmxk_k2b_prefill_rope(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t q_pos0, const void* pages, const void* coefs,
+                          const void* basis_f16, const int32_t* page_table, int table_stride, const int32_t* n_pages, int batch,
+                          const void* rope_cos, const void* rope_sin, int64_t pos_offset, const void* k_tail, const void* v_tail,
+                          const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
+                          int32_t* status, void* out, int n_split, int rope_pages, void* workspace, size_t workspace_bytes, void* stream) {
+  BMXK_REQUIRE(rope_pages >= 0 && rope_pages <= (1 << 24), "bmxk_k2b_prefill_rope: rope_pages=%d", rope_pages);
+  return prefill_impl(g, q, n_q, q_pos0, pages, coefs, basis_f16, page_table, table_stride, n_pages, batch, rope_cos, rope_sin, pos_offset,
+                      k_tail, v_tail, tail_len, tail_cap, v_lut, signs, sm_scale, status, out, n_split, rope_pages, workspace, workspace_bytes,
+                      stream);
 }
 
 }  // extern "C"
@@ -440,7 +453,7 @@ static int prefill_impl(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t 
                         const void* basis_f16, const int32_t* page_table, int table_stride, const int32_t* n_pages, int batch,
                         const void* rope_cos, const void* rope_sin, int64_t pos_offset, const void* k_tail, const void* v_tail,
                         const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
-                        int32_t* status, void* out, int n_split, void* workspace, size_t workspace_bytes, void* stream) {
+                        int32_t* status, void* out, int n_split, int rope_pages, void* workspace, size_t workspace_bytes, void* stream) {
   BMXK_REQUIRE(g != nullptr, "bmxk_k2b_prefill: null geometry");
   BMXK_REQUIRE(g->layout == 1 && g->page == 128, "bmxk_k2b_prefill: layout=%d page=%d (row-order pools of 128-token pages only)", g->layout,
                g->page);
@@ -478,11 +491,13 @@ static int prefill_impl(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t 
   const bool t5 = g_prefill_kernel.load(std::memory_order_relaxed) == 0 && aligned16;
   BMXK_REQUIRE(n_split >= 1 && n_split <= 64, "bmxk_k2b_prefill_split: n_split=%d must be in 1..64", n_split);
   if (!t5) n_split = 1;  // the split is the tcgen05 kernel's; the mma.sync kernel walks every page of a block in one CTA
+  if (!t5) rope_pages = 0;
   prm.n_split = n_split, prm.part = (float*)workspace;
+  const size_t part_bytes = bmxk_k2b_prefill_workspace_bytes(g, n_q, batch, n_split), need = part_bytes + bmxk_k2b_prefill_rope_bytes(rope_pages);
+  prm.rope_pages = rope_pages, prm.rope_frag = rope_pages > 0 ? reinterpret_cast<uint4*>((uint8_t*)workspace + part_bytes) : nullptr;
+  BMXK_REQUIRE(need == 0 || (workspace && workspace_bytes >= need && ((uintptr_t)workspace & 15) == 0),
+               "bmxk_k2b_prefill_split: workspace of %zu bytes needed (16-byte aligned), %zu given", need, workspace_bytes);
   if (n_split > 1) {
-    const size_t need = bmxk_k2b_prefill_workspace_bytes(g, n_q, batch, n_split);
-    BMXK_REQUIRE(workspace && workspace_bytes >= need && ((uintptr_t)workspace & 15) == 0,
-                 "bmxk_k2b_prefill_split: workspace of %zu bytes needed (16-byte aligned), %zu given", need, workspace_bytes);
     BMXK_REQUIRE((int64_t)grid.x * n_split <= 0x7fffffff && (int64_t)batch * g->h_kv * g->n_q_groups * n_q <= 0x7fffffff,
                  "bmxk_k2b_prefill_split: n_q=%d batch=%d n_split=%d too large", n_q, batch, n_split);
     return launch_prefill_t5(prm, dim3(grid.x * (unsigned)n_split, grid.y, grid.z), s);

@@ -101,7 +101,8 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
 
 }  // namespace
 
-template <int RANK>
+// FRAG: the rotation tables of every page come from the rearranged copy (p.rope_frag)
+template <int RANK, bool FRAG>
 __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const PrefillParams p) {
   constexpr int KS = RANK / 16;
   constexpr int COEF_BYTES = 128 * RANK * 2;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
   const int64_t pq_max = p.q_pos0 + min(i0 + PP, p.n_q) - 1;           // last one
   const int n_pg = p.n_pages[b];
   const int64_t vis = pq_max - p.pos_offset;
-  const int NPv = (vis < 0) ? 0 : (int)min((int64_t)n_pg, vis / 128 + 1);  // pages whose first token the last position sees
+  const int NPv = (vis < 0) ? 0 : (int)min((int64_t)(FRAG ? min(n_pg, p.rope_pages) : n_pg), vis / 128 + 1);  // pages whose first token the last position sees
   // this CTA's share of them: pages T0 .. T0 + NP - 1; the window goes with the last share
   const int per_share = (NPv + n_split - 1) / n_split;
   const int T0 = min(NPv, share * per_share), NP = min(NPv, T0 + per_share) - T0;
@@ -196,13 +197,21 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
     const __half* kt = p.k_tail + ((int64_t)b * g.h_kv + h) * p.tail_cap * HEAD_DIM;
     const float inv_scale = 1.0f / p.scale_log2;
     // cos / sin of this token's rotary pairs 16k .. 16k+15 for both chunks, fetched one tile ahead: the registers of a
-    // chunk are reloaded for the next tile as soon as the chunk is done, so the loads have a whole tile to land
+    // chunk are reloaded for the next tile as soon as the chunk is done, so the loads have a whole tile to land.
+    // From the tables themselves a warp's load touches 32 rows of 256 bytes; from the rearranged copy it is 512 bytes on end.
     uint4 cs4[2][2], sn4[2][2];
+    const uint4* frag0 = FRAG ? p.rope_frag + (int64_t)T0 * ROPE_FRAG_UINT4 + (k0 * 4 + wq) * 64 + lane : nullptr;
     auto load_rope = [&](int n, int kk) {
-      const int64_t pos = page_pos0 + (int64_t)n * 128 + row;
-      const uint4* pc = reinterpret_cast<const uint4*>(p.rope_cos + pos * HEAD_DIM + 16 * (k0 + kk));
-      const uint4* ps = reinterpret_cast<const uint4*>(p.rope_sin + pos * HEAD_DIM + 16 * (k0 + kk));
-      cs4[kk][0] = pc[0], cs4[kk][1] = pc[1], sn4[kk][0] = ps[0], sn4[kk][1] = ps[1];
+      if constexpr (FRAG) {
+        const uint4* pc = frag0 + (int64_t)n * ROPE_FRAG_UINT4 + kk * 256;
+        const uint4* ps = pc + ROPE_FRAG_UINT4 / 2;
+        cs4[kk][0] = pc[0], cs4[kk][1] = pc[32], sn4[kk][0] = ps[0], sn4[kk][1] = ps[32];
+      } else {
+        const int64_t pos = page_pos0 + (int64_t)n * 128 + row;
+        const uint4* pc = reinterpret_cast<const uint4*>(p.rope_cos + pos * HEAD_DIM + 16 * (k0 + kk));
+        const uint4* ps = reinterpret_cast<const uint4*>(p.rope_sin + pos * HEAD_DIM + 16 * (k0 + kk));
+        cs4[kk][0] = pc[0], cs4[kk][1] = pc[1], sn4[kk][0] = ps[0], sn4[kk][1] = ps[1];
+      }
     };
     if (NP > 0) load_rope(0, 0), load_rope(0, 1);
     int s = 0;
@@ -731,19 +740,31 @@ static size_t p5_smem_bytes(int rank, int group) {
          (size_t)128 * rank * 2 + 128 * 4 + sizeof(P5Smem) + 128;
 }
 
-template <int RANK>
+template <int RANK, bool FRAG>
 static int launch_p5(const PrefillParams& prm, dim3 grid, size_t smem, cudaStream_t s) {
   static PerDeviceOnce configured;
   if (configured.first()) {
-    cudaError_t e = cudaFuncSetAttribute(k2b_prefill_t5_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute((k2b_prefill_t5_kernel<RANK, FRAG>), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) {
       configured.retract();
       set_error("bmxk_k2b_prefill: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       return BMXK_ERR_CUDA;
     }
   }
-  k2b_prefill_t5_kernel<RANK><<<grid, P5_THREADS, smem, s>>>(prm);
+  k2b_prefill_t5_kernel<RANK, FRAG><<<grid, P5_THREADS, smem, s>>>(prm);
   return check_launch("bmxk_k2b_prefill(tcgen05)");
+}
+
+// Rotation tables in the order of the key warps' reads.  Every block of query positions and every head walks the same pages, and
+// reading the tables row by row (16 bytes out of each of 32 rows per load) kept the L1 tag stage 79 % busy and the key warps
+// waiting.  The copy costs 256 bytes and about 0.25 ns per position.  One block per 256 of a page's 2048 pieces.
+__global__ void __launch_bounds__(256) rope_fragments_kernel(const __half* __restrict__ rope_cos, const __half* __restrict__ rope_sin,
+                                                             int64_t pos_offset, uint4* __restrict__ frag) {
+  const int u = (blockIdx.x & 7) * 256 + threadIdx.x, page = blockIdx.x >> 3;
+  const int lane = u & 31, half = (u >> 5) & 1, wq = (u >> 6) & 3, chunk = (u >> 8) & 3;
+  const __half* t = (u >> 10) ? rope_sin : rope_cos;
+  const int64_t pos = pos_offset + (int64_t)page * 128 + 32 * wq + lane;
+  frag[(int64_t)page * ROPE_FRAG_UINT4 + u] = reinterpret_cast<const uint4*>(t + pos * HEAD_DIM)[2 * chunk + half];
 }
 
 // out[row] = sum_s 2^(m_s - M) O_s / sum_s 2^(m_s - M) l_s over the n_split partial records of the row; one block of 128
@@ -765,7 +786,15 @@ __global__ void __launch_bounds__(128) prefill_merge_kernel(const float* __restr
 int launch_prefill_t5(const PrefillParams& prm, dim3 grid, cudaStream_t s) {
   const size_t smem = p5_smem_bytes(prm.g.rank, prm.g.group);
   BMXK_REQUIRE(smem <= 227 * 1024, "bmxk_k2b_prefill: rank=%d group=%d needs %zu bytes of shared memory", prm.g.rank, prm.g.group, smem);
-  const int rc = prm.g.rank == 32 ? launch_p5<32>(prm, grid, smem, s) : launch_p5<16>(prm, grid, smem, s);
+  int rc;
+  if (prm.rope_frag) {
+    rope_fragments_kernel<<<(unsigned)prm.rope_pages * 8, 256, 0, s>>>(prm.rope_cos, prm.rope_sin, prm.pos_offset, prm.rope_frag);
+    rc = check_launch("bmxk_k2b_prefill(rope fragments)");
+    if (rc) return rc;
+    rc = prm.g.rank == 32 ? launch_p5<32, true>(prm, grid, smem, s) : launch_p5<16, true>(prm, grid, smem, s);
+  } else {
+    rc = prm.g.rank == 32 ? launch_p5<32, false>(prm, grid, smem, s) : launch_p5<16, false>(prm, grid, smem, s);
+  }
   if (rc != BMXK_OK || prm.n_split <= 1) return rc;
   const int64_t rows = (int64_t)grid.z * prm.g.h_kv * prm.g.n_q_groups * prm.n_q;
   prefill_merge_kernel<<<(unsigned)rows, 128, 0, s>>>(prm.part, prm.n_split, prm.out);

@@ -33,7 +33,12 @@ struct PrefillParams {
   // maximum (log2 units), sum of weights, 2 unused -- to `part`; prefill_merge_kernel combines them into `out`.
   int n_split;
   float* part;
+  // Rotation tables of the first rope_pages pages in the order the key warps read them (tcgen05 kernel, see
+  // rope_fragments_kernel), or null: the tables are read where they are.
+  uint4* rope_frag;
+  int rope_pages;
 };
+constexpr int ROPE_FRAG_UINT4 = 2048;  // per page: [cos, sin][chunk of 16 pairs][32 tokens x 4][half of the chunk][lane]
 constexpr int PF_PART_STRIDE = 132;  // floats per (row, share) record: 16-byte aligned rows
 
 // tcgen05 prefill kernel (k2b_prefill_t5.cu); the mma.sync kernel's grid with x multiplied by n_split.  Needs q, out and the

@@ -173,6 +173,17 @@ int bmxk_k2b_prefill_split(const bmxk_k2b_geom* g, const void* q, int n_q, int64
                            const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
                            int32_t* status, void* out, int n_split, void* workspace, size_t workspace_bytes, void* stream);
 
+/* bmxk_k2b_prefill_split (n_split = 1: unsplit) that first rearranges the rotation tables of the positions pos_offset ..
+ * pos_offset + 128 * rope_pages - 1 into the order its key warps read, behind the partial records in `workspace`
+ * (bmxk_k2b_prefill_workspace_bytes + bmxk_k2b_prefill_rope_bytes).  Worth its few microseconds when many blocks and heads walk the
+ * same pages.  rope_pages has to cover every committed page that a row of q sees.  Same results. */
+size_t bmxk_k2b_prefill_rope_bytes(int rope_pages);
+int bmxk_k2b_prefill_rope(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t q_pos0, const void* pages, const void* coefs,
+                          const void* basis_f16, const int32_t* page_table, int table_stride, const int32_t* n_pages, int batch,
+                          const void* rope_cos, const void* rope_sin, int64_t pos_offset, const void* k_tail, const void* v_tail,
+                          const int32_t* tail_len, int tail_cap, const uint32_t* v_lut, const float* signs, float sm_scale,
+                          int32_t* status, void* out, int n_split, int rope_pages, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Which kernel bmxk_k2b_prefill launches (process-wide; no counterpart in bmx).  0 (default): the tcgen05 kernel when q
  * and out are 16-byte aligned, else the mma.sync kernel; 1: always the mma.sync kernel.  Both give the same attention
  * within the path's tolerance. */

@@ -287,3 +287,30 @@ def test_cache_prefill_takes_the_paged_route_and_agrees_with_the_dense_one():
     # layer 2 quantizes keys and values that come out of layer 1's attention, where the two routes differ in the last fp16
     # bits, and 2-bit codes are discontinuous: a few codes move, so the bound here is looser than the kernel's own (1e-3)
     assert diff < 5e-2
+
+
+@pytest.mark.parametrize("rank,G,n_q,tokens,n_split", [(32, 4, 70, 900, 1), (16, 8, 33, 1500, 3), (32, 1, 200, 129 + 128, 1), (16, 2, 5, 4000, 8), (32, 4, 300, 300, 1)])
+def test_rearranged_rotation_tables_change_nothing(rank, G, n_q, tokens, n_split):
+    """The prefill kernel gives the same bits from the rotation tables and from their rearranged copy."""
+    from bmx_b200 import kernels as K
+    from bmx_b200.engine import K2bLayerState
+    from bmx_b200.rope import default_rope_tables
+
+    dev = torch.device("cuda:0")
+    h, B = 3, 2
+    gen = torch.Generator(device=dev).manual_seed(tokens)
+    cos, sin = (t.half() for t in default_rope_tables(5e5, 128, tokens + 256, device=dev))
+    st = K2bLayerState(K.k2b_geom(h, G, 128, rank, 64, h), B, tokens, 100, dev, cos, sin)
+    st.set_basis(torch.randn(h * 128, rank, generator=gen, device=dev) / 11)
+    k, v = (torch.randn(B, h, tokens, 128, generator=gen, device=dev).half() for _ in range(2))
+    st.append(k, k, v)
+    q = torch.randn(B, h * G, n_q, 128, generator=gen, device=dev).half()
+    pages = st.committed // 128
+
+    def run(rope_pages):
+        return K.k2b_prefill(st.pool, q, tokens - n_q, st.basis_f16, st.page_table, st.n_pages_dev, cos, sin, st.k_win, st.v_win, st.tail_len_dev,
+                             st.v_lut, st.signs, 128 ** -0.5, st.workspace.view(torch.int32), n_split=n_split, rope_pages=rope_pages)
+
+    want = run(0)
+    assert torch.equal(run(pages), want) and (pages == 0 or bool(want.abs().sum() > 0))
+    K.check_status(st.workspace)
