@@ -42,11 +42,11 @@ namespace bmxk {
 
 namespace {
 
-constexpr int P5_THREADS = 768;  // warps 0-7 key, 8-11 softmax, 12 copies + U1, 13 U2, 14 U3 (15 idle), 16-23 value
+constexpr int P5_THREADS = 896;  // warps 0-7 key, 8-15 softmax (8-11 first halves, 12-15 second halves), 16 copies + U1, 17 U2, 18 U3 (19 idle), 20-27 value
 constexpr int P5_STAGES = 3;
 // Registers per thread after each group of four warps resizes itself; the pool is what the launch handed out.
-constexpr int P5_REG_LAUNCH = 80, P5_REG_KEY = 112, P5_REG_SOFTMAX = 112, P5_REG_SERVICE = 48, P5_REG_VALUE = 48;
-static_assert(8 * P5_REG_KEY + 4 * P5_REG_SOFTMAX + 4 * P5_REG_SERVICE + 8 * P5_REG_VALUE <= 24 * P5_REG_LAUNCH,
+constexpr int P5_REG_LAUNCH = 72, P5_REG_KEY = 96, P5_REG_SOFTMAX = 96, P5_REG_SERVICE = 40, P5_REG_VALUE = 40;
+static_assert(8 * P5_REG_KEY + 8 * P5_REG_SOFTMAX + 4 * P5_REG_SERVICE + 8 * P5_REG_VALUE <= 28 * P5_REG_LAUNCH,
               "register split exceeds the CTA's pool");
 // A [128 rows][144 K] fp16 operand in the unswizzled K-major form: 8-row x 16-byte core matrices, the 18 core matrices
 // of one row group 128 bytes apart along K, row groups 2304 bytes apart.  K index 128 / 129: the norm pair (see above).
@@ -64,9 +64,11 @@ struct P5Smem {
   uint64_t low, sdone[2][2], odone[2];  // completion of U1, of U2 [half][tile parity] and of U3 [half] (tcgen05.commit)
   uint32_t tmem_base;
   // Arrivals, never reset: key warps (8 per tile, counted per tile parity: a key warp may be two tiles ahead of another
-  // one, never two tiles of the same parity), value warps (8), scores read (4 per half tile), weights written (4 per half tile)
+  // one, never two tiles of the same parity); per half: value warps, scores read, weights written (4 each per tile)
   // klcnt: key warps that hold K_low of the tile in registers (U1 of the next tile may start)
-  int kcnt[2], klcnt[2], vcnt, scnt, pcnt;
+  // turn: half tiles whose running maximum is settled, per group of 32 rows (the two softmax warps of a group alternate)
+  int kcnt[2], klcnt[2], vcnt[2], scnt[2], pcnt[2], turn[4];
+  float m[128];  // the running maximum of each row, valid for the halves settled so far
 };
 
 // Per-role wait / work cycle counters of CTA (0, 0, 0), compiled in with -DP5_PROF only: written behind the status words
@@ -147,10 +149,11 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
     for (int s = 0; s < P5_STAGES; ++s) mbar_init(&sh->full[s], 1);
     mbar_init(&sh->low, 1);
     for (int e = 0; e < 2; ++e) mbar_init(&sh->sdone[0][e], 1), mbar_init(&sh->sdone[1][e], 1), mbar_init(&sh->odone[e], 1);
-    sh->kcnt[0] = sh->kcnt[1] = sh->klcnt[0] = sh->klcnt[1] = sh->vcnt = sh->scnt = sh->pcnt = 0;
+    for (int e = 0; e < 2; ++e) sh->kcnt[e] = sh->klcnt[e] = sh->vcnt[e] = sh->scnt[e] = sh->pcnt[e] = 0;
+    for (int e = 0; e < 4; ++e) sh->turn[e] = 0;
     fence_barrier_init();
   }
-  if (warp == 12) {
+  if (warp == 16) {
     tc5::alloc(smem_u32(&sh->tmem_base), TM_COLS);
     tc5::relinquish();
   }
@@ -312,20 +315,20 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       PROF_ADD(4)
     }
     PROF_OUT(16, 6)
-  } else if (warp >= 16) {
+  } else if (warp >= 20) {
     // ===================== value warps: thread = channel, warp = one half (64 tokens) of the tile =====================
     // (levels as stored in the table: the norm is in the weights)
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P5_REG_VALUE));
-    const int wq = warp & 3, cc = (warp - 16) >> 2, ch = 32 * wq + lane;
+    const int wq = warp & 3, cc = (warp - 20) >> 2, ch = 32 * wq + lane;
     uint8_t* vrow = vop + (ch >> 3) * V_SBO + (ch & 7) * 16;
-    __half* vinv = reinterpret_cast<__half*>(vop + 16 * V_SBO + (ch >> 3) * 128) + (ch & 7);  // rows 128 / 129, token = ch (warps 16 - 19)
+    __half* vinv = reinterpret_cast<__half*>(vop + 16 * V_SBO + (ch >> 3) * 128) + (ch & 7);  // rows 128 / 129, token = ch (the threads whose ch lies in their half)
     const __half* vt = p.v_tail + ((int64_t)b * g.h_kv + h) * p.tail_cap * HEAD_DIM;
     int s = 0;
     uint32_t fp = 0;
     PROF_DECL(4)
     for (int n = 0; n < NT; ++n) {
-      // the buffer still feeds U3 of tile n-1
-      if (n >= 1 && !(warp_wait(&sh->odone[0], (uint32_t)(n - 1) & 1u, p.status, 44) && warp_wait(&sh->odone[1], (uint32_t)(n - 1) & 1u, p.status, 44))) break;
+      // this half of the buffer still feeds U3 of the same half of tile n-1
+      if (n >= 1 && !warp_wait(&sh->odone[cc], (uint32_t)(n - 1) & 1u, p.status, 44)) break;
       PROF_ADD(0)
       if (n < NP) {
         if (!warp_wait(&sh->full[s], fp, p.status, 45)) break;
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
           *reinterpret_cast<uint4*>(vrow + (8 * cc + 2 * jw) * 128) = make_uint4(outw[0], outw[1], outw[2], outw[3]);
           *reinterpret_cast<uint4*>(vrow + (8 * cc + 2 * jw + 1) * 128) = make_uint4(outw[4], outw[5], outw[6], outw[7]);
         }
-        if (cc == 0) {  // rows 128 / 129, token = ch: 1 / norm as high part + remainder
+        if ((ch >> 6) == cc) {  // rows 128 / 129, token = ch: 1 / norm as high part + remainder
           const float nj = fmaxf(__half2float(reinterpret_cast<const __half*>(blk + k2b_off_vnorm(128, g.group))[ch]), MIN_NORM);
           const float r = 1.0f / nj;
           const __half rh = __float2half_rn(r);
@@ -371,18 +374,22 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
           }
           *reinterpret_cast<uint4*>(vrow + (8 * cc + i) * 128) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
         }
-        if (cc == 0) vinv[0] = __float2half_rn(1.f), vinv[8] = __float2half_rn(0.f);
+        if ((ch >> 6) == cc) vinv[0] = __float2half_rn(1.f), vinv[8] = __float2half_rn(0.f);
       }
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) smem_add_release(&sh->vcnt, 1);
+      if (lane == 0) smem_add_release(&sh->vcnt[cc], 1);
       PROF_ADD(2)
     }
     PROF_OUT(32, 4)
-  } else if (warp < 12) {
+  } else if (warp < 16) {
     // ===================== softmax warps: thread = attention row = TMEM lane =====================
+    // Two sets of four warps, one per half of the tiles, so that the exponentials of one half overlap the tensor-memory round trips
+    // of the other.  They share one accumulator and hence one running maximum per row: a warp computes its weights with the
+    // maximum it knows, waits for its turn (the other warp of its 32 rows has settled the half before), starts over in the rare
+    // case that the maximum has moved since, raises it if it has to, and settles its own half.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P5_REG_SOFTMAX));
-    const int wq = warp & 3, row = 32 * wq + lane;
+    const int wq = warp & 3, row = 32 * wq + lane, hf = (warp - 8) >> 2;
     const uint32_t tl_ = tmem + ((uint32_t)(32 * wq) << 16);
     const int qi = row / PP, ip = i0 + row % PP;
     const int64_t pq = p.q_pos0 + ip;
@@ -464,18 +471,31 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       return acc;
     };
 
-    // keys of the current half visible to this row / to the CTA's first row: position - first key position + 1
-    int64_t rel = pq - page_pos0 + 1, rel_min = pq_min - page_pos0 + 1;
+    auto turn_is = [&](int u, int where) {  // half tiles 0 .. u-1 are settled; bounded
+      if (smem_load_acquire(&sh->turn[wq]) >= u) return true;
+      const long long t0 = clock64();
+      for (uint32_t spin = 1;; ++spin) {
+        if (smem_load_acquire(&sh->turn[wq]) >= u) return true;
+        if ((spin & 255u) == 0u) {
+          if (*reinterpret_cast<volatile int32_t*>(p.status) != 0) return false;
+          if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
+            if (lane == 0 && atomicCAS(p.status, 0, 1) == 0) p.status[1] = blockIdx.x, p.status[2] = where;
+            return false;
+          }
+        }
+      }
+    };
     PROF_DECL(8)
-    for (int u = 0; u < 2 * NT && alive; ++u) {  // half tile u = (tile n, half hf): tokens 64 hf .. 64 hf + 63
-      const int n = u >> 1, hf = u & 1, e = n & 1;
-      if (u == 2 * NP) rel = pq - tail_pos0 + 1, rel_min = pq_min - tail_pos0 + 1;  // the window's first token follows the last page
+    for (int n = 0; n < NT && alive; ++n) {  // half tile u = (tile n, half hf): tokens 64 hf .. 64 hf + 63
+      const int u = 2 * n + hf, e = n & 1;
+      // keys of the half visible to this row / to the CTA's first row: position - first key position + 1
+      const int64_t key0 = (n < NP ? page_pos0 + (int64_t)n * 128 : tail_pos0 + (int64_t)(n - NP) * 128) + 64 * hf;
+      const int64_t rel = pq - key0 + 1, rel_min = pq_min - key0 + 1;
       const int n_valid = (n < NP) ? 64 : max(0, min(64, tl - (n - NP) * 128 - 64 * hf));
       const bool masked = (rel_min < 64) || (n_valid < 64);                               // the same for the whole CTA
       const int jl = (int)max((int64_t)0, min((int64_t)n_valid, rel));                    // keys [0, jl) of the half are visible to this row
-      rel -= 64, rel_min -= 64;
       const uint32_t tS = tl_ + TM_S + 64 * hf, tP = tl_ + TM_P + 32 * hf;
-      if (u == 2 * NP && NP > 0) {  // first window tile after pages: leave the rotated space of the value codec
+      if (hf == 0 && n == NP && NP > 0) {  // first window tile after pages: leave the rotated space of the value codec
         if (!(warp_wait(&sh->odone[0], (uint32_t)(n - 1) & 1u, p.status, 46) && warp_wait(&sh->odone[1], (uint32_t)(n - 1) & 1u, p.status, 46))) {
           alive = false;
           break;
@@ -490,7 +510,10 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       if (n >= 1 && !warp_wait(&sh->odone[hf], (uint32_t)(n - 1) & 1u, p.status, 48)) { alive = false; break; }
       tc5::fence_after();
       PROF_ADD(2)
-      for (int attempt = 0; attempt < 2; ++attempt) {
+      bool settled_before = smem_load_acquire(&sh->turn[wq]) >= u;  // not needed yet, but if it is so the maximum is final
+      settled_before = __all_sync(0xffffffffu, settled_before);
+      if (settled_before && u > 0) m = sh->m[row];
+      for (;;) {
         uint32_t ra[32], rb[32];
         const float negm = -m;
         tc5::ld32(tS, ra);
@@ -498,6 +521,16 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
         tc5::wait_ld();
         float tmax = weights32(ra, tP, 0, masked, jl, negm, -INFINITY);
         tmax = weights32(rb, tP, 32, masked, jl, negm, tmax);
+        PROF_ADD(3)
+        if (!settled_before) {
+          settled_before = __all_sync(0xffffffffu, turn_is(u, 53));
+          if (!settled_before) { alive = false; break; }
+          const float mc = u > 0 ? sh->m[row] : m;
+          const bool moved = mc != m;
+          m = mc;
+          PROF_ADD(5)
+          if (__any_sync(0xffffffffu, moved)) continue;
+        }
         // Lazy maximum: as long as no score exceeds the running maximum by more than 8 (weights below 2^8) the weights
         // just written stand.  Otherwise the whole warp (TMEM access is warp-wide) rescales its rows of the accumulator
         // once every earlier U3 has finished, and goes through the half again with the new maximum.
@@ -530,18 +563,26 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
         }
       }
       if (!alive) break;
-      PROF_ADD(3)
+      // this half's maximum is settled: the other set may settle the next one
+      sh->m[row] = m;
+      __syncwarp();
+      if (lane == 0) smem_add_release(&sh->turn[wq], 1);
       // every score of the half has been read: U2 of the next tile's same half may overwrite them
       tc5::fence_before();
       __syncwarp();
-      if (lane == 0) smem_add_release(&sh->scnt, 1);
+      if (lane == 0) smem_add_release(&sh->scnt[hf], 1);
       tc5::wait_st();
       tc5::fence_before();
       __syncwarp();
-      if (lane == 0) smem_add_release(&sh->pcnt, 1);
+      if (lane == 0) smem_add_release(&sh->pcnt[hf], 1);
       PROF_ADD(4)
     }
     PROF_OUT(48, 8)
+    if (hf == 1) alive = false;  // the first set finishes the rows
+    if (alive && NT > 0) {
+      alive = __all_sync(0xffffffffu, turn_is(2 * NT, 54));
+      m = sh->m[row];
+    }
 
     // ---- the last U3, the rotation if no window tile undid it, normalise and store ----
     if (alive && NT > 0 && !(warp_wait(&sh->odone[0], (uint32_t)(NT - 1) & 1u, p.status, 49) && warp_wait(&sh->odone[1], (uint32_t)(NT - 1) & 1u, p.status, 49)))
@@ -610,7 +651,7 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P5_REG_SERVICE));
-    // ===================== service warps: 12 copies + U1, 13 U2, 14 U3 (15 idle) =====================
+    // ===================== service warps: 16 copies + U1, 17 U2, 18 U3 (19 idle) =====================
     // Tile n:  copy -> full[n % 3];  A: U1 -> low;  per half hf:  B: U2 -> sdone[hf][n & 1];  C: U3 -> odone[hf].
     // A(n) needs the copy landed and K_low of tile n-1 read by every key warp; B(n, hf) the keys of tile n and the
     // scores of the same half of tile n-1 read; C(n, hf) the weights of the half and the values of tile n; copy(n) the
@@ -634,7 +675,7 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       }
       return false;
     };
-    if (warp == 12) {
+    if (warp == 16) {
       constexpr uint32_t ID_U1 = tc5::idesc_f16_f16(128, 128);
       const uint64_t d_stage = tc5::smem_desc(smem_u32(stage0), 128, AB_SBO), d_b = tc5::smem_desc(smem_u32(bop), 128, AB_SBO);
       const int chd = (g.n_coef_heads == 1) ? 0 : h;
@@ -644,7 +685,8 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       int slot = (NP > 0) ? table[0] : 0;  // page slot of the next copy, fetched one copy ahead
       while (ok && nA < NP) {
         bool progressed = false;
-        const int kc0 = smem_load_acquire(&sh->kcnt[0]), kc1 = smem_load_acquire(&sh->kcnt[1]), vc = smem_load_acquire(&sh->vcnt);
+        const int kc0 = smem_load_acquire(&sh->kcnt[0]), kc1 = smem_load_acquire(&sh->kcnt[1]);
+        const int vc = min(smem_load_acquire(&sh->vcnt[0]), smem_load_acquire(&sh->vcnt[1]));
         const int kl0 = smem_load_acquire(&sh->klcnt[0]), kl1 = smem_load_acquire(&sh->klcnt[1]);
         auto kdone = [&](int t) { return t < 0 || ((t & 1) ? kc1 : kc0) >= 8 * ((t >> 1) + 1); };   // every key warp is through tile t
         auto kldone = [&](int t) { return t < 0 || ((t & 1) ? kl1 : kl0) >= 8 * ((t >> 1) + 1); };  // ... holds K_low of tile t in registers
@@ -663,7 +705,7 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
           progressed = true;
         }
         // ---- copy ----
-        if (nP < NP && (nP < P5_STAGES || (kdone(nP - P5_STAGES) && vc >= 8 * (nP - P5_STAGES + 1)))) {
+        if (nP < NP && (nP < P5_STAGES || (kdone(nP - P5_STAGES) && vc >= 4 * (nP - P5_STAGES + 1)))) {
           uint8_t* st = stage0 + (size_t)sP * STAGE_BYTES;
           if (el) {
             mbar_arrive_expect_tx(&sh->full[sP], (uint32_t)STAGE_BYTES);
@@ -679,15 +721,15 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
         }
         if (stalled(progressed, 40)) ok = false;
       }
-    } else if (warp == 13) {
+    } else if (warp == 17) {
       constexpr uint32_t ID_U2 = tc5::idesc_f16_f32(128, 64);
       const uint64_t d_q = tc5::smem_desc(smem_u32(qop), 128, OP_SBO), d_k = tc5::smem_desc(smem_u32(kop0), 128, OP_SBO);
       int uB = 0;  // half tiles issued
       while (ok && uB < 2 * NT) {
         const int n = uB >> 1, hf = uB & 1;
-        const int kc = smem_load_acquire(&sh->kcnt[n & 1]), sc = smem_load_acquire(&sh->scnt);
+        const int kc = smem_load_acquire(&sh->kcnt[n & 1]), sc = smem_load_acquire(&sh->scnt[hf]);
         bool progressed = false;
-        if (kc >= 8 * ((n >> 1) + 1) && sc >= 4 * (uB - 1)) {
+        if (kc >= 8 * ((n >> 1) + 1) && sc >= 4 * n) {
           tc5::fence_after();
           const uint64_t db = d_k + (uint64_t)((n & 1) * (OP_BYTES >> 4) + hf * (8 * OP_SBO >> 4));  // token rows 64 hf ..
           if (el) {
@@ -701,15 +743,15 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
         }
         if (stalled(progressed, 51)) ok = false;
       }
-    } else if (warp == 14) {
+    } else if (warp == 18) {
       constexpr uint32_t ID_U3 = tc5::idesc_f16_f32(128, VROWS);
       const uint64_t d_v = tc5::smem_desc(smem_u32(vop), 128, V_SBO);
       int uC = 0;
       while (ok && uC < 2 * NT) {
-        const int hf = uC & 1;
-        const int pc = smem_load_acquire(&sh->pcnt), vc = smem_load_acquire(&sh->vcnt);
+        const int hf = uC & 1, n = uC >> 1;
+        const int pc = smem_load_acquire(&sh->pcnt[hf]), vc = smem_load_acquire(&sh->vcnt[hf]);
         bool progressed = false;
-        if (pc >= 4 * (uC + 1) && vc >= 8 * ((uC >> 1) + 1)) {
+        if (pc >= 4 * (n + 1) && vc >= 4 * (n + 1)) {
           tc5::fence_after();
           if (el) {
 #pragma unroll
@@ -729,7 +771,7 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
   // ---- epilogue: every role ends here; the tensor memory goes back before the CTA leaves ----
   tc5::fence_before();
   __syncthreads();
-  if (warp == 12) {
+  if (warp == 16) {
     tc5::fence_after();
     tc5::dealloc(tmem, TM_COLS);
   }
