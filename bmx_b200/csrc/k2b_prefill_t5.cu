@@ -16,8 +16,8 @@
 //   U2  S[128 rows x 64 tok]     = Q (smem) x K^T over 144 channels, fp32, once per half of the tile: the two halves
 //                                  have their own score and weight columns, so U2 of one half runs while the other
 //                                  half is in the softmax
-//   softmax warps (4; thread = row): one pass per half with the running maximum (base 2); only when a score exceeds it
-//                                  by more than 8 is the accumulator rescaled and the half redone;
+//   softmax warps (2 x 4; thread = row, one set per half): running maximum (base 2) by turns; only when a score exceeds it
+//                                  by more than 8 does it move and the accumulator get rescaled;
 //                                  weights -> tensor memory as fp16 (A operand of U3)
 //   value warps (8; thread = channel, warp = 64 tokens): 2-bit codes -> the four fp16 levels of the value table
 //                                  -> shared memory as the B operand of U3.  Rows 128 / 129 of that operand hold
@@ -385,9 +385,9 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
   } else if (warp < 16) {
     // ===================== softmax warps: thread = attention row = TMEM lane =====================
     // Two sets of four warps, one per half of the tiles, so that the exponentials of one half overlap the tensor-memory round trips
-    // of the other.  They share one accumulator and hence one running maximum per row: a warp computes its weights with the
-    // maximum it knows, waits for its turn (the other warp of its 32 rows has settled the half before), starts over in the rare
-    // case that the maximum has moved since, raises it if it has to, and settles its own half.
+    // of the other.  They share one accumulator and hence one running maximum per row: a warp takes its half's scores to
+    // registers, finds their maximum, waits for its turn (the other warp of its 32 rows has settled the half before), raises the running
+    // maximum if it has to, passes the turn on and only then computes the weights.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P5_REG_SOFTMAX));
     const int wq = warp & 3, row = 32 * wq + lane, hf = (warp - 8) >> 2;
     const uint32_t tl_ = tmem + ((uint32_t)(32 * wq) << 16);
@@ -447,28 +447,13 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       }
       tc5::wait_st();
     };
-    // 32 scores (token columns col0 .. of the half tile) -> weights with the running maximum -> 16 columns of fp16
-    // pairs; returns the maximum of the visible scores together with `acc`
-    auto weights32 = [&](const uint32_t (&r)[32], uint32_t tp, int col0, bool masked, int jl, float negm, float acc) {
+    // 32 scores -> weights with the running maximum -> 16 columns of fp16 pairs
+    auto weights32 = [&](const uint32_t (&r)[32], uint32_t tp, float negm) {
       uint32_t pk[16];
-      if (masked) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const bool v0 = col0 + 2 * i < jl, v1 = col0 + 2 * i + 1 < jl;
-          const float s0 = __uint_as_float(r[2 * i]), s1 = __uint_as_float(r[2 * i + 1]);
-          acc = fmaxf(acc, fmaxf(v0 ? s0 : -INFINITY, v1 ? s1 : -INFINITY));
-          pk[i] = pack_h2(v0 ? ex2_approx(fmaf(s0, p.scale_log2, negm)) : 0.f, v1 ? ex2_approx(fmaf(s1, p.scale_log2, negm)) : 0.f);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float s0 = __uint_as_float(r[2 * i]), s1 = __uint_as_float(r[2 * i + 1]);
-          acc = fmaxf(acc, fmaxf(s0, s1));
-          pk[i] = pack_h2(ex2_approx(fmaf(s0, p.scale_log2, negm)), ex2_approx(fmaf(s1, p.scale_log2, negm)));
-        }
-      }
-      tc5::st16(tp + (col0 >> 1), pk);
-      return acc;
+      for (int i = 0; i < 16; ++i)
+        pk[i] = pack_h2(ex2_approx(fmaf(__uint_as_float(r[2 * i]), p.scale_log2, negm)), ex2_approx(fmaf(__uint_as_float(r[2 * i + 1]), p.scale_log2, negm)));
+      tc5::st16(tp, pk);
     };
 
     auto turn_is = [&](int u, int where) {  // half tiles 0 .. u-1 are settled; bounded
@@ -506,45 +491,40 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       PROF_ADD(0)
       if (!warp_wait(&sh->sdone[hf][e], (uint32_t)(n >> 1) & 1u, p.status, 47)) { alive = false; break; }
       PROF_ADD(1)
-      // the weight columns of this half still feed U3 of the previous tile's same half
-      if (n >= 1 && !warp_wait(&sh->odone[hf], (uint32_t)(n - 1) & 1u, p.status, 48)) { alive = false; break; }
       tc5::fence_after();
+      // the scores go to registers at once: U2 of the next tile's same half may overwrite them while they are worked on
+      uint32_t ra[32], rb[32];
+      tc5::ld32(tS, ra);
+      tc5::ld32(tS + 32, rb);
+      tc5::wait_ld();
+      tc5::fence_before();
+      __syncwarp();
+      if (lane == 0) smem_add_release(&sh->scnt[hf], 1);
       PROF_ADD(2)
-      bool settled_before = smem_load_acquire(&sh->turn[wq]) >= u;  // not needed yet, but if it is so the maximum is final
-      settled_before = __all_sync(0xffffffffu, settled_before);
-      if (settled_before && u > 0) m = sh->m[row];
-      for (;;) {
-        uint32_t ra[32], rb[32];
-        const float negm = -m;
-        tc5::ld32(tS, ra);
-        tc5::ld32(tS + 32, rb);
-        tc5::wait_ld();
-        float tmax = weights32(ra, tP, 0, masked, jl, negm, -INFINITY);
-        tmax = weights32(rb, tP, 32, masked, jl, negm, tmax);
-        PROF_ADD(3)
-        if (!settled_before) {
-          settled_before = __all_sync(0xffffffffu, turn_is(u, 53));
-          if (!settled_before) { alive = false; break; }
-          const float mc = u > 0 ? sh->m[row] : m;
-          const bool moved = mc != m;
-          m = mc;
-          PROF_ADD(5)
-          if (__any_sync(0xffffffffu, moved)) continue;
+      if (masked) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          ra[i] = i < jl ? ra[i] : 0xFF800000u;  // -inf: weight 0
+          rb[i] = 32 + i < jl ? rb[i] : 0xFF800000u;
         }
-        // Lazy maximum: as long as no score exceeds the running maximum by more than 8 (weights below 2^8) the weights
-        // just written stand.  Otherwise the whole warp (TMEM access is warp-wide) rescales its rows of the accumulator
-        // once every earlier U3 has finished, and goes through the half again with the new maximum.
-        const float ts = tmax * p.scale_log2;
-        const bool need = ts > m + 8.f;
-        if (!__any_sync(0xffffffffu, need)) break;
+      }
+      float t4[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) t4[i] = fmaxf(__uint_as_float(ra[i]), __uint_as_float(rb[i]));
+#pragma unroll
+      for (int i = 4; i < 32; ++i) t4[i & 3] = fmaxf(fmaxf(t4[i & 3], __uint_as_float(ra[i])), __uint_as_float(rb[i]));
+      const float ts = fmaxf(fmaxf(t4[0], t4[1]), fmaxf(t4[2], t4[3])) * p.scale_log2;
+      if (!__all_sync(0xffffffffu, turn_is(u, 53))) { alive = false; break; }
+      if (u > 0) m = sh->m[row];
+      // Lazy maximum: it moves only when a score exceeds it by more than 8 (weights stay below 2^8).  Then the whole warp (TMEM
+      // access is warp-wide) rescales its rows of the accumulator once every earlier U3 has finished.
+      const bool need = ts > m + 8.f;
+      if (__any_sync(0xffffffffu, need)) {
         if (u > 0) {  // the U3 just before this half: the other half of this tile, or of the previous one
           const bool ok = hf ? warp_wait(&sh->odone[0], (uint32_t)n & 1u, p.status, 50) : warp_wait(&sh->odone[1], (uint32_t)(n - 1) & 1u, p.status, 50);
           if (!ok) { alive = false; break; }
           tc5::fence_after();
-        }
-        const float f = need ? ex2_approx(m - ts) : 1.f;
-        if (need) m = ts;
-        if (u > 0) {
+          const float f = need ? ex2_approx(m - ts) : 1.f;
           uint32_t r4[4];
           tc5::ld4(tl_ + TM_O + 128, r4);
           tc5::wait_ld();
@@ -552,25 +532,29 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
           for (int i = 0; i < 4; ++i) r4[i] = __float_as_uint(__uint_as_float(r4[i]) * f);
           tc5::st4(tl_ + TM_O + 128, r4);
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t r[32];
-            tc5::ld32(tl_ + TM_O + 32 * c, r);
+          for (int c = 0; c < 16; ++c) {
+            uint32_t r[8];
+            tc5::ld8(tl_ + TM_O + 8 * c, r);
             tc5::wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
-            tc5::st32(tl_ + TM_O + 32 * c, r);
+            for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * f);
+            tc5::st8(tl_ + TM_O + 8 * c, r);
           }
         }
+        if (need) m = ts;
       }
-      if (!alive) break;
       // this half's maximum is settled: the other set may settle the next one
       sh->m[row] = m;
       __syncwarp();
       if (lane == 0) smem_add_release(&sh->turn[wq], 1);
-      // every score of the half has been read: U2 of the next tile's same half may overwrite them
-      tc5::fence_before();
-      __syncwarp();
-      if (lane == 0) smem_add_release(&sh->scnt[hf], 1);
+      PROF_ADD(5)
+      // the weight columns of this half still feed U3 of the previous tile's same half
+      if (n >= 1 && !warp_wait(&sh->odone[hf], (uint32_t)(n - 1) & 1u, p.status, 48)) { alive = false; break; }
+      tc5::fence_after();
+      PROF_ADD(6)
+      weights32(ra, tP, -m);
+      weights32(rb, tP + 16, -m);
+      PROF_ADD(3)
       tc5::wait_st();
       tc5::fence_before();
       __syncwarp();
