@@ -567,6 +567,19 @@ constexpr int RTN_MAX_STAGES = 6;
 constexpr int RTN_Q_STRIDE = 20;     // words of a lane's query fragments in shared memory (16, padded: 128-bit reads free of conflicts)
 constexpr int RTN_FIXED_SMEM = (8 * 8 * HEAD_DIM + 128 + 32 * RTN_Q_STRIDE) * 4 + 2 * RTN_MAX_STAGES * 8;  // range reduction, queries, barriers
 
+// Bounded wait that reports where it ran out.  It does not look at the status word first: this entry point never asked for a
+// cleared workspace, so what the word holds before the call means nothing.
+__device__ __forceinline__ bool rtn_wait(uint64_t* bar, uint32_t parity, int32_t* status, int where) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  for (uint32_t spin = 1;; ++spin) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((spin & 255u) == 0u && clock64() - t0 > WAIT_LIMIT_CYCLES) {
+      status[0] = 1, status[1] = blockIdx.x, status[2] = where;
+      return false;
+    }
+  }
+}
 __device__ __forceinline__ void rtn_consumers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // What bounds it: instruction issue and latency, not bytes (112 per token and head with groups of 32).  One warp issues the copies of
@@ -619,7 +632,7 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
       int st = 0, issued = 0;
       uint32_t ph = 1;  // parity to wait for on `empty`: the first pass over the ring finds every stage free
       for (int f = f_begin; f < f_end; ++f) {
-        if (!wait_or_flag(empty + st, ph, p.status, 60)) break;
+        if (!rtn_wait(empty + st, ph, p.status, 60)) break;
         const int pages_here = min(PAGES_PER_TILE, npg_sm[cur.b] - cur.j * PAGES_PER_TILE);
         mbar_arrive_expect_tx(full + st, (uint32_t)(pages_here * PB));
         for (int i = 0; i < pages_here; ++i) {
@@ -719,7 +732,7 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
       rtn_consumers_sync();
       s_scale = p.scale_log2 * exp2f((float)(e + 24));  // the codes enter as multiples of 2^-24
     }
-    if (alive) alive = __all_sync(0xffffffffu, wait_or_flag(full + st, ph, p.status, 61));
+    if (alive) alive = __all_sync(0xffffffffu, rtn_wait(full + st, ph, p.status, 61));
     if (alive && valid) {
       const uint8_t* tile = ring + st * stage_bytes;
       // ---- keys ----
