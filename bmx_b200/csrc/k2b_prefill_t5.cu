@@ -223,15 +223,15 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
     for (int n = 0; n < NT; ++n) {
       const int e = n & 1;
       uint8_t* krow = kop0 + (size_t)e * OP_BYTES + (row >> 3) * OP_SBO + (row & 7) * 16;
-      // the buffer still feeds U2 of tile n-2
-      if (n >= 2 && !(warp_wait(&sh->sdone[0][e], (uint32_t)((n - 2) >> 1) & 1u, p.status, 41) &&
-                      warp_wait(&sh->sdone[1][e], (uint32_t)((n - 2) >> 1) & 1u, p.status, 41))) break;
+      // the buffer still feeds U2 of tile n-2 (one thread issues both halves: the second one's completion covers the first's)
+      if (n >= 2 && !warp_wait(&sh->sdone[1][e], (uint32_t)((n - 2) >> 1) & 1u, p.status, 41)) break;
       PROF_ADD(0)
       if (n < NP) {
         const uint8_t* blk = stage0 + (size_t)s * STAGE_BYTES + COEF_BYTES;
-        if (!warp_wait(&sh->full[s], fp, p.status, 42)) break;
-        PROF_ADD(1)
+        // U1 comes after the copy: waiting for it first leaves one wait that never blocks
         if (!warp_wait(&sh->low, (uint32_t)n & 1u, p.status, 43)) break;
+        PROF_ADD(1)
+        if (!warp_wait(&sh->full[s], fp, p.status, 42)) break;
         PROF_ADD(2)
         tc5::fence_after();
         uint32_t dl[2][8], dh[2][8];
