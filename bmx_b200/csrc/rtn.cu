@@ -591,6 +591,8 @@ __device__ __forceinline__ void rtn_consumers_sync() { asm volatile("bar.sync 1,
 //           second product with constant rows (tensor pipe, idle otherwise) and the same queries, so it cancels exactly up to the
 //           fp32 accumulation.  rtn_channel: the scales of the warp's token group multiply the queries (16 products instead of
 //           32).  The queries are scaled by a power of two so that max |q| < 1: the product with any fp16 scale stays finite.
+//           A scaled query is carried as an fp16 pair, rounded product and remainder: a scale is shared by the whole group, so the
+//           rounding alone would shift all of the group's scores together (it tripled the error of 2-bit keys).
 //           rtn_token: one accumulator pair per channel group, scaled in float32.
 //   values  codes 0, 1, -2, -1 as fp16 have zero low bytes: one byte-permute lookup yields the high bytes of four codes.
 // The weights' running maximum moves only when a score passes it by more than 8 (log2): that test needs no cross-lane reduction.
@@ -752,20 +754,32 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
 #pragma unroll
         for (int qd = gi * QD_PER; qd < (gi + 1) * QD_PER; ++qd) {
           const uint4 q4 = *reinterpret_cast<const uint4*>(q_sm + lane * RTN_Q_STRIDE + 4 * qd);
-          uint32_t b[4] = {q4.x, q4.y, q4.z, q4.w};  // channel octets 4qd .. 4qd+3
+          uint32_t b[4] = {q4.x, q4.y, q4.z, q4.w}, lo[4];  // channel octets 4qd .. 4qd+3
           if (ARM == RTN_CHANNEL) {
             const uint4 s4 = *reinterpret_cast<const uint4*>(tile + off_ks + 64 * qd);
             const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) b[i] = h2_as_u32(__hmul2(u32_as_h2(b[i]), u32_as_h2(sw[i])));
+            for (int i = 0; i < 4; ++i) {
+              const __half2 prod = __hmul2(u32_as_h2(b[i]), u32_as_h2(sw[i]));
+              lo[i] = h2_as_u32(__hfma2(u32_as_h2(b[i]), u32_as_h2(sw[i]), __hneg2(prod)));  // what the rounding left
+              b[i] = h2_as_u32(prod);
+            }
           }
           const uint32_t w0 = ww[0][qd], w1 = ww[1][qd], x0 = w0 >> 8, x1 = w1 >> 8;
-          mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], lop3<0x6A>(w0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(w1, 0x000F000Fu, 0x00080008u),
-                     lop3<0x6A>(x0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(x1, 0x000F000Fu, 0x00080008u), b[0], b[2]);
-          mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], lop3<0x6A>(w0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(w1, 0x00F000F0u, 0x00800080u),
-                     lop3<0x6A>(x0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(x1, 0x00F000F0u, 0x00800080u), b[1], b[3]);
+          const uint32_t ka[4] = {lop3<0x6A>(w0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(w1, 0x000F000Fu, 0x00080008u),
+                                  lop3<0x6A>(x0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(x1, 0x000F000Fu, 0x00080008u)};
+          const uint32_t kb[4] = {lop3<0x6A>(w0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(w1, 0x00F000F0u, 0x00800080u),
+                                  lop3<0x6A>(x0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(x1, 0x00F000F0u, 0x00800080u)};
+          mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], ka[0], ka[1], ka[2], ka[3], b[0], b[2]);
+          mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], kb[0], kb[1], kb[2], kb[3], b[1], b[3]);
           mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], M8A, M8A, M8A, M8A, b[0], b[2]);
           mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], M8B, M8B, M8B, M8B, b[1], b[3]);
+          if (ARM == RTN_CHANNEL) {
+            mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], ka[0], ka[1], ka[2], ka[3], lo[0], lo[2]);
+            mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], kb[0], kb[1], kb[2], kb[3], lo[1], lo[3]);
+            mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], M8A, M8A, M8A, M8A, lo[0], lo[2]);
+            mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], M8B, M8B, M8B, M8B, lo[1], lo[3]);
+          }
         }
         if (ARM == RTN_CHANNEL) {
 #pragma unroll
