@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(RTND_THREADS) rtn_dequant_dense_kernel(RtnGeom
 }
 
 // ---------------------------------------------------------------------------------------------
-// Split-KV decode.  Persistent grid, 8 warps per CTA, warp w owns token rows 16w..16w+15 of every
-// 128-token tile of its CTA's range; same flat decomposition, partial record and merge kernel as k2b.
+// Split-KV decode.  Persistent grid, one CTA per SM; score warp w and value warp w own token rows 16w..16w+15 of every
+// 128-token tile of their CTA's range; same flat decomposition, partial record and merge kernel as k2b.
 // ---------------------------------------------------------------------------------------------
 struct RtnDecodeParams {
   RtnGeom g;
@@ -561,11 +561,12 @@ struct RtnDecodeParams {
   int n_stages;
 };
 
-constexpr int RTN_CTAS_PER_SM = 2;   // resident decode CTAs
-constexpr int RTN_THREADS = 288;     // eight computing warps and one that issues the copies
-constexpr int RTN_MAX_STAGES = 6;
-constexpr int RTN_Q_STRIDE = 20;     // words of a lane's query fragments in shared memory (16, padded: 128-bit reads free of conflicts)
-constexpr int RTN_FIXED_SMEM = (8 * 8 * HEAD_DIM + 128 + 32 * RTN_Q_STRIDE) * 4 + 2 * RTN_MAX_STAGES * 8;  // range reduction, queries, barriers
+constexpr int RTN_WARPS = 8;                             // score warps, and as many value warps
+constexpr int RTN_THREADS = (2 * RTN_WARPS + 1) * 32;    // and one warp that issues the copies
+constexpr int RTN_MAX_STAGES = 8;
+constexpr int RTN_S_BYTES = RTN_WARPS * 32 * 16;         // scores of a tile, beside its stage of the ring
+constexpr int RTN_FIXED_SMEM = (8 * 8 * HEAD_DIM + 128) * 4 + (2 + RTN_WARPS) * RTN_MAX_STAGES * 8;  // range reduction, barriers
+constexpr int RTN_SMEM = 200 * 1024;                     // most that the ring may grow to
 
 // Bounded wait that reports where it ran out.  It does not look at the status word first: this entry point never asked for a
 // cleared workspace, so what the word holds before the call means nothing.
@@ -580,26 +581,31 @@ __device__ __forceinline__ bool rtn_wait(uint64_t* bar, uint32_t parity, int32_t
     }
   }
 }
-__device__ __forceinline__ void rtn_consumers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ bool rtn_warp_wait(uint64_t* bar, uint32_t parity, int32_t* status, int where) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;  // the usual case, without divergence
+  return __all_sync(0xffffffffu, rtn_wait(bar, parity, status, where));
+}
+__device__ __forceinline__ void rtn_value_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// What bounds it: instruction issue and latency, not bytes (112 per token and head with groups of 32).  One warp issues the copies of
+// A score maximum as the running maximum takes it: rounded to fp16, and from 8192 on as it is (there the rounding would be off by
+// more than 2, and a weight of 2^(8 + error) times a value scale leaves the range of fp16).
+__device__ __forceinline__ float rtn_coarse(float x) { return fabsf(x) <= 8192.f ? __half2float(__float2half_rn(x)) : x; }
+
+// What bounds it: latency and instruction issue, not bytes (112 per token and head with groups of 32).  One warp issues the copies of
 // whole page blocks, up to n_stages tiles ahead (a register prefetch of one tile left the page-table lookup and the DRAM latency on the
-// path of every tile); eight warps own 16 token rows each.  The arm and the groups are template parameters, so that every operand index
-// is a constant, and two CTAs share an SM.  Integer operands stay integers until the product:
-//   keys    a nibble becomes the fp16 SUBNORMAL (code + 8) * 2^-24 (low nibbles) or * 2^-20 (high nibbles) with one LOP3; low and
-//           high nibbles go to separate products, whose accumulators differ by an exact factor 16; the offset 8 is taken out by a
-//           second product with constant rows (tensor pipe, idle otherwise) and the same queries, so it cancels exactly up to the
-//           fp32 accumulation.  rtn_channel: the scales of the warp's token group multiply the queries (16 products instead of
-//           32).  The queries are scaled by a power of two so that max |q| < 1: the product with any fp16 scale stays finite.
-//           A scaled query is carried as an fp16 pair, rounded product and remainder: a scale is shared by the whole group, so the
-//           rounding alone would shift all of the group's scores together (it tripled the error of 2-bit keys).
-//           rtn_token: one accumulator pair per channel group, scaled in float32.
+// path of every tile).  The work on 16 token rows is split over two warps, so that the dependent products of one tile's scores run
+// beside the value lookups of the tile before: a score warp hands its four scores per lane on through shared memory.  One CTA per SM:
+// a range is walked in one piece, so the running maximum and the sums see the tiles in one order whatever the overlap.  The arm and
+// the groups are template parameters, so that every operand index is a constant.
+//   keys    code * scale rounded once to fp16 (the stored scale is fp16: subnormal scales lose nothing), against the queries as they
+//           come: the scores do not depend on how the other heads of the group are scaled.
 //   values  codes 0, 1, -2, -1 as fp16 have zero low bytes: one byte-permute lookup yields the high bytes of four codes.
-// The weights' running maximum moves only when a score passes it by more than 8 (log2): that test needs no cross-lane reduction.
-// Measured, 16 sequences x 8192 tokens x 8 heads, 4-bit keys, groups of 32: step (with merge) 123 -> 59 us, kernel 115 -> 50 us = 2.4 TB/s;
-// 43 -> 26 million warp instructions, 650 -> 400 per 16 token rows; the byte permutes and LOP3s (half-rate pipe, 49 % busy) lead.
+// The running maximum moves only when a score passes it by more than 8 (log2): that test needs no cross-lane reduction.
+// Measured, 8 heads, 4-bit keys per channel, groups of 32, step with merge, passes back to back: 16 sequences x 8192 tokens 122.0 ->
+// 60.8 us, one sequence of 4096 tokens 12.4 -> 10.4, one of 12000 20.6 -> 17.4 (both warps' work in one warp, two CTAs per SM, nibbles
+// as integers against queries that carry the scales: 82.9, 16.7, 22.6 us, and scores that depend on the other heads' magnitudes).
 template <int PAGE, int ARM, int KG, int VG>
-__global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kernel(const RtnDecodeParams p) {
+__global__ void __launch_bounds__(RTN_THREADS, 1) rtn_decode_kernel(const RtnDecodeParams p) {
   constexpr int PAGES_PER_TILE = TILE_TOKENS / PAGE, WR_PER_PAGE = PAGE / 16;
   extern __shared__ __align__(16) uint8_t smem[];
   const RtnGeom g = p.g;
@@ -608,16 +614,18 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
   float* red = reinterpret_cast<float*>(smem + p.n_stages * stage_bytes);  // [8 warps][8 q][128]
   float* red_m = red + 8 * 8 * HEAD_DIM;                                    // [8][8]
   float* red_l = red_m + 64;
-  uint32_t* q_sm = reinterpret_cast<uint32_t*>(red_l + 64);                 // [32 lanes][RTN_Q_STRIDE] query fragments, the same for all warps
-  uint64_t* full = reinterpret_cast<uint64_t*>(q_sm + 32 * RTN_Q_STRIDE);   // [RTN_MAX_STAGES] a tile's blocks have landed
-  uint64_t* empty = full + RTN_MAX_STAGES;                                  // [RTN_MAX_STAGES] all eight warps are done with it
-  int* cum = reinterpret_cast<int*>(empty + RTN_MAX_STAGES);                // [batch + 1]
+  float4* s_sm = reinterpret_cast<float4*>(red_l + 64);                     // [n_stages][8 warps][32 lanes] scores, log2 units
+  uint64_t* full = reinterpret_cast<uint64_t*>(s_sm + p.n_stages * RTN_WARPS * 32);  // [RTN_MAX_STAGES] a tile's blocks have landed
+  uint64_t* empty = full + RTN_MAX_STAGES;                                  // [RTN_MAX_STAGES] all value warps (and so all score warps) are done with it
+  uint64_t* scored = empty + RTN_MAX_STAGES;                                // [RTN_MAX_STAGES][8] a score warp is done with its rows
+  int* cum = reinterpret_cast<int*>(scored + RTN_MAX_STAGES * RTN_WARPS);   // [batch + 1]
   int* npg_sm = cum + p.batch + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t4 = lane & 3;
   asm volatile("griddepcontrol.launch_dependents;");  // the merge kernel is this kernel's programmatic dependent (see launch_merge)
   if (warp == 0) fill_cum(cum, p.n_pages, p.batch, g.h_kv, PAGE, lane);
   if (tid == 32) {
-    for (int i = 0; i < p.n_stages; ++i) mbar_init(full + i, 1), mbar_init(empty + i, 8);
+    for (int i = 0; i < p.n_stages; ++i) mbar_init(full + i, 1), mbar_init(empty + i, RTN_WARPS);
+    for (int i = 0; i < p.n_stages * RTN_WARPS; ++i) mbar_init(scored + i, 1);
     fence_barrier_init();
   }
   for (int i = tid; i < p.batch; i += RTN_THREADS) npg_sm[i] = p.n_pages[i];
@@ -629,36 +637,102 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
   TileCursor cur;
   cur.init(cum, npg_sm, f_begin, PAGE);
 
-  if (warp == 8) {  // copies
-    if (lane == 0) {
-      int st = 0, issued = 0;
-      uint32_t ph = 1;  // parity to wait for on `empty`: the first pass over the ring finds every stage free
-      for (int f = f_begin; f < f_end; ++f) {
-        if (!rtn_wait(empty + st, ph, p.status, 60)) break;
-        const int pages_here = min(PAGES_PER_TILE, npg_sm[cur.b] - cur.j * PAGES_PER_TILE);
-        mbar_arrive_expect_tx(full + st, (uint32_t)(pages_here * PB));
-        for (int i = 0; i < pages_here; ++i) {
-          const int slot = p.page_table[(int64_t)cur.b * p.table_stride + cur.j * PAGES_PER_TILE + i];
-          bulk_g2s(ring + st * stage_bytes + i * PB, p.pages + ((int64_t)slot * g.h_kv + cur.h) * PB, (uint32_t)PB, full + st);
-        }
-        ++issued;
-        cur.next(npg_sm, g.h_kv, PAGE, p.batch);
-        if (++st == p.n_stages) st = 0, ph ^= 1;
+  if (warp == 2 * RTN_WARPS) {
+    // ===================== copies: the lanes hold the slots of the next 32 pages of the sequence =====================
+    int st = 0, issued = 0, slots = 0, slots_b = -1, slots_j = 0;
+    uint32_t ph = 1;  // parity to wait for on `empty`: the first pass over the ring finds every stage free
+    for (int f = f_begin; f < f_end; ++f) {
+      const int page0 = cur.j * PAGES_PER_TILE, pages_here = min(PAGES_PER_TILE, npg_sm[cur.b] - page0);
+      if (cur.b != slots_b || page0 < slots_j || page0 + PAGES_PER_TILE > slots_j + 32) {
+        slots_b = cur.b, slots_j = page0;
+        slots = page0 + lane < npg_sm[cur.b] ? p.page_table[(int64_t)cur.b * p.table_stride + page0 + lane] : 0;
       }
-      if (issued < f_end - f_begin)  // a wait ran out: no copy may be in flight when this CTA ends
-        for (int i = max(0, issued - p.n_stages); i < issued; ++i) mbar_wait_bounded(full + i % p.n_stages, (i / p.n_stages) & 1);
+      if (!rtn_warp_wait(empty + st, ph, p.status, 60)) break;
+      if (lane == 0) mbar_arrive_expect_tx(full + st, (uint32_t)(pages_here * PB));
+#pragma unroll
+      for (int i = 0; i < PAGES_PER_TILE; ++i) {
+        const int slot = __shfl_sync(0xffffffffu, slots, page0 - slots_j + i);
+        if (lane == 0 && i < pages_here)
+          bulk_g2s(ring + st * stage_bytes + i * PB, p.pages + ((int64_t)slot * g.h_kv + cur.h) * PB, (uint32_t)PB, full + st);
+      }
+      ++issued;
+      cur.next(npg_sm, g.h_kv, PAGE, p.batch);
+      if (++st == p.n_stages) st = 0, ph ^= 1;
+    }
+    for (int i = max(0, issued - p.n_stages); i < issued; ++i)  // no copy is in flight when this CTA ends, whatever became of its readers
+      rtn_warp_wait(full + i % p.n_stages, (uint32_t)(i / p.n_stages) & 1u, p.status, 62);
+    return;
+  }
+
+  const int w8 = warp & (RTN_WARPS - 1);  // 16 rows of the tile
+  const int sub_page = w8 / WR_PER_PAGE, wr = w8 % WR_PER_PAGE;
+  int st = 0;
+  uint32_t ph = 0;
+
+  if (warp < RTN_WARPS) {
+    // ===================== scores =====================
+    // byte offsets of this lane's pieces inside a tile's stage
+    const int off_k = sub_page * PB + (wr * 64 + lane) * 16;
+    const int off_ks = sub_page * PB + rtn_off_kscale(g) + (ARM == RTN_CHANNEL ? (((16 * wr) / KG) * 128 + t4 * 8) * 2 : (16 * wr + gq) * 8);
+    const __half2 c1032 = __floats2half2_rn(1032.f, 1032.f), c16th = __floats2half2_rn(0.0625f, 0.0625f), cm72 = __floats2half2_rn(-72.f, -72.f);
+    uint32_t qb[16];  // B operands: channel pairs (8n + 2t, + 1) of query g
+    int cur_bh = -1;
+    for (int f = f_begin; f < f_end; ++f) {
+      const int bh = cur.b * g.h_kv + cur.h;
+      const bool valid = PAGES_PER_TILE == 1 || cur.j * PAGES_PER_TILE + sub_page < npg_sm[cur.b];
+      if (bh != cur_bh) {
+        cur_bh = bh;
+        const __half* qp = p.q + ((int64_t)bh * G + gq) * HEAD_DIM + 2 * t4;
+#pragma unroll
+        for (int n = 0; n < 16; ++n) qb[n] = (gq < G) ? *reinterpret_cast<const uint32_t*>(qp + 8 * n) : 0u;
+      }
+      if (!rtn_warp_wait(full + st, ph, p.status, 61)) break;
+      if (valid) {
+        const uint8_t* tile = ring + st * stage_bytes;
+        const uint4 k0 = *reinterpret_cast<const uint4*>(tile + off_k), k1 = *reinterpret_cast<const uint4*>(tile + off_k + 512);
+        const uint32_t ww[2][4] = {{k0.x, k0.y, k0.z, k0.w}, {k1.x, k1.y, k1.z, k1.w}};
+        uint32_t tsc[4];  // rtn_token: the four scales of row g, then those of row g + 8
+        if (ARM == RTN_TOKEN) {
+          const uint2 x = *reinterpret_cast<const uint2*>(tile + off_ks), y = *reinterpret_cast<const uint2*>(tile + off_ks + 64);
+          tsc[0] = x.x, tsc[1] = x.y, tsc[2] = y.x, tsc[3] = y.y;
+        }
+        float S[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int qd = 0; qd < 4; ++qd) {  // channels 32 qd .. 32 qd + 31
+          uint32_t a[4][2];
+          uint4 s4 = make_uint4(0u, 0u, 0u, 0u);
+          if (ARM == RTN_CHANNEL) s4 = *reinterpret_cast<const uint4*>(tile + off_ks + 64 * qd);
+          const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {  // rows g, g + 8
+            const uint32_t lo = ww[c][qd], hi = ww[c][qd] >> 8;
+            const __half2 code[4] = {__hsub2(u32_as_h2(lop3<0x6A>(lo, 0x000F000Fu, 0x64086408u)), c1032),
+                                     __hfma2(u32_as_h2(lop3<0x6A>(lo, 0x00F000F0u, 0x64806480u)), c16th, cm72),
+                                     __hsub2(u32_as_h2(lop3<0x6A>(hi, 0x000F000Fu, 0x64086408u)), c1032),
+                                     __hfma2(u32_as_h2(lop3<0x6A>(hi, 0x00F000F0u, 0x64806480u)), c16th, cm72)};
+            const int gi = (32 * qd) / KG;
+            const uint32_t tok = ARM == RTN_TOKEN ? prmt(tsc[2 * c + (gi >> 1)], 0u, (gi & 1) ? 0x3232u : 0x1010u) : 0u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i][c] = h2_as_u32(__hmul2(code[i], u32_as_h2(ARM == RTN_CHANNEL ? sw[i] : tok)));
+          }
+          mma_f32acc(S[0], S[1], S[2], S[3], a[0][0], a[0][1], a[1][0], a[1][1], qb[4 * qd], qb[4 * qd + 1]);
+          mma_f32acc(S[0], S[1], S[2], S[3], a[2][0], a[2][1], a[3][0], a[3][1], qb[4 * qd + 2], qb[4 * qd + 3]);
+        }
+        // the place's last scores were read before this stage was filled again
+        s_sm[(st * RTN_WARPS + w8) * 32 + lane] = make_float4(S[0] * p.scale_log2, S[1] * p.scale_log2, S[2] * p.scale_log2, S[3] * p.scale_log2);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(scored + st * RTN_WARPS + w8);
+      cur.next(npg_sm, g.h_kv, PAGE, p.batch);
+      if (++st == p.n_stages) st = 0, ph ^= 1;
     }
     return;
   }
 
-  const int sub_page = warp / WR_PER_PAGE, wr = warp % WR_PER_PAGE;
-  // byte offsets of this lane's pieces inside a tile's stage
-  const int off_k = sub_page * PB + (wr * 64 + lane) * 16, off_v = sub_page * PB + rtn_off_vcode(g) + (wr * 32 + lane) * 16;
-  const int off_ks = sub_page * PB + rtn_off_kscale(g) + (ARM == RTN_CHANNEL ? (((16 * wr) / KG) * 128 + t4 * 8) * 2 : (16 * wr + gq) * 8);
-  const int off_vs = sub_page * PB + rtn_off_vscale(g) + (16 * wr + gq) * 8;
-
+  // ===================== weights and values =====================
+  const int off_v = sub_page * PB + rtn_off_vcode(g) + (wr * 32 + lane) * 16, off_vs = sub_page * PB + rtn_off_vscale(g) + (16 * wr + gq) * 8;
   float O[8][4];
-  float m0 = 0.f, m1 = 0.f, l0 = 0.f, l1 = 0.f, s_scale = 0.f;  // s_scale: scores in log2 units per accumulated unit
+  float m0 = 0.f, m1 = 0.f, l0 = 0.f, l1 = 0.f;
   int cur_bh = -1, cur_b = 0, cur_h = 0;
   // two's-complement 2-bit value codes as fp16: 0, 1, -2, -1 (high bytes; the low bytes are zero)
   const uint32_t lut_hi = 0xBCC03C00u;
@@ -667,20 +741,20 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
 #pragma unroll
     for (int m = 4; m <= 16; m <<= 1) l0 += __shfl_xor_sync(0xffffffffu, l0, m), l1 += __shfl_xor_sync(0xffffffffu, l1, m);
     if (gq == 0) {
-      red_m[warp * 8 + 2 * t4] = m0, red_m[warp * 8 + 2 * t4 + 1] = m1;
-      red_l[warp * 8 + 2 * t4] = l0, red_l[warp * 8 + 2 * t4 + 1] = l1;
+      red_m[w8 * 8 + 2 * t4] = m0, red_m[w8 * 8 + 2 * t4 + 1] = m1;
+      red_l[w8 * 8 + 2 * t4] = l0, red_l[w8 * 8 + 2 * t4 + 1] = l1;
     }
 #pragma unroll
     for (int mt = 0; mt < 8; ++mt) {
-      float* o = red + (warp * 8) * HEAD_DIM;
+      float* o = red + (w8 * 8) * HEAD_DIM;
       o[(2 * t4) * HEAD_DIM + 16 * mt + gq] = O[mt][0];
       o[(2 * t4 + 1) * HEAD_DIM + 16 * mt + gq] = O[mt][1];
       o[(2 * t4) * HEAD_DIM + 16 * mt + gq + 8] = O[mt][2];
       o[(2 * t4 + 1) * HEAD_DIM + 16 * mt + gq + 8] = O[mt][3];
     }
-    rtn_consumers_sync();
+    rtn_value_warps_sync();
     float* dst = p.part + ((int64_t)(blockIdx.x + b_ * g.h_kv + h_) * G) * PART_STRIDE;
-    for (int o = tid; o < G * HEAD_DIM; o += 256) {
+    for (int o = tid - 32 * RTN_WARPS; o < G * HEAD_DIM; o += 256) {
       const int qi = o / HEAD_DIM, ch = o % HEAD_DIM;
       float M = -INFINITY;
 #pragma unroll
@@ -696,109 +770,40 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
       dst[qi * PART_STRIDE + 2 + ch] = acc;
       if (ch == 0) dst[qi * PART_STRIDE] = M, dst[qi * PART_STRIDE + 1] = l;
     }
-    rtn_consumers_sync();
+    rtn_value_warps_sync();
   };
 
-  int st = 0;
-  uint32_t ph = 0;
-  bool alive = true;  // false once a wait ran out: nothing is computed any more, barriers are still met
-  for (int f = f_begin; f < f_end; ++f) {
-    const int b = cur.b, h = cur.h, bh = cur.b * g.h_kv + cur.h;
-    const bool valid = cur.j * PAGES_PER_TILE + sub_page < npg_sm[b];
+  bool alive = true;  // false once a wait ran out: nothing is read or handed back any more, the barriers of flush() are still met
+  for (int f = f_begin;; ++f) {
+    const int b = cur.b, h = cur.h, bh = f < f_end ? cur.b * g.h_kv + cur.h : -1;
     if (bh != cur_bh) {
       if (cur_bh >= 0) flush(cur_b, cur_h);
+      if (f == f_end) break;
       cur_bh = bh, cur_b = b, cur_h = h;
       m0 = (2 * t4 < G) ? -INFINITY : 0.f, m1 = (2 * t4 + 1 < G) ? -INFINITY : 0.f, l0 = l1 = 0.f;
 #pragma unroll
       for (int mt = 0; mt < 8; ++mt) O[mt][0] = O[mt][1] = O[mt][2] = O[mt][3] = 0.f;
-      // B operands: channel pair (8n + 2t, + 1) of query g, n = 0..15, scaled by 2^-e; every warp computes them, warp 0 stores
-      // them (the barriers of flush() lie between the last use of the previous ones and this store)
-      const __half* qp = p.q + ((int64_t)bh * G + gq) * HEAD_DIM + 2 * t4;
-      uint32_t qb[16];
-      float qm = 0.f;
-#pragma unroll
-      for (int n = 0; n < 16; ++n) {
-        qb[n] = (gq < G) ? *reinterpret_cast<const uint32_t*>(qp + 8 * n) : 0u;
-        const float2 x = __half22float2(u32_as_h2(qb[n]));
-        qm = fmaxf(qm, fmaxf(fabsf(x.x), fabsf(x.y)));
-      }
-#pragma unroll
-      for (int m = 16; m >= 1; m >>= 1) qm = fmaxf(qm, __shfl_xor_sync(0xffffffffu, qm, m));
-      int e = 0;
-      if (qm > 0.f && qm <= 65504.f) e = max(-13, min(15, ilogbf(qm) + 1));  // |q| < 2^e (<= 2^15 * 2); 2^-e is an fp16 number
-      if (warp == 0) {
-        const __half2 dn = __float2half2_rn(exp2f((float)-e));
-#pragma unroll
-        for (int n = 0; n < 16; ++n) q_sm[lane * RTN_Q_STRIDE + n] = h2_as_u32(__hmul2(u32_as_h2(qb[n]), dn));
-      }
-      rtn_consumers_sync();
-      s_scale = p.scale_log2 * exp2f((float)(e + 24));  // the codes enter as multiples of 2^-24
     }
-    if (alive) alive = __all_sync(0xffffffffu, rtn_wait(full + st, ph, p.status, 61));
+    const bool valid = PAGES_PER_TILE == 1 || cur.j * PAGES_PER_TILE + sub_page < npg_sm[b];
+    if (alive) alive = rtn_warp_wait(full + st, ph, p.status, 64);
+    uint2 vs0 = make_uint2(0u, 0u), vs1 = vs0;
+    uint4 vc = make_uint4(0u, 0u, 0u, 0u);
     if (alive && valid) {
       const uint8_t* tile = ring + st * stage_bytes;
-      // ---- keys ----
-      const uint4 k0 = *reinterpret_cast<const uint4*>(tile + off_k), k1 = *reinterpret_cast<const uint4*>(tile + off_k + 512);
-      const uint32_t ww[2][4] = {{k0.x, k0.y, k0.z, k0.w}, {k1.x, k1.y, k1.z, k1.w}};
-      uint32_t tsc[4];  // rtn_token: the four scales of row g, then those of row g + 8
-      if (ARM == RTN_TOKEN) {
-        const uint2 x = *reinterpret_cast<const uint2*>(tile + off_ks), y = *reinterpret_cast<const uint2*>(tile + off_ks + 64);
-        tsc[0] = x.x, tsc[1] = x.y, tsc[2] = y.x, tsc[3] = y.y;
-      }
-      constexpr uint32_t M8A = 0x80088008u, M8B = 0x80808080u;  // -8 * 2^-24 and -8 * 2^-20, as fp16 pairs
-      float S[4] = {0.f, 0.f, 0.f, 0.f};
-      constexpr int NG = ARM == RTN_CHANNEL ? 1 : HEAD_DIM / KG, QD_PER = 4 / NG;  // channel groups with an accumulator of their own
-#pragma unroll
-      for (int gi = 0; gi < NG; ++gi) {
-        float Sa[4] = {0.f, 0.f, 0.f, 0.f}, Sb[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int qd = gi * QD_PER; qd < (gi + 1) * QD_PER; ++qd) {
-          const uint4 q4 = *reinterpret_cast<const uint4*>(q_sm + lane * RTN_Q_STRIDE + 4 * qd);
-          uint32_t b[4] = {q4.x, q4.y, q4.z, q4.w}, lo[4];  // channel octets 4qd .. 4qd+3
-          if (ARM == RTN_CHANNEL) {
-            const uint4 s4 = *reinterpret_cast<const uint4*>(tile + off_ks + 64 * qd);
-            const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const __half2 prod = __hmul2(u32_as_h2(b[i]), u32_as_h2(sw[i]));
-              lo[i] = h2_as_u32(__hfma2(u32_as_h2(b[i]), u32_as_h2(sw[i]), __hneg2(prod)));  // what the rounding left
-              b[i] = h2_as_u32(prod);
-            }
-          }
-          const uint32_t w0 = ww[0][qd], w1 = ww[1][qd], x0 = w0 >> 8, x1 = w1 >> 8;
-          const uint32_t ka[4] = {lop3<0x6A>(w0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(w1, 0x000F000Fu, 0x00080008u),
-                                  lop3<0x6A>(x0, 0x000F000Fu, 0x00080008u), lop3<0x6A>(x1, 0x000F000Fu, 0x00080008u)};
-          const uint32_t kb[4] = {lop3<0x6A>(w0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(w1, 0x00F000F0u, 0x00800080u),
-                                  lop3<0x6A>(x0, 0x00F000F0u, 0x00800080u), lop3<0x6A>(x1, 0x00F000F0u, 0x00800080u)};
-          mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], ka[0], ka[1], ka[2], ka[3], b[0], b[2]);
-          mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], kb[0], kb[1], kb[2], kb[3], b[1], b[3]);
-          mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], M8A, M8A, M8A, M8A, b[0], b[2]);
-          mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], M8B, M8B, M8B, M8B, b[1], b[3]);
-          if (ARM == RTN_CHANNEL) {
-            mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], ka[0], ka[1], ka[2], ka[3], lo[0], lo[2]);
-            mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], kb[0], kb[1], kb[2], kb[3], lo[1], lo[3]);
-            mma_f32acc(Sa[0], Sa[1], Sa[2], Sa[3], M8A, M8A, M8A, M8A, lo[0], lo[2]);
-            mma_f32acc(Sb[0], Sb[1], Sb[2], Sb[3], M8B, M8B, M8B, M8B, lo[1], lo[3]);
-          }
-        }
-        if (ARM == RTN_CHANNEL) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) S[i] = fmaf(Sb[i], 0.0625f, Sa[i]);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const uint32_t wsel = tsc[2 * c + (gi >> 1)];
-            const float sc = __half2float(__ushort_as_half((unsigned short)((gi & 1) ? (wsel >> 16) : (wsel & 0xFFFFu))));
-            S[2 * c] = fmaf(fmaf(Sb[2 * c], 0.0625f, Sa[2 * c]), sc, S[2 * c]);
-            S[2 * c + 1] = fmaf(fmaf(Sb[2 * c + 1], 0.0625f, Sa[2 * c + 1]), sc, S[2 * c + 1]);
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) S[i] *= s_scale;
+      vs0 = *reinterpret_cast<const uint2*>(tile + off_vs), vs1 = *reinterpret_cast<const uint2*>(tile + off_vs + 64);
+      vc = *reinterpret_cast<const uint4*>(tile + off_v);
+    }
+    if (alive) alive = rtn_warp_wait(scored + st * RTN_WARPS + w8, ph, p.status, 63);
+    float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (alive) {
+      if (valid) S = s_sm[(st * RTN_WARPS + w8) * 32 + lane];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty + st);  // this pair of warps holds all it needs of the stage
+    }
+    if (alive && valid) {
       // ---- online softmax (base 2, lazy rescale), this lane owns queries 2t and 2t+1 ----
-      if (__any_sync(0xffffffffu, fmaxf(S[0], S[2]) > m0 + 8.f || fmaxf(S[1], S[3]) > m1 + 8.f)) {
-        float t0 = fmaxf(S[0], S[2]), t1 = fmaxf(S[1], S[3]);
+      float t0 = rtn_coarse(fmaxf(S.x, S.z)), t1 = rtn_coarse(fmaxf(S.y, S.w));
+      if (__any_sync(0xffffffffu, t0 > m0 + 8.f || t1 > m1 + 8.f)) {
 #pragma unroll
         for (int m = 4; m <= 16; m <<= 1) t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, m)), t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, m));
         const float n0 = t0 > m0 + 8.f ? t0 + 0.5f : m0, n1 = t1 > m1 + 8.f ? t1 + 0.5f : m1;
@@ -807,12 +812,11 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
 #pragma unroll
         for (int mt = 0; mt < 8; ++mt) O[mt][0] *= f0, O[mt][1] *= f1, O[mt][2] *= f0, O[mt][3] *= f1;
       }
-      const float p0 = ex2_approx(S[0] - m0), p1 = ex2_approx(S[1] - m1), p2 = ex2_approx(S[2] - m0), p3 = ex2_approx(S[3] - m1);
+      const float p0 = ex2_approx(S.x - m0), p1 = ex2_approx(S.y - m1), p2 = ex2_approx(S.z - m0), p3 = ex2_approx(S.w - m1);
       l0 += p0 + p2, l1 += p1 + p3;
       // ---- values: weights times the per-(row, channel group) scale, one B fragment per group ----
       constexpr int NV = HEAD_DIM / VG;
       uint32_t pb[NV][2];
-      const uint2 vs0 = *reinterpret_cast<const uint2*>(tile + off_vs), vs1 = *reinterpret_cast<const uint2*>(tile + off_vs + 64);
       const uint32_t vsw[4] = {vs0.x, vs0.y, vs1.x, vs1.y};
 #pragma unroll
       for (int gi = 0; gi < NV; ++gi) {
@@ -821,7 +825,6 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
         pb[gi][0] = movmatrix_trans(h2_as_u32(__floats2half2_rn(p0 * sa, p1 * sa)));
         pb[gi][1] = movmatrix_trans(h2_as_u32(__floats2half2_rn(p2 * sb, p3 * sb)));
       }
-      const uint4 vc = *reinterpret_cast<const uint4*>(tile + off_v);
       const uint32_t vv[4] = {vc.x, vc.y, vc.z, vc.w};
 #pragma unroll
       for (int jw = 0; jw < 4; ++jw) {
@@ -836,19 +839,16 @@ __global__ void __launch_bounds__(RTN_THREADS, RTN_CTAS_PER_SM) rtn_decode_kerne
         }
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty + st);
     cur.next(npg_sm, g.h_kv, PAGE, p.batch);
     if (++st == p.n_stages) st = 0, ph ^= 1;
   }
-  if (cur_bh >= 0) flush(cur_b, cur_h);
 }
 
 template <int PAGE, int ARM, int KG, int VG>
 static int launch_rtn_decode(const RtnDecodeParams& prm, int grid, size_t smem, cudaStream_t s) {
   static PerDeviceOnce configured;
   if (configured.first()) {
-    const cudaError_t e = cudaFuncSetAttribute(rtn_decode_kernel<PAGE, ARM, KG, VG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(rtn_decode_kernel<PAGE, ARM, KG, VG>, cudaFuncAttributeMaxDynamicSharedMemorySize, RTN_SMEM);
     if (e != cudaSuccess) {
       configured.retract();
       set_error("bmxk_rtn_decode: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -936,7 +936,7 @@ size_t bmxk_rtn_page_block_bytes(const bmxk_rtn_geom* g) { return g ? (size_t)rt
 size_t bmxk_rtn_decode_workspace_bytes(const bmxk_rtn_geom* g, int batch, int max_pages) {
   if (!g || batch <= 0) return 0;
   (void)max_pages;
-  return 256 + ((size_t)num_sms() * RTN_CTAS_PER_SM + (size_t)batch * g->h_kv) * g->n_q_groups * PART_STRIDE * sizeof(float);
+  return 256 + ((size_t)num_sms() + (size_t)batch * g->h_kv) * g->n_q_groups * PART_STRIDE * sizeof(float);
 }
 
 int bmxk_rtn_append(const bmxk_rtn_geom* g, const void* k, const void* v, int src_dtype, int64_t stride_seq,
@@ -1032,19 +1032,17 @@ int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, co
   cudaStream_t s = (cudaStream_t)stream;
   float* part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + 256);
   const int64_t max_tiles = (int64_t)batch * g->h_kv * (((int64_t)max_pages * g->page + TILE_TOKENS - 1) / TILE_TOKENS);
-  const int most = num_sms() * RTN_CTAS_PER_SM;
-  const int grid = (int)(max_tiles < most ? (max_tiles < 1 ? 1 : max_tiles) : most);
+  const int grid = (int)(max_tiles < num_sms() ? (max_tiles < 1 ? 1 : max_tiles) : num_sms());
   const float scale_log2 = sm_scale * 1.4426950408889634f;
   if (max_pages > 0) {
     RtnDecodeParams prm;
     prm.g = to_rtn(g), prm.q = (const __half*)q, prm.pages = (const uint8_t*)pages, prm.page_table = page_table;
     prm.table_stride = table_stride, prm.n_pages = n_pages, prm.batch = batch, prm.scale_log2 = scale_log2, prm.part = part;
     prm.status = reinterpret_cast<int32_t*>(workspace);
-    // the ring takes what two CTAs per SM leave of the 227 KB; batches of thousands of sequences (page counts in shared memory) get a
-    // shorter ring, never fewer than two stages
-    const size_t fixed = RTN_FIXED_SMEM + (size_t)(2 * batch + 1) * 4 + 16, stage = (size_t)rtn_block_bytes(prm.g) * (TILE_TOKENS / g->page);
+    // batches of thousands of sequences (page counts in shared memory) get a shorter ring
+    const size_t fixed = RTN_FIXED_SMEM + (size_t)(2 * batch + 1) * 4 + 16, stage = (size_t)rtn_block_bytes(prm.g) * (TILE_TOKENS / g->page) + RTN_S_BYTES;
     prm.n_stages = 2;
-    while (prm.n_stages < RTN_MAX_STAGES && fixed + (prm.n_stages + 1) * stage <= 112 * 1024) ++prm.n_stages;
+    while (prm.n_stages < RTN_MAX_STAGES && fixed + (prm.n_stages + 1) * stage <= RTN_SMEM) ++prm.n_stages;
     const size_t smem = fixed + prm.n_stages * stage;
     rc = g->page == 128 ? launch_rtn_decode_k<128>(prm, grid, smem, s) : launch_rtn_decode_k<64>(prm, grid, smem, s);
     if (rc) return rc;

@@ -192,7 +192,7 @@ def test_decode_every_kernel_variant_over_many_tiles(page, arm, k_group, v_group
     """Each instantiation of the decode kernel with more tiles per CTA than its copy ring has stages (ranges that cross heads and
     sequences, ragged page counts, an empty sequence, a half-filled last tile), against float32 attention over the exported
     dequantized pages; queries and keys scaled by opposite powers of two must give the same attention.  Bar: 2e-3 of the largest
-    output, the one of the other decode tests (fp16 rounding of scaled queries and of weights, 2^-11 each)."""
+    output, the one of the other decode tests (fp16 rounding of the dequantized keys and of the weights, 2^-11 each)."""
     from bmx_b200 import kernels as K
 
     if arm == "rtn_channel" and k_group > page:
@@ -226,6 +226,44 @@ def test_decode_every_kernel_variant_over_many_tiles(page, arm, k_group, v_group
             ref = torch.einsum("hgt,htd->hgd", torch.softmax(s, -1), vv).reshape(h_kv * G, 128)
             err = float((out[b].float() - ref).abs().max() / ref.abs().max())
             assert err < 2e-3, f"scale {ks}, sequence {b}: {err:.2e}"
+
+
+@pytest.mark.parametrize("arm,k_group", [("rtn_channel", 32), ("rtn_channel", 128), ("rtn_token", 32), ("rtn_token", 64)])
+@pytest.mark.parametrize("kind", ["plain", "large scores", "mixed heads", "tiny keys"])
+def test_decode_error_does_not_depend_on_ranges_or_other_heads(arm, k_group, kind):
+    """Relative error (2-norm over all channels of a query head) against float64 attention over the exported codes and scales,
+    head by head.  Two-bit keys, and four-bit keys so small that their products with the scale are multiples of 2^-24, are exact
+    fp16 numbers: what is left is one fp16 rounding of each weight, 2^-11 at most.  Rounding queries times scales instead
+    (9e-4 for plain two-bit keys) or scaling the queries of a group together (3e-2 for the small heads) does not stay below
+    that.  "mixed heads": one head's scores pass 2^16, far beyond fp16; the others' are ordinary."""
+    from bmx_b200 import kernels as K
+
+    dev = torch.device("cuda:0")
+    h, G, B, pages = 4, 4, 2, 20
+    kbits, k_scale, q_scale = {"plain": (2, 1.0, [1.0] * 4), "large scores": (2, 1.0, [3.0] * 4),
+                               "mixed heads": (2, 256.0, [1024.0, 2.0 ** -8, 2.0 ** -8, 2.0 ** -10]),
+                               "tiny keys": (4, 2.0 ** -16, [2.0 ** 13] * 4)}[kind]
+    gen = torch.Generator(device=dev).manual_seed(1)
+    channel = torch.exp(torch.randn(1, h, 1, 128, generator=gen, device=dev) * 0.7) * k_scale
+    k = torch.randn(B, h, pages * 128, 128, generator=gen, device=dev) * channel  # float32: tiny keys are not fp16 numbers
+    v = torch.randn(B, h, pages * 128, 128, generator=gen, device=dev)
+    q = (torch.randn(B, h * G, 128, generator=gen, device=dev) * torch.tensor(q_scale, device=dev).repeat(h)[:, None]).half()
+    pool = K.RtnPool(K.rtn_geom(h, G, 128, arm, k_group, 64, kbits, 2), B * pages, dev)
+    table = torch.arange(B * pages, dtype=torch.int32, device=dev).view(B, pages)
+    n_pages = torch.tensor([pages, pages - 3], dtype=torch.int32, device=dev)
+    K.rtn_append(pool, k, v, table.reshape(-1), pages)
+    ws = K.rtn_workspace(pool.geom, B, pages, dev)
+    out = torch.empty(B, h * G, 128, dtype=torch.float32, device=dev)
+    K.rtn_decode(pool, q, table, n_pages, pages, None, None, None, 128 ** -0.5, ws, out=out)
+    K.check_status(ws)
+    ex = K.rtn_export(pool, table.reshape(-1), dequant=True)
+    kd, vd = (ex[n].view(B, pages * 128, h, 128).permute(0, 2, 1, 3).double() for n in ("k_deq", "v_deq"))
+    for b in range(B):
+        n = int(n_pages[b]) * 128
+        s = torch.einsum("hgd,htd->hgt", q[b].double().view(h, G, 128), kd[b, :, :n]) * 128 ** -0.5
+        want = torch.einsum("hgt,htd->hgd", torch.softmax(s, -1), vd[b, :, :n])
+        err = (out[b].double().view(h, G, 128) - want).norm(dim=(0, 2)) / want.norm(dim=(0, 2))
+        assert bool((err < 2.0 ** -11).all()), f"sequence {b}: {err.tolist()}"
 
 
 def _rtn_codes(x, bits, group, dim):
