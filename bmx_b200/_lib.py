@@ -130,6 +130,8 @@ _SIGNATURES = {
     "bmxk_check_workspace_status": (c_int, [c_void_p, c_void_p]),
     "bmxk_k2b_decode_static_status": (c_int, [c_void_p]),
     "bmxk_selftest_bounded_wait": (c_int, [c_void_p, ctypes.c_int64, c_void_p]),
+    "bmxk_selftest_rtn_lost_copy": (c_int, [POINTER(RtnGeom), c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_float, c_void_p,
+                                            c_size_t, c_void_p, c_int, ctypes.c_int64, c_void_p]),
 }
 
 _lib = None

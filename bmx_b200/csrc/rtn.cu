@@ -559,6 +559,8 @@ struct RtnDecodeParams {
   float* part;
   int32_t* status;
   int n_stages;
+  long long wait_limit;  // cycles after which a wait gives up
+  int lost;              // self-test: the tile of every range whose copy is left out, or -1
 };
 
 constexpr int RTN_WARPS = 8;                             // score warps, and as many value warps
@@ -569,21 +571,23 @@ constexpr int RTN_FIXED_SMEM = (8 * 8 * HEAD_DIM + 128) * 4 + (2 + RTN_WARPS) * 
 constexpr int RTN_SMEM = 200 * 1024;                     // most that the ring may grow to
 
 // Bounded wait that reports where it ran out.  It does not look at the status word first: this entry point never asked for a
-// cleared workspace, so what the word holds before the call means nothing.
-__device__ __forceinline__ bool rtn_wait(uint64_t* bar, uint32_t parity, int32_t* status, int where) {
+// cleared workspace, so what the word holds before the call means nothing.  A warp whose wait ran out hands nothing on, so the waits of
+// those that depend on it run out as well: the copy warp never fills a stage that was not given back, and waits for the copies in
+// flight before it ends.
+__device__ __forceinline__ bool rtn_wait(uint64_t* bar, uint32_t parity, const RtnDecodeParams& p, int where) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (uint32_t spin = 1;; ++spin) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 255u) == 0u && clock64() - t0 > WAIT_LIMIT_CYCLES) {
-      status[0] = 1, status[1] = blockIdx.x, status[2] = where;
+    if ((spin & 255u) == 0u && clock64() - t0 > p.wait_limit) {
+      p.status[0] = 1, p.status[1] = blockIdx.x, p.status[2] = where;
       return false;
     }
   }
 }
-__device__ __forceinline__ bool rtn_warp_wait(uint64_t* bar, uint32_t parity, int32_t* status, int where) {
+__device__ __forceinline__ bool rtn_warp_wait(uint64_t* bar, uint32_t parity, const RtnDecodeParams& p, int where) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;  // the usual case, without divergence
-  return __all_sync(0xffffffffu, rtn_wait(bar, parity, status, where));
+  return __all_sync(0xffffffffu, rtn_wait(bar, parity, p, where));
 }
 __device__ __forceinline__ void rtn_value_warps_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
@@ -647,12 +651,13 @@ __global__ void __launch_bounds__(RTN_THREADS, 1) rtn_decode_kernel(const RtnDec
         slots_b = cur.b, slots_j = page0;
         slots = page0 + lane < npg_sm[cur.b] ? p.page_table[(int64_t)cur.b * p.table_stride + page0 + lane] : 0;
       }
-      if (!rtn_warp_wait(empty + st, ph, p.status, 60)) break;
-      if (lane == 0) mbar_arrive_expect_tx(full + st, (uint32_t)(pages_here * PB));
+      if (!rtn_warp_wait(empty + st, ph, p, 60)) break;
+      const bool copies = lane == 0 && f - f_begin != p.lost;
+      if (copies) mbar_arrive_expect_tx(full + st, (uint32_t)(pages_here * PB));
 #pragma unroll
       for (int i = 0; i < PAGES_PER_TILE; ++i) {
         const int slot = __shfl_sync(0xffffffffu, slots, page0 - slots_j + i);
-        if (lane == 0 && i < pages_here)
+        if (copies && i < pages_here)
           bulk_g2s(ring + st * stage_bytes + i * PB, p.pages + ((int64_t)slot * g.h_kv + cur.h) * PB, (uint32_t)PB, full + st);
       }
       ++issued;
@@ -660,7 +665,7 @@ __global__ void __launch_bounds__(RTN_THREADS, 1) rtn_decode_kernel(const RtnDec
       if (++st == p.n_stages) st = 0, ph ^= 1;
     }
     for (int i = max(0, issued - p.n_stages); i < issued; ++i)  // no copy is in flight when this CTA ends, whatever became of its readers
-      rtn_warp_wait(full + i % p.n_stages, (uint32_t)(i / p.n_stages) & 1u, p.status, 62);
+      rtn_warp_wait(full + i % p.n_stages, (uint32_t)(i / p.n_stages) & 1u, p, 62);
     return;
   }
 
@@ -686,7 +691,7 @@ __global__ void __launch_bounds__(RTN_THREADS, 1) rtn_decode_kernel(const RtnDec
 #pragma unroll
         for (int n = 0; n < 16; ++n) qb[n] = (gq < G) ? *reinterpret_cast<const uint32_t*>(qp + 8 * n) : 0u;
       }
-      if (!rtn_warp_wait(full + st, ph, p.status, 61)) break;
+      if (!rtn_warp_wait(full + st, ph, p, 61)) break;
       if (valid) {
         const uint8_t* tile = ring + st * stage_bytes;
         const uint4 k0 = *reinterpret_cast<const uint4*>(tile + off_k), k1 = *reinterpret_cast<const uint4*>(tile + off_k + 512);
@@ -785,7 +790,7 @@ __global__ void __launch_bounds__(RTN_THREADS, 1) rtn_decode_kernel(const RtnDec
       for (int mt = 0; mt < 8; ++mt) O[mt][0] = O[mt][1] = O[mt][2] = O[mt][3] = 0.f;
     }
     const bool valid = PAGES_PER_TILE == 1 || cur.j * PAGES_PER_TILE + sub_page < npg_sm[b];
-    if (alive) alive = rtn_warp_wait(full + st, ph, p.status, 64);
+    if (alive) alive = rtn_warp_wait(full + st, ph, p, 64);
     uint2 vs0 = make_uint2(0u, 0u), vs1 = vs0;
     uint4 vc = make_uint4(0u, 0u, 0u, 0u);
     if (alive && valid) {
@@ -793,7 +798,7 @@ __global__ void __launch_bounds__(RTN_THREADS, 1) rtn_decode_kernel(const RtnDec
       vs0 = *reinterpret_cast<const uint2*>(tile + off_vs), vs1 = *reinterpret_cast<const uint2*>(tile + off_vs + 64);
       vc = *reinterpret_cast<const uint4*>(tile + off_v);
     }
-    if (alive) alive = rtn_warp_wait(scored + st * RTN_WARPS + w8, ph, p.status, 63);
+    if (alive) alive = rtn_warp_wait(scored + st * RTN_WARPS + w8, ph, p, 63);
     float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
     if (alive) {
       if (valid) S = s_sm[(st * RTN_WARPS + w8) * 32 + lane];
@@ -1014,10 +1019,10 @@ int bmxk_rtn_dequant_dense(const bmxk_rtn_geom* g, const void* pages, const int3
   return check_launch("bmxk_rtn_dequant_dense");
 }
 
-int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,
-                    const int32_t* n_pages, int batch, int max_pages, const void* k_tail, const void* v_tail,
-                    const int32_t* tail_len, int tail_cap, float sm_scale, void* workspace, size_t workspace_bytes, void* out,
-                    int out_dtype, float* partial_out, void* stream) {
+static int rtn_decode_impl(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,
+                           const int32_t* n_pages, int batch, int max_pages, const void* k_tail, const void* v_tail,
+                           const int32_t* tail_len, int tail_cap, float sm_scale, void* workspace, size_t workspace_bytes, void* out,
+                           int out_dtype, float* partial_out, long long wait_limit, int lost, void* stream) {
   int rc = check_rtn_geom(g, "bmxk_rtn_decode");
   if (rc) return rc;
   BMXK_REQUIRE(batch >= 1 && (int64_t)batch * g->h_kv <= MAX_BH, "bmxk_rtn_decode: batch*h_kv out of range");
@@ -1038,7 +1043,7 @@ int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, co
     RtnDecodeParams prm;
     prm.g = to_rtn(g), prm.q = (const __half*)q, prm.pages = (const uint8_t*)pages, prm.page_table = page_table;
     prm.table_stride = table_stride, prm.n_pages = n_pages, prm.batch = batch, prm.scale_log2 = scale_log2, prm.part = part;
-    prm.status = reinterpret_cast<int32_t*>(workspace);
+    prm.status = reinterpret_cast<int32_t*>(workspace), prm.wait_limit = wait_limit, prm.lost = lost;
     // batches of thousands of sequences (page counts in shared memory) get a shorter ring
     const size_t fixed = RTN_FIXED_SMEM + (size_t)(2 * batch + 1) * 4 + 16, stage = (size_t)rtn_block_bytes(prm.g) * (TILE_TOKENS / g->page) + RTN_S_BYTES;
     prm.n_stages = 2;
@@ -1056,6 +1061,25 @@ int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, co
   mp.tail_cap = tail_cap, mp.signs = nullptr, mp.scale_log2 = scale_log2, mp.out = out, mp.out_dtype = out_dtype;
   mp.partial_out = partial_out;
   return launch_merge(mp, s, max_pages > 0);
+}
+
+int bmxk_rtn_decode(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,
+                    const int32_t* n_pages, int batch, int max_pages, const void* k_tail, const void* v_tail,
+                    const int32_t* tail_len, int tail_cap, float sm_scale, void* workspace, size_t workspace_bytes, void* out,
+                    int out_dtype, float* partial_out, void* stream) {
+  return rtn_decode_impl(g, q, pages, page_table, table_stride, n_pages, batch, max_pages, k_tail, v_tail, tail_len, tail_cap, sm_scale, workspace,
+                         workspace_bytes, out, out_dtype, partial_out, WAIT_LIMIT_CYCLES, -1, stream);
+}
+
+int bmxk_selftest_rtn_lost_copy(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,
+                                const int32_t* n_pages, int batch, int max_pages, float sm_scale, void* workspace, size_t workspace_bytes,
+                                void* out, int lost_tile, int64_t limit_cycles, void* stream) {
+  BMXK_REQUIRE(lost_tile >= 0, "bmxk_selftest_rtn_lost_copy: lost_tile=%d", lost_tile);
+  BMXK_REQUIRE(limit_cycles >= 1000 && limit_cycles <= 200000000,
+               "bmxk_selftest_rtn_lost_copy: limit of %lld cycles outside [1e3, 2e8] (this test must end within a fraction of a second)",
+               (long long)limit_cycles);
+  return rtn_decode_impl(g, q, pages, page_table, table_stride, n_pages, batch, max_pages, nullptr, nullptr, nullptr, 0, sm_scale, workspace,
+                         workspace_bytes, out, BMXK_DTYPE_F16, nullptr, (long long)limit_cycles, lost_tile, stream);
 }
 
 }  // extern "C"

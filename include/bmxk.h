@@ -436,6 +436,13 @@ int bmxk_check_workspace_status(const void* workspace, void* stream);
  * caller; read it with bmxk_check_workspace_status, which must then return BMXK_ERR_DEVICE. */
 int bmxk_selftest_bounded_wait(int32_t* status, int64_t limit_cycles, void* stream);
 
+/* The RTN decode step (fp16 output, no window) with the copy of one tile of every CTA's range left out and waits limited to
+ * limit_cycles: the waits that depend on it run out, the kernel reports in the workspace's status word and ends with no copy in
+ * flight.  The output is not meaningful. */
+int bmxk_selftest_rtn_lost_copy(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,
+                                const int32_t* n_pages, int batch, int max_pages, float sm_scale, void* workspace, size_t workspace_bytes,
+                                void* out, int lost_tile, int64_t limit_cycles, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -68,6 +68,43 @@ def test_bounded_wait_runs_out_and_reports_block_and_site():
         K.selftest_bounded_wait(status, 10**12)
 
 
+@pytest.mark.parametrize("page,lost", [(128, 0), (128, 5), (128, 20), (64, 3)])
+def test_decode_with_a_lost_copy_reports_and_ends(page, lost):
+    """The RTN decode kernel whose copy warp leaves one tile out: everything that depends on it gives up after ~1 ms, no stage is
+    filled again that was not given back, and the next step over the same buffers is the one that a fresh workspace gives."""
+    import ctypes
+
+    from bmx_b200 import kernels as K
+    from bmx_b200._lib import BmxkError, call
+
+    dev = _dev()
+    B, h_kv, G, pages = 9, 8, 2, 46 * 128 // page  # 3312 tiles: 23 per CTA, several passes over the ring
+    g = K.rtn_geom(h_kv, G, page, "rtn_channel", 32, 32, 4, 2)
+    gen = torch.Generator(device=dev).manual_seed(page + lost)
+    k, v = (torch.randn(B, h_kv, pages * page, D, generator=gen, device=dev).half() for _ in range(2))
+    q = torch.randn(B, h_kv * G, D, generator=gen, device=dev).half()
+    pool = K.RtnPool(g, B * pages, dev)
+    table = torch.arange(B * pages, dtype=torch.int32, device=dev).view(B, pages)
+    n_pages = torch.full((B,), pages, dtype=torch.int32, device=dev)
+    K.rtn_append(pool, k, v, table.reshape(-1), pages)
+    ws = K.rtn_workspace(g, B, pages, dev)
+    want = K.rtn_decode(pool, q, table, n_pages, pages, None, None, None, D ** -0.5, ws)
+    out = torch.empty_like(want)
+    for _ in range(2):
+        call("bmxk_selftest_rtn_lost_copy", ctypes.byref(g), q.data_ptr(), pool.pages.data_ptr(), table.data_ptr(), table.stride(0),
+             n_pages.data_ptr(), B, pages, D ** -0.5, ws.data_ptr(), ws.numel(), out.data_ptr(), lost, 2_000_000,
+             torch.cuda.current_stream().cuda_stream)
+        with pytest.raises(BmxkError) as ei:
+            K.check_status(ws)
+        assert ei.value.code == 3 and "site 6" in str(ei.value)
+        ws[:16].zero_()
+    assert torch.equal(K.rtn_decode(pool, q, table, n_pages, pages, None, None, None, D ** -0.5, ws), want)
+    K.check_status(ws)
+    with pytest.raises(BmxkError):
+        call("bmxk_selftest_rtn_lost_copy", ctypes.byref(g), q.data_ptr(), pool.pages.data_ptr(), table.data_ptr(), table.stride(0),
+             n_pages.data_ptr(), B, pages, D ** -0.5, ws.data_ptr(), ws.numel(), out.data_ptr(), lost, 10 ** 12, None)
+
+
 def test_exchange_kernel_alone_on_one_gpu():
     """bmxk_xchg_merge with a world of one: the rank stores its state into its own buffer, flags, finds its flag and
     normalises; two steps use both buffer parities, a third takes the step number from the buffer's own count.  (Several
