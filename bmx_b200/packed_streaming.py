@@ -435,9 +435,8 @@ class PackedStreamingLayer(DynamicLayer):
         if self._mask_is_causal(attention_mask, n_q, S):  # the model's plain causal mask: no per-sequence mask, no copies of K / V
             if n_q == S:
                 return F.scaled_dot_product_attention(q, Kd, Vd, is_causal=n_q > 1, scale=scaling, enable_gqa=gqa)
-            if attention_mask.dtype == torch.bool:  # it is that mask: one row block for all sequences
-                mask = attention_mask[:1]
-            else:
+            mask = attention_mask[:1]  # one row block for all sequences
+            if mask.dtype != torch.bool or mask.device != q.device or not mask.is_contiguous():
                 mask = torch.ones(n_q, S, dtype=torch.bool, device=q.device).tril(S - n_q)
             return F.scaled_dot_product_attention(q, Kd, Vd, attn_mask=mask, scale=scaling, enable_gqa=gqa)
         Kx = Kd.repeat_interleave(self._n_q_groups, dim=1)
