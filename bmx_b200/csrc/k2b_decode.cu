@@ -954,6 +954,10 @@ int bmxk_check_workspace_status(const void* workspace, void* stream) {
     set_error("window append: a sequence's fp16 window was full (a flush was skipped); nothing was written");
     return BMXK_ERR_DEVICE;
   }
+  if (st[0] == 3) {
+    set_error("paged prefill: rotation tables rearranged for %d pages, %d are visible; the output lacks keys", st[1], st[2]);
+    return BMXK_ERR_DEVICE;
+  }
   if (st[0] != 0) {
     set_error("decode kernel: a bounded wait ran out in block %d (site %d)", st[1], st[2]);
     return BMXK_ERR_DEVICE;

@@ -784,8 +784,16 @@ static int launch_p5(const PrefillParams& prm, dim3 grid, size_t smem, cudaStrea
 // Rotation tables in the order of the key warps' reads.  Every block of query positions and every head walks the same pages, and
 // reading the tables row by row (16 bytes out of each of 32 rows per load) kept the L1 tag stage 79 % busy and the key warps
 // waiting.  The copy costs 256 bytes and about 0.25 ns per position.  One block per 256 of a page's 2048 pieces.
+// The first block also reports a sequence whose last row (position last_pos) sees more pages than are rearranged: the kernel that
+// follows leaves them out.  (The test in that kernel's prologue cost it 1 %.)
 __global__ void __launch_bounds__(256) rope_fragments_kernel(const __half* __restrict__ rope_cos, const __half* __restrict__ rope_sin,
-                                                             int64_t pos_offset, uint4* __restrict__ frag) {
+                                                             int64_t pos_offset, uint4* __restrict__ frag, int rope_pages, const int32_t* __restrict__ n_pages,
+                                                             int batch, int64_t last_pos, int32_t* __restrict__ status) {
+  if (blockIdx.x == 0 && last_pos >= pos_offset)
+    for (int b = threadIdx.x; b < batch; b += 256) {
+      const int visible = (int)min((int64_t)n_pages[b], (last_pos - pos_offset) / 128 + 1);
+      if (visible > rope_pages && atomicCAS(status, 0, 3) == 0) status[1] = rope_pages, status[2] = visible;
+    }
   const int u = (blockIdx.x & 7) * 256 + threadIdx.x, page = blockIdx.x >> 3;
   const int lane = u & 31, half = (u >> 5) & 1, wq = (u >> 6) & 3, chunk = (u >> 8) & 3;
   const __half* t = (u >> 10) ? rope_sin : rope_cos;
@@ -814,7 +822,8 @@ int launch_prefill_t5(const PrefillParams& prm, dim3 grid, cudaStream_t s) {
   BMXK_REQUIRE(smem <= 227 * 1024, "bmxk_k2b_prefill: rank=%d group=%d needs %zu bytes of shared memory", prm.g.rank, prm.g.group, smem);
   int rc;
   if (prm.rope_frag) {
-    rope_fragments_kernel<<<(unsigned)prm.rope_pages * 8, 256, 0, s>>>(prm.rope_cos, prm.rope_sin, prm.pos_offset, prm.rope_frag);
+    rope_fragments_kernel<<<(unsigned)prm.rope_pages * 8, 256, 0, s>>>(prm.rope_cos, prm.rope_sin, prm.pos_offset, prm.rope_frag, prm.rope_pages,
+                                                                              prm.n_pages, (int)grid.z, prm.q_pos0 + prm.n_q - 1, prm.status);
     rc = check_launch("bmxk_k2b_prefill(rope fragments)");
     if (rc) return rc;
     rc = prm.g.rank == 32 ? launch_p5<32, true>(prm, grid, smem, s) : launch_p5<16, true>(prm, grid, smem, s);

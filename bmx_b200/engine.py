@@ -225,13 +225,15 @@ class K2bLayerState:
     ROPE_FRAGMENT_TILES = 24
 
     def prefill_rope_pages(self, n_q: int, q_pos0: int) -> int:
-        """Pages whose rotation tables the prefill kernel should rearrange first (all that the last row sees), or 0."""
-        pages = min(self.committed // self.page, max(0, q_pos0 + n_q - 1) // self.page + 1)
+        """Pages whose rotation tables the prefill kernel should rearrange first (all that the last row's position can see, whatever
+        the page counts are when a captured call runs), or 0."""
+        seen = max(0, q_pos0 + n_q - 1) // self.page + 1
+        pages = min(self.committed // self.page, seen)
         blocks = -(-n_q // (128 // self.geom.n_q_groups)) * self.geom.h_kv * self.batch
         n_sm = _sm_count(self.device)
-        if blocks * pages < self.ROPE_FRAGMENT_TILES * n_sm or self.rope_cos.shape[0] < pages * self.page:
+        if blocks * pages < self.ROPE_FRAGMENT_TILES * n_sm or self.rope_cos.shape[0] < seen * self.page:
             return 0
-        return pages
+        return seen
 
     def prefill_split(self, n_q: int) -> int:
         """Shares of the page walk per block of query positions.  One CTA per (block, KV head, sequence) fills the GPU only

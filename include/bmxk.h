@@ -176,7 +176,8 @@ int bmxk_k2b_prefill_split(const bmxk_k2b_geom* g, const void* q, int n_q, int64
 /* bmxk_k2b_prefill_split (n_split = 1: unsplit) that first rearranges the rotation tables of the positions pos_offset ..
  * pos_offset + 128 * rope_pages - 1 into the order its key warps read, behind the partial records in `workspace`
  * (bmxk_k2b_prefill_workspace_bytes + bmxk_k2b_prefill_rope_bytes).  Worth its few microseconds when many blocks and heads walk the
- * same pages.  rope_pages has to cover every committed page that a row of q sees.  Same results. */
+ * same pages.  rope_pages has to cover every committed page that a row of q sees (the page counts are on the device: too few are
+ * reported in the status word as (3, rope_pages, visible)).  Same results. */
 size_t bmxk_k2b_prefill_rope_bytes(int rope_pages);
 int bmxk_k2b_prefill_rope(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t q_pos0, const void* pages, const void* coefs,
                           const void* basis_f16, const int32_t* page_table, int table_stride, const int32_t* n_pages, int batch,

@@ -314,3 +314,13 @@ def test_rearranged_rotation_tables_change_nothing(rank, G, n_q, tokens, n_split
     want = run(0)
     assert torch.equal(run(pages), want) and (pages == 0 or bool(want.abs().sum() > 0))
     K.check_status(st.workspace)
+    # tables for too few pages: reported, and the engine's own rule covers every page that the positions can see
+    if pages > 1 and tokens - n_q > 128 * (pages - 1):
+        from bmx_b200._lib import BmxkError
+
+        run(pages - 1)
+        with pytest.raises(BmxkError, match=f"{pages - 1} pages, {pages} are visible"):
+            K.check_status(st.workspace)
+        st.workspace[:16].zero_()
+    st.ROPE_FRAGMENT_TILES = 0
+    assert st.prefill_rope_pages(n_q, tokens - n_q) * 128 >= tokens
