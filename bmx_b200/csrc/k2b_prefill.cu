@@ -488,7 +488,9 @@ static int prefill_impl(const bmxk_k2b_geom* g, const void* q, int n_q, int64_t 
   const dim3 grid((unsigned)((n_q + pp - 1) / pp), (unsigned)g->h_kv, (unsigned)batch);
   cudaStream_t s = (cudaStream_t)stream;
   const bool aligned16 = ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 15) == 0;
-  const bool t5 = g_prefill_kernel.load(std::memory_order_relaxed) == 0 && aligned16;
+  // the tcgen05 kernel takes maxima of unscaled scores, hides keys as minus infinity before the scale and divides log norms by it: positive
+  // scales only
+  const bool t5 = g_prefill_kernel.load(std::memory_order_relaxed) == 0 && aligned16 && sm_scale > 0.f;
   BMXK_REQUIRE(n_split >= 1 && n_split <= 64, "bmxk_k2b_prefill_split: n_split=%d must be in 1..64", n_split);
   if (!t5) n_split = 1;  // the split is the tcgen05 kernel's; the mma.sync kernel walks every page of a block in one CTA
   if (!t5) rope_pages = 0;

@@ -186,7 +186,7 @@ int bmxk_k2b_prefill_rope(const bmxk_k2b_geom* g, const void* q, int n_q, int64_
                           int32_t* status, void* out, int n_split, int rope_pages, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Which kernel bmxk_k2b_prefill launches (process-wide; no counterpart in bmx).  0 (default): the tcgen05 kernel when q
- * and out are 16-byte aligned, else the mma.sync kernel; 1: always the mma.sync kernel.  Both give the same attention
+ * and out are 16-byte aligned and sm_scale is positive, else the mma.sync kernel; 1: always the mma.sync kernel.  Both give the same attention
  * within the path's tolerance. */
 int bmxk_k2b_prefill_select(int kernel);
 

@@ -324,3 +324,30 @@ def test_rearranged_rotation_tables_change_nothing(rank, G, n_q, tokens, n_split
         st.workspace[:16].zero_()
     st.ROPE_FRAGMENT_TILES = 0
     assert st.prefill_rope_pages(n_q, tokens - n_q) * 128 >= tokens
+
+
+@pytest.mark.parametrize("sm_scale", [-0.05, 0.0, 0.05])
+@pytest.mark.parametrize("n_q,tokens", [(70, 900), (5, 200)])
+def test_any_softmax_scale(sm_scale, n_q, tokens):
+    """Negative and zero scales attend as in the general formula (hidden keys stay hidden): against float64 over the dequantized pages."""
+    from bmx_b200 import kernels as K
+    from bmx_b200.engine import K2bLayerState
+    from bmx_b200.rope import default_rope_tables
+
+    dev = torch.device("cuda:0")
+    h, G, B = 2, 4, 1
+    gen = torch.Generator(device=dev).manual_seed(tokens)
+    cos, sin = (t.half() for t in default_rope_tables(5e5, 128, tokens + 256, device=dev))
+    st = K2bLayerState(K.k2b_geom(h, G, 128, 32, 64, h), B, tokens, 100, dev, cos, sin)
+    st.set_basis(torch.randn(h * 128, 32, generator=gen, device=dev) / 11)
+    k, v = (torch.randn(B, h, tokens, 128, generator=gen, device=dev).half() for _ in range(2))
+    st.append(k, k, v)
+    st.sm_scale = sm_scale
+    q = torch.randn(B, h * G, n_q, 128, generator=gen, device=dev).half()
+    got = st.prefill_attend(q, tokens - n_q).double().view(h, G, n_q, 128)
+    K.check_status(st.workspace)
+    kd, vd = (t[0].double() for t in st.dense_kv(torch.float16))
+    s = torch.einsum("hgnd,htd->hgnt", q[0].double().view(h, G, n_q, 128), kd) * sm_scale
+    s = s.masked_fill(~torch.ones(n_q, tokens, dtype=torch.bool, device=dev).tril(tokens - n_q), float("-inf"))
+    want = torch.einsum("hgnt,htd->hgnd", torch.softmax(s, -1), vd)
+    assert float((got - want).norm() / want.norm()) < 2e-3  # fp16 keys, weights and outputs, 2^-11 each
