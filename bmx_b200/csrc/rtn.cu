@@ -45,10 +45,12 @@ BMXK_HD int rtn_block_bytes(const RtnGeom& g) { return rtn_off_vscale(g) + g.pag
 // the codes inside the clamp.
 // Two-bit codes of 16-bit sources (all values; keys of the kivi recipe) need no quotient: qmax is 1, the scale is the group's
 // maximum s itself, and x / s > 1/2 exactly when x > s / 2 (two 11-bit numbers whose quotient is not 1/2 are 2^-12 away from it, so
-// the division's rounding cannot reach it; a tie is code 0 either way): two packed compares per pair.  A page with a NaN, an
-// infinite, zero or subnormal maximum takes the general way.
-// Measured, 4096 blocks (four sequences of 16384 tokens x 8 heads, 2-bit keys per channel, groups of 64, fp16): 417 -> 109 us = 3.0 TB/s;
-// 4-bit keys in groups of 32, half as many blocks: 243 -> 82 us (float32 sources 253 -> 121 us).
+// the division's rounding cannot reach it; a tie is code 0 either way): two packed compares per pair.  A group of
+// zeros (a padded token, a dead channel) needs nothing else: no value is above a threshold of zero.  A page whose two-bit groups
+// include one with a NaN or an infinite or subnormal maximum takes the general way.
+// Measured, 4096 blocks (four sequences of 16384 tokens x 8 heads, 2-bit keys per channel, groups of 64, fp16): 417 -> 109 us = 3.0 TB/s,
+// the same with a padded token or a dead channel in every page (419, 489 before), 210 us where every page takes the general way;
+// 4-bit keys in groups of 32: 413 -> 153 us, half as many blocks 243 -> 82 us (float32 sources 253 -> 121 us).
 // ---------------------------------------------------------------------------------------------
 constexpr int RTNQ_THREADS = 256;
 constexpr float RTN_NEAR = 4e-6f, RTN_MAGIC = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer, ties to even
@@ -64,7 +66,7 @@ struct RtnSrc<__half> {
   static __device__ __forceinline__ uint32_t above(Pair x, uint32_t t) { return __hgt2_mask(u32_as_h2(x), u32_as_h2(t)); }  // 0xFFFF per half
   static __device__ __forceinline__ uint32_t below(Pair x, uint32_t t) { return __hlt2_mask(u32_as_h2(x), __hneg2(u32_as_h2(t))); }
   static __device__ __forceinline__ uint32_t halves(float a, float b) { return h2_as_u32(__floats2half2_rn(0.5f * a, 0.5f * b)); }
-  static __device__ __forceinline__ bool plain(float m) { return m >= 2.5e-4f && m <= 65504.f; }  // m / 2 is a normal number of the type
+  static __device__ __forceinline__ bool plain(float m) { return m == 0.f || (m >= 2.5e-4f && m <= 65504.f); }  // m / 2 is zero or a normal number of the type
 };
 template <>
 struct RtnSrc<__nv_bfloat16> {
@@ -85,7 +87,7 @@ struct RtnSrc<__nv_bfloat16> {
     const __nv_bfloat162 r = __floats2bfloat162_rn(0.5f * a, 0.5f * b);
     return *reinterpret_cast<const uint32_t*>(&r);
   }
-  static __device__ __forceinline__ bool plain(float m) { return m >= 1e-30f && m <= 3.3e38f; }
+  static __device__ __forceinline__ bool plain(float m) { return m == 0.f || (m >= 1e-30f && m <= 3.3e38f); }
 };
 template <>
 struct RtnSrc<float> {
@@ -146,6 +148,8 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
   __half* vscale = reinterpret_cast<__half*>(blk + rtn_off_vscale(g));
   const float kq = (float)((1 << (g.kbits - 1)) - 1), vq = (float)((1 << (g.vbits - 1)) - 1);
 
+  __shared__ int odd_s;
+  if (tid == 0) odd_s = 0;
   // ---- staging ----
   if (vec & 1) {
     constexpr int PER_ROW = HEAD_DIM * (int)sizeof(T) / 16, N = PAGE * PER_ROW / RTNQ_THREADS, PER = 16 / (int)sizeof(T);
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       float2 mf = S::f(m);
       if (mf.x != mf.x || mf.y != mf.y) {  // the reference's maximum passes over NaN
         m = Pair{};
-        odd = true;
+        odd |= two;
         for (int i = 0; i < 16; ++i) m = S::absmax(m, *reinterpret_cast<const Pair*>(st + rtn_at<ROW>(r, (16 * qt + i) * (int)sizeof(Pair))));
         mf = S::f(m);
       }
@@ -200,7 +204,7 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       if (grp == 128) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
       const float s = fmaxf(am, 1e-12f) / qmax;
       sc[u] = s;  // [row][32-channel quarter]
-      odd |= !S::plain(am);
+      odd |= two && !S::plain(am);
       if (two) reinterpret_cast<uint32_t*>(inv)[u] = S::halves(s, s);
       else inv[u] = 1.f / s;
       const int per = grp / 32;
@@ -217,7 +221,7 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       float2 mf = S::f(m);
       if (mf.x != mf.x || mf.y != mf.y) {
         m = Pair{};
-        odd = true;
+        odd |= k2;
         for (int r = 0; r < 32; ++r) m = S::absmax(m, *reinterpret_cast<const Pair*>(kst + rtn_at<ROW>(32 * rb + r, c2 * (int)sizeof(Pair))));
         mf = S::f(m);
       }
@@ -232,7 +236,7 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
       float am = 0.f;
       for (int i = 0; i < per; ++i) am = fmaxf(am, ksc[(g0 + i) * HEAD_DIM + c]);
       sc[n] = fmaxf(am, 1e-12f) / kq;
-      odd |= !S::plain(am);
+      odd |= k2 && !S::plain(am);
       if (rb == g0) kscale[k2b_kscale_idx(rb / per, c)] = __float2half_rn(sc[n]);
     }
     __syncthreads();
@@ -251,7 +255,9 @@ __global__ void __launch_bounds__(RTNQ_THREADS, sizeof(T) == 2 ? 3 : 1) rtn_quan
     token_scales(kst, g.k_group, kq, k2, ksc, kinv, kscale);
   }
   token_scales(vst, g.v_group, vq, V2, vsc, vinv, vscale);
-  const bool packed = !__syncthreads_or(odd);
+  if (odd) odd_s = 1;
+  __syncthreads();
+  const bool packed = odd_s == 0;
 
   // ---- keys: thread = (16-row block, row g and g + 8, lane t of the quad): channels 8n + 2t, + 1 of two rows, 16 bytes each ----
   for (int u = tid; u < PAGE * 2; u += RTNQ_THREADS) {

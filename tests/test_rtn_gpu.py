@@ -282,7 +282,7 @@ def _rtn_codes(x, bits, group, dim):
 @pytest.mark.parametrize("page,arm,k_group,v_group,kbits", [
     (128, "rtn_channel", 64, 64, 2), (128, "rtn_channel", 32, 128, 4), (128, "rtn_channel", 128, 32, 3), (128, "rtn_token", 32, 64, 4),
     (128, "rtn_token", 128, 128, 2), (64, "rtn_channel", 32, 32, 3), (64, "rtn_channel", 64, 64, 4), (64, "rtn_token", 64, 32, 2)])
-@pytest.mark.parametrize("kind", ["normal", "ties", "extremes"])
+@pytest.mark.parametrize("kind", ["normal", "ties", "padded", "extremes"])
 def test_append_codes_equal_the_divided_ones(dtype, page, arm, k_group, v_group, kbits, kind):
     """Every code and scale of the page quantizer, whose divisions are products with the inverse scale, equals the divided one, ties,
     zeros, infinities and NaN included; also from rows that start off the sixteen-byte boundaries."""
@@ -295,6 +295,9 @@ def test_append_codes_equal_the_divided_ones(dtype, page, arm, k_group, v_group,
     k, v = torch.randn(n, h, T, 128, generator=gen), torch.randn(n, h, T, 128, generator=gen)
     if kind == "ties":  # a coarse grid: quotients fall on halves
         k, v = torch.randint(-7, 8, k.shape, generator=gen) * 0.5, torch.randint(-3, 4, v.shape, generator=gen) * 0.25
+    elif kind == "padded":  # groups of nothing but zeros, of either sign, among ordinary ones
+        for x in (k, v):
+            x[:, :, 3::17], x[:, :, 4::17], x[..., 7], x[..., 64:96] = 0.0, -0.0, 0.0, -0.0
     elif kind == "extremes":
         for x in (k, v):
             x[:, :, 3::17] = 0
