@@ -936,6 +936,25 @@ static int rtn_append_impl(const RtnGeom& g, const void* k, const void* v, int64
   return launch_rtn_quant<T, 64>(g, (const T*)k, (const T*)v, ss, sh, st, slots, blocks, n_pages, pages, vec, s);
 }
 
+template <typename OutT, int PAGE>
+static int launch_rtn_dense(const RtnGeom& g, int blocks, const uint8_t* pages, const int32_t* page_table, int table_stride, int n_pages,
+                            const __half* k_tail, const __half* v_tail, int tail_len, int tail_cap, OutT* k_out, OutT* v_out, int64_t row_stride,
+                            cudaStream_t s) {
+  constexpr int smem = 2 * PAGE * 256;
+  static PerDeviceOnce configured;
+  if (configured.first()) {
+    const cudaError_t e = cudaFuncSetAttribute(rtn_dequant_dense_kernel<OutT, PAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+      configured.retract();
+      set_error("bmxk_rtn_dequant_dense: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      return BMXK_ERR_CUDA;
+    }
+  }
+  rtn_dequant_dense_kernel<OutT, PAGE><<<dim3((unsigned)blocks, (unsigned)g.h_kv), RTND_THREADS, smem, s>>>(
+      g, pages, page_table, table_stride, n_pages, k_tail, v_tail, tail_len, tail_cap, k_out, v_out, row_stride);
+  return check_launch("bmxk_rtn_dequant_dense");
+}
+
 }  // namespace bmxk
 
 using namespace bmxk;
@@ -1004,25 +1023,14 @@ int bmxk_rtn_dequant_dense(const bmxk_rtn_geom* g, const void* pages, const int3
   BMXK_REQUIRE(out_dtype == BMXK_DTYPE_F16 || out_dtype == BMXK_DTYPE_BF16, "bmxk_rtn_dequant_dense: out_dtype=%d (fp16 or bf16)", out_dtype);
   BMXK_REQUIRE((((uintptr_t)pages | (uintptr_t)k_out | (uintptr_t)v_out | (uintptr_t)k_tail | (uintptr_t)v_tail) & 15) == 0,
                "bmxk_rtn_dequant_dense: misaligned buffer");
-  const dim3 grid((unsigned)blocks, (unsigned)g->h_kv);
+  const RtnGeom gg = to_rtn(g);
   cudaStream_t s = (cudaStream_t)stream;
-#define BMXK_RTN_DENSE(OutT, PAGE)                                                                                                          \
-  {                                                                                                                                          \
-    static PerDeviceOnce configured;                                                                                                         \
-    if (configured.first()) cudaFuncSetAttribute(rtn_dequant_dense_kernel<OutT, PAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * PAGE * 256); \
-    rtn_dequant_dense_kernel<OutT, PAGE><<<grid, RTND_THREADS, 2 * PAGE * 256, s>>>(to_rtn(g), (const uint8_t*)pages, page_table, table_stride, n_pages,   \
-                                                                     (const __half*)k_tail, (const __half*)v_tail, tail_len, tail_cap,      \
-                                                                     (OutT*)k_out, (OutT*)v_out, row_stride);     \
-  }
-  if (out_dtype == BMXK_DTYPE_F16) {
-    if (g->page == 128) BMXK_RTN_DENSE(__half, 128)
-    else BMXK_RTN_DENSE(__half, 64)
-  } else {
-    if (g->page == 128) BMXK_RTN_DENSE(__nv_bfloat16, 128)
-    else BMXK_RTN_DENSE(__nv_bfloat16, 64)
-  }
+#define BMXK_RTN_DENSE(OutT, PAGE)                                                                                                      \
+  launch_rtn_dense<OutT, PAGE>(gg, (int)blocks, (const uint8_t*)pages, page_table, table_stride, n_pages, (const __half*)k_tail,        \
+                               (const __half*)v_tail, tail_len, tail_cap, (OutT*)k_out, (OutT*)v_out, row_stride, s)
+  if (out_dtype == BMXK_DTYPE_F16) return g->page == 128 ? BMXK_RTN_DENSE(__half, 128) : BMXK_RTN_DENSE(__half, 64);
+  return g->page == 128 ? BMXK_RTN_DENSE(__nv_bfloat16, 128) : BMXK_RTN_DENSE(__nv_bfloat16, 64);
 #undef BMXK_RTN_DENSE
-  return check_launch("bmxk_rtn_dequant_dense");
 }
 
 static int rtn_decode_impl(const bmxk_rtn_geom* g, const void* q, const void* pages, const int32_t* page_table, int table_stride,

@@ -4,6 +4,8 @@ arguments on the host before any launch (no GPU needed for any of this)."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 
@@ -58,6 +60,22 @@ def test_argument_errors_are_reported_not_launched(lib):
     assert b"block_bytes" in lib.bmxk_last_error()
     assert lib.bmxk_vblock_bytes() == 128 * 32 + 128 * 2
     assert lib.bmxk_vblock_append(0, None, 0, 0, 0, 0, None, None, None, 1, 1, None, None) == _lib.BMXK_ERR_INVALID
+
+
+def test_a_failed_kernel_set_up_is_reported_by_name_every_time():
+    """Without a device (hidden from the child process) the shared-memory opt-in of the dense RTN route fails: the first call and the next one
+    say so, instead of a launch that fails for a reason of its own."""
+    child = """
+import ctypes
+from bmx_b200 import _lib
+lib, g = _lib.lib(), _lib.RtnGeom(2, 4, 128, 1, 64, 64, 2, 2)
+for dtype in (_lib.DTYPE_F16, _lib.DTYPE_BF16):
+    for _ in range(2):
+        rc = lib.bmxk_rtn_dequant_dense(ctypes.byref(g), 4096, 4096, 4, 4, 1, 4096, 4096, 8, 8, 4096, 4096, 520, dtype, None)
+        assert rc == 2 and b"cudaFuncSetAttribute" in lib.bmxk_last_error(), (rc, lib.bmxk_last_error())
+"""
+    r = subprocess.run([sys.executable, "-c", child], cwd=ROOT, env={**os.environ, "CUDA_VISIBLE_DEVICES": "-1"}, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-800:]
 
 
 def test_value_table_is_exact_to_1e6(lib):
