@@ -24,6 +24,23 @@ def test_only_the_plain_causal_mask_passes(n_q, S):
     assert not is_causal(base[None, None][..., : S - 1], n_q, S)
 
 
+@pytest.mark.parametrize("n_q,S", [(3, 64), (3, 61), (40, 4096)])
+def test_any_byte_but_zero_is_true(n_q, S):
+    """The answer does not depend on which byte stands for true, in the wide loop (rows on 16-byte boundaries) as in the other."""
+    from bmx_b200 import kernels as K
+
+    dev = torch.device("cuda:0")
+    ones = torch.ones(n_q, S, dtype=torch.uint8, device=dev).tril(S - n_q)[None, None]
+    for byte in (1, 2, 0x80, 0xFF):
+        mask = ones * byte
+        assert K.mask_is_causal(mask.view(torch.bool), n_q, S), byte
+        mask[0, 0, 0, 1] = 0
+        assert not K.mask_is_causal(mask.view(torch.bool), n_q, S), byte
+        mask[0, 0, 0, 1] = byte
+        mask[0, 0, 0, S - 1] = byte
+        assert not K.mask_is_causal(mask.view(torch.bool), n_q, S), byte
+
+
 @pytest.mark.parametrize("n_q", [1, 5, 70])
 def test_a_causal_mask_may_be_anywhere_and_laid_out_anyhow(n_q):
     """The plain causal mask on the host, as a transposed view, as a slice of a wider one or expanded over the sequences gives the
