@@ -855,8 +855,12 @@ def config_prefill(device) -> dict:
         legacy_us = _event_us(lambda: state.prefill_attend(q, S - n_q, out=o), 3, warm=1)
         K.k2b_prefill_select(0)  # the tcgen05 kernel (default); few rows: the page walk shared out over CTAs + merge kernel
         paged_us = _event_us(lambda: state.prefill_attend(q, S - n_q, out=o), 3, warm=1)
+        torch.cuda.reset_peak_memory_stats(device)
+        base = torch.cuda.memory_allocated(device)
+        state.prefill_attend(q, S - n_q, out=o)
+        paged_peak = torch.cuda.max_memory_allocated(device) - base  # partial records of a shared walk, rearranged rotation tables
         K.check_status(state.workspace)
-        n_split = state.prefill_split(n_q)
+        n_split, n_rope = state.prefill_split(n_q), state.prefill_rope_pages(n_q, S - n_q)
 
         def dense():  # the product's dense route: one dequantizer kernel writes rotated fp16 K and V in place, then SDPA
             kx, vx = state.dense_kv(torch.float16)
@@ -877,8 +881,8 @@ def config_prefill(device) -> dict:
                      "speedup": dense_us / paged_us,
                      "paged_tflops": flops / paged_us / 1e6, "peak_tflops": tf_peak,
                      "frac_of_tensor_peak": None if not tf_peak else flops / paged_us / 1e6 / tf_peak,
-                     "dense_route_transient_bytes": int(dense_peak), "paged_route_transient_bytes": 0,
-                     "max_rel_diff_between_routes": err, "page_walk_shares": n_split, "gpu_launches": 1 if n_split == 1 else 2}
+                     "dense_route_transient_bytes": int(dense_peak), "paged_route_transient_bytes": int(paged_peak),
+                     "max_rel_diff_between_routes": err, "page_walk_shares": n_split, "gpu_launches": 1 + (n_split > 1) + (n_rope > 0)}
         del q, o, ref
     return out
 

@@ -66,7 +66,7 @@ static inline int grid_for(int64_t n, int block) {
 }
 
 // Is a boolean mask the plain causal one (row i of n_q sees columns 0 .. S - n_q + i)?  One block per row; a differing byte sets the
-// flag.  What bounds it: one read of the mask (8.5 MB for 1024 rows over 8320 columns: 4 us; building the expected mask,
+// flag.  What bounds it: one read of the mask (8.5 MB for 1024 rows over 8320 columns: 6 us; building the expected mask,
 // comparing and reducing took four launches and 50 us).
 __global__ void __launch_bounds__(128) mask_is_causal_kernel(const uint8_t* __restrict__ mask, int64_t stride_b, int64_t stride_q, int n_q, int S,
                                                              int wide, int32_t* __restrict__ differs) {

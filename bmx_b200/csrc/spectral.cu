@@ -51,9 +51,11 @@ __device__ __forceinline__ float code_by_division(float x, float scale, float lo
 //               skipped.  Chains need 3 to 10 rounds (mean 6), the slowest of 32 nearly always 10: after rounds 4, 6 and 8 the chains
 //               that still move are packed to the front of the block (after every round costs more in barriers than it saves).
 //               Divisions become products with the reciprocal (codes_by_product); rounds with a value near a half divide.
-// Measured, 2048 blocks (four sequences of 8192 tokens x 8 heads, 104 of 128 directions with bits, groups of 64), with the value half
-// (60 us): 968 -> 375 us; of the rest about 150 are the product (104 at the fp32 peak), 90 the refinement, 50 the loads, 20 the codes.
-// Packed fp32 pairs for the product (409 us: operand bandwidth), 64-row blocks at three or four per SM (397, 427 us) are slower.
+// Measured, 2048 blocks (four sequences of 8192 tokens x 8 heads, 104 of 128 directions with bits, groups of 64): 927 -> 320 us (with
+// the value blocks of value_blocks.cu 1013 -> 374 us), of which about 150 are the product (104 at the fp32 peak), 90 the refinement, 50
+// the loads, 20 the codes.
+// Packed fp32 pairs for the product (409 us with the values: operand bandwidth), 64-row blocks at three or four per SM (397, 427 us) are
+// slower.
 constexpr int SQ_THREADS = 256, SQ_CHUNK = 32;
 __host__ __device__ constexpr int sq_stride(int page) { return page + 4; }  // floats per channel row: 128-bit reads of consecutive rows hit distinct banks
 __host__ __device__ constexpr int sq_smem(int page) { return (HEAD_DIM * sq_stride(page) + 2 * SQ_CHUNK * HEAD_DIM + 2 * HEAD_DIM + 16) * 4; }

@@ -13,7 +13,7 @@ namespace bmxk {
 constexpr int VBLOCK_BYTES = 128 * 32 + 128 * 2;
 
 // 16-bit sources.  One block of 256 threads per (item, head); see value_quant.cuh for what bounds it.  Measured, 2048 blocks (four
-// sequences of 8192 tokens x 8 heads, fp16): 85 -> 40 us for the values of a spectral append.
+// sequences of 8192 tokens x 8 heads, fp16): 90 -> 47 us for the values of a spectral append; 1024 blocks 51 -> 27, 512 blocks 33 -> 17.
 template <typename T>
 __global__ void __launch_bounds__(VQ_THREADS, 2) vblock_quant_kernel(int h_kv, const T* __restrict__ v, int64_t stride_seq,
                                                                      int64_t stride_head, int64_t stride_tok,
