@@ -521,7 +521,11 @@ __global__ void __launch_bounds__(P5_THREADS, 1) k2b_prefill_t5_kernel(const Pre
       const bool need = ts > m + 8.f;
       if (__any_sync(0xffffffffu, need)) {
         if (u > 0) {  // the U3 just before this half: the other half of this tile, or of the previous one
-          const bool ok = hf ? warp_wait(&sh->odone[0], (uint32_t)n & 1u, p.status, 50) : warp_wait(&sh->odone[1], (uint32_t)(n - 1) & 1u, p.status, 50);
+          // A parity names a phase only to a warp that knows the phase before it to be over.  That of the other half's barrier is not known
+          // here (its U3 may lag by a tile), so this half's own U3 of the previous tile comes first: U3s finish in the order of
+          // issue, and the phase before the one waited for belongs to an earlier one.
+          const bool ok = (n == 0 || warp_wait(&sh->odone[hf], (uint32_t)(n - 1) & 1u, p.status, 55)) &&
+                          (hf ? warp_wait(&sh->odone[0], (uint32_t)n & 1u, p.status, 50) : warp_wait(&sh->odone[1], (uint32_t)(n - 1) & 1u, p.status, 50));
           if (!ok) { alive = false; break; }
           tc5::fence_after();
           const float f = need ? ex2_approx(m - ts) : 1.f;

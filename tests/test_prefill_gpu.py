@@ -351,3 +351,44 @@ def test_any_softmax_scale(sm_scale, n_q, tokens):
     s = s.masked_fill(~torch.ones(n_q, tokens, dtype=torch.bool, device=dev).tril(tokens - n_q), float("-inf"))
     want = torch.einsum("hgnt,htd->hgnd", torch.softmax(s, -1), vd)
     assert float((got - want).norm() / want.norm()) < 2e-3  # fp16 keys, weights and outputs, 2^-11 each
+
+
+@pytest.mark.parametrize("rank,G,B,h,n_q,tokens,growth,sm_scale", [
+    (32, 4, 2, 3, 300, 3000, 3.0, 128 ** -0.5), (16, 8, 3, 3, 590, 4700, 1.0, 1.0), (32, 1, 1, 5, 300, 3300, 1.0, 0.3), (16, 2, 3, 5, 520, 3900, 6.0, 0.3),
+    (32, 4, 1, 2, 40, 4500, 4.0, 0.3), (16, 8, 1, 1, 60, 257 + 128, 8.0, 0.3)])
+def test_a_running_maximum_that_keeps_moving(rank, G, B, h, n_q, tokens, growth, sm_scale):
+    """Scores that grow along the context (or are large everywhere) move the running maximum in many tiles, each time rescaling the
+    accumulator that the other half's products go to: the same bits every time, and float64 attention over the dequantized pages."""
+    from bmx_b200 import kernels as K
+    from bmx_b200.engine import K2bLayerState
+    from bmx_b200.rope import default_rope_tables
+
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(tokens + n_q)
+    cos, sin = (t.half() for t in default_rope_tables(5e5, 128, tokens + 256, device=dev))
+    st = K2bLayerState(K.k2b_geom(h, G, 128, rank, 64, h), B, tokens, 100, dev, cos, sin)
+    st.set_basis(torch.randn(h * 128, rank, generator=gen, device=dev) / 11)
+    k, v = (torch.randn(B, h, tokens, 128, generator=gen, device=dev).half() for _ in range(2))
+    k = k * torch.linspace(0.3, growth, tokens, device=dev)[:, None].half()
+    st.append(k, k, v)
+    st.sm_scale = sm_scale
+    q = torch.randn(B, h * G, n_q, 128, generator=gen, device=dev).half()
+    first = st.prefill_attend(q, tokens - n_q).clone()
+    for fragments in (0, 10 ** 9):  # rearranged rotation tables and not: the same bits
+        st.ROPE_FRAGMENT_TILES = fragments
+        for _ in range(6):
+            assert torch.equal(st.prefill_attend(q, tokens - n_q), first)
+    K.check_status(st.workspace)
+    K.k2b_prefill_select(1)
+    try:
+        other = st.prefill_attend(q, tokens - n_q)
+    finally:
+        K.k2b_prefill_select(0)
+    kd, vd = st.dense_kv(torch.float16)
+    for b in range(B):
+        s = torch.einsum("hgnd,htd->hgnt", q[b].double().view(h, G, n_q, 128), kd[b].double()) * sm_scale
+        s = s.masked_fill(~torch.ones(n_q, tokens, dtype=torch.bool, device=dev).tril(tokens - n_q), float("-inf"))
+        want = torch.einsum("hgnt,htd->hgnd", torch.softmax(s, -1), vd[b].double()).reshape(h * G, n_q, 128)
+        # the keys' fp16 rounding shifts a score by up to 2^-11 of its terms: the two kernels and the dense pages round at different places
+        floor = float((other[b].double() - want).norm() / want.norm())
+        assert float((first[b].double() - want).norm() / want.norm()) < max(3e-3, 1.5 * floor)
